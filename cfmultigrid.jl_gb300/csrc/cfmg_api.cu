@@ -52,6 +52,16 @@ struct cfmg_handle {
   cfmg::Op* prog_pool = nullptr;   // device program store
   int pool_cap = 0, pool_used = 0;
   std::unordered_map<std::string, int> prog_cache;
+  // coarse tail (k_tail.cu): levels >= tail_from[prec] run there (0: none);
+  // pending_tail: the pending Ops are the tail's, not the cluster engine's
+  int tail_from[2] = {0, 0};
+  bool pending_tail = false;
+  unsigned char* tail_pool = nullptr;  // device store of tail programs
+  size_t tail_cap = 0, tail_used = 0;
+  // the levels' cell lists need remaking; coef_exposed: a coefficient's device
+  // address was handed out, so they are remade at every call that uses them
+  bool lists_dirty = true, coef_exposed = false;
+  std::unordered_map<std::string, size_t> tail_cache;
   bool tb_on = true;  // temporally blocked FP32 smoothing on fine levels
   bool fuse_on = true;  // V-cycle descent: residual and restriction in the last pre-smoothing pass
   // mixed loop: the FP64 solution update in the cycle's last level-1
@@ -96,6 +106,7 @@ struct cfmg_handle {
 };
 
 constexpr int kProgPoolOps = 8192;  // device store of engine programs (~1.9 MB)
+constexpr size_t kTailPoolBytes = 1 << 21;  // device store of coarse-tail programs
 
 // Batched solves: independent instances (each a full handle on the batch's
 // stream) whose whole mixed-precision solves run as programs of the
@@ -216,6 +227,7 @@ int harvest(cfmg_handle* h) {
 }
 
 int flush(cfmg_handle* h);
+int tail_lists(cfmg_handle* h);
 
 int sync(cfmg_handle* h) {
   TRY(flush(h));
@@ -312,9 +324,329 @@ long long box_count(const Box& b) {
   return (long long)(b.i1 - b.i0 + 1) * (b.j1 - b.j0 + 1) * (b.k1 - b.k0 + 1);
 }
 
+// The engine's 8 SMs give about 1/19 of the GPU's FP64 rate, which suits
+// only small FP64 levels; FP32 levels up to engine_cells cells go there.
+long long engine_limit(const cfmg_handle* h, int prec) { return prec == 0 ? h->engine_cells / 16 : h->engine_cells; }
+
+bool coarsest_in_fp64(const cfmg_handle* h) {
+  return L(h) > 1 && (h->coarsest_fp64 > 0 ||
+                      (h->coarsest_fp64 < 0 && (long long)h->lv[L(h) - 1].len <= engine_limit(h, CFMG_FP64)));
+}
+
+// The levels of the coarse tail, per precision: the deepest ones whose
+// smoothing arrays fit one block's shared memory beside the program. FP64
+// levels of more than 6/5 of the engine's FP64 threshold (1500 cells by
+// default) stay out, because one SM's FP64 pipe then takes longer for a sweep
+// than a launch on all SMs does: a 38^2 level with every cell wet takes
+// 2.1 us a sweep in the tail and 2.2 us as a launch.
+constexpr size_t kTailBlobReserve = 24 * 1024;
+constexpr size_t tail_al(size_t b) { return (b + 15) & ~(size_t)15; }
+size_t tail_hot_bytes(const cfmg_handle* h, const Level& l, int prec) {
+  const size_t n = l.len, es = prec ? 4 : 8;
+  return (h->d.op == CFMG_VARCOEF ? 6 : 4) * tail_al(n * es) + tail_al(kTailListHdr + 2 * n);
+}
+void plan_tail(cfmg_handle* h) {
+  for (int prec = 0; prec < 2; ++prec) {
+    h->tail_from[prec] = 0;
+    if (!h->engine_on || h->small_min <= 0 || !h->tail_pool || (prec == 1 && h->d.precision != CFMG_MIXED)) continue;
+    const long long cap = prec == 0 ? engine_limit(h, 0) * 6 / 5 : engine_limit(h, 1);
+    size_t used = kTailBlobReserve;
+    if (prec == 1 && coarsest_in_fp64(h)) used += tail_hot_bytes(h, h->lv.back(), 0);
+    for (int lev = L(h); lev >= 1 && L(h) - lev < kTailMaxCtx - 2; --lev) {
+      const Level& l = h->lv[lev - 1];
+      used += tail_hot_bytes(h, l, prec);
+      if (used > kTailSmemMax || (long long)l.len > cap || !l.tlist) break;
+      h->tail_from[prec] = lev;
+    }
+  }
+}
+bool in_tail(const cfmg_handle* h, int lev, int prec) {
+  return !h->record && h->engine_on && h->tail_from[prec] > 0 && lev >= h->tail_from[prec];
+}
+
+// Builds the pending Ops into tail programs and launches them: pairs of
+// sweeps become smoothing calls, every array they touch is staged in shared
+// memory, the smoothing arrays first, then the others while they fit (those
+// left out are used in place). done = false: the Ops do not form such a
+// program (or the store is full), nothing was launched.
+int flush_tail(cfmg_handle* h, bool& done) {
+  done = false;
+  const std::vector<Op>& P = h->pending;
+  std::vector<TailOp> ops;
+  std::vector<TailCtx> ctxs;
+  struct CtxPtr { const void *x, *y, *b, *w, *cE, *cN, *list; int lev; };
+  std::vector<CtxPtr> cptr;
+  auto u = [](const void* p) { return (unsigned long long)(uintptr_t)p; };
+  for (size_t i = 0; i < P.size();) {
+    const Op& a = P[i];
+    TailOp t;
+    std::memset(&t, 0, sizeof(t));
+    t.prec = a.prec;
+    t.ctxi = -1;
+    t.tx = a.g.tx; t.ty = a.g.ty; t.tz = a.g.tz; t.nh = a.g.nh;
+    t.ctx = a.gc.tx; t.cty = a.gc.ty;
+    if (a.kind >= OPK_SWEEP5 && a.kind <= OPK_SWEEPVC) {
+      // [x -> y, y -> x, fill x] repeated
+      int pairs = 0, fill = -1;
+      size_t k = i;
+      while (k + 1 < P.size() && P[k].kind == a.kind && P[k + 1].kind == a.kind && P[k].lev == a.lev &&
+             P[k].prec == a.prec && P[k].x == a.x && P[k].y == a.y && P[k + 1].x == a.y && P[k + 1].y == a.x &&
+             P[k + 1].lev == a.lev && P[k + 1].prec == a.prec) {
+        const int f = k + 2 < P.size() && P[k + 2].kind == OPK_FILL && P[k + 2].y == a.x ? 1 : 0;
+        if (fill >= 0 && f != fill) break;
+        fill = f;
+        k += 2 + f;
+        ++pairs;
+      }
+      if (!pairs) return CFMG_OK;
+      int q = 0;
+      while (q < (int)ctxs.size() && !(cptr[q].x == a.x && cptr[q].w == a.w)) ++q;
+      if (q == (int)ctxs.size()) {
+        if (q == kTailMaxCtx) return CFMG_OK;
+        const Level& l = h->lv[a.lev - 1];
+        TailCtx c;
+        std::memset(&c, 0, sizeof(c));
+        c.stencil = a.kind == OPK_SWEEP5 ? TAIL_5 : a.kind == OPK_SWEEP7 ? TAIL_7 : a.kind == OPK_SWEEP9 ? TAIL_9
+                    : a.kind == OPK_SWEEP19 ? TAIL_19 : TAIL_VC;
+        c.prec = a.prec;
+        c.n1 = (int)a.g.n1; c.n2 = (int)a.g.n2;
+        c.lines = l.ty * l.tz; c.nh = l.nh;
+        c.cff = a.cff;
+        ctxs.push_back(c);
+        const bool vc = a.kind == OPK_SWEEPVC;
+        cptr.push_back({a.x, a.y, a.b, a.w, vc ? a.cE : nullptr, vc ? a.cN : nullptr, l.tlist, a.lev});
+      }
+      t.kind = TAIL_SMOOTH;
+      t.ctxi = q;
+      t.npairs = pairs;
+      t.fill = fill;
+      i = k;
+    } else {
+      const bool pro = a.kind >= OPK_PROLONG0 && a.kind <= OPK_PROLONG3;
+      if (!(a.kind >= OPK_RESID5 && a.kind <= OPK_F64TO32) || a.n > 0x7fffffff || a.assign) return CFMG_OK;
+      t.kind = a.kind;
+      t.n = (int)a.n;
+      t.lo = (int)a.lo;
+      t.box = a.box;
+      if (pro) { t.np_i = a.np_i; t.np_j = a.np_j; t.kf0 = a.kf0; }
+      t.x = u(a.x); t.b = u(a.b); t.d = u(a.d); t.cE = u(a.cE); t.cN = u(a.cN); t.coef = u(a.coef); t.y = u(a.y);
+      t.m = pro ? 0 : u(a.m);
+      t.lo = (int)a.lo;
+      if (a.kind >= OPK_RESID5 && a.kind <= OPK_RESIDVC) t.npairs = a.lev;  // resolved to a context below
+      ++i;
+    }
+    ops.push_back(t);
+  }
+  // a residual below level 1 takes its level's list (level 1's r keeps the
+  // reference's signed zeros in dry cells)
+  for (TailOp& t : ops) {
+    if (!(t.kind >= OPK_RESID5 && t.kind <= OPK_RESIDVC)) continue;
+    const int lev = t.npairs;
+    t.npairs = 0;
+    for (int q = 0; q < (int)ctxs.size(); ++q)
+      if (lev > 1 && cptr[q].lev == lev && ctxs[q].prec == t.prec && u(cptr[q].x) == t.x) t.ctxi = q;
+  }
+  // program pieces that fit the reserve
+  struct Launchable { size_t off; int bytes, nctx, nstore, ncopy, nops; size_t smem; };
+  std::vector<Launchable> todo;
+  constexpr size_t kPiece = 100;
+  for (size_t o0 = 0; o0 < ops.size(); o0 += kPiece) {
+    std::vector<TailOp> po(ops.begin() + o0, ops.begin() + std::min(ops.size(), o0 + kPiece));
+    std::vector<TailCtx> pcx;
+    std::vector<int> renum(ctxs.size(), -1);
+    struct Arr { unsigned long long g; size_t bytes; bool hot, written, in; unsigned off; };
+    std::vector<Arr> arr;
+    typedef std::vector<unsigned long long> Set;
+    Set rd, wr, rd_all, wr_all;  // operands of this operator / of those since the last barrier
+    auto use = [&](unsigned long long g, size_t bytes, bool hot, bool written) {
+      if (!g) return;
+      (written ? wr : rd).push_back(g);
+      for (Arr& r : arr)
+        if (r.g == g) {
+          r.bytes = std::max(r.bytes, bytes);
+          r.hot |= hot;
+          r.written |= written;
+          return;
+        }
+      arr.push_back({g, bytes, hot, written, false, 0});
+    };
+    auto meet = [](const Set& a, const Set& b) {
+      for (unsigned long long p : a)
+        for (unsigned long long q : b)
+          if (p == q) return true;
+      return false;
+    };
+    for (size_t k = 0; k < po.size(); ++k) {
+      TailOp& t = po[k];
+      const size_t es = t.prec ? 4 : 8;
+      const size_t nf = (size_t)t.tx * t.ty * t.tz * es;
+      rd.clear();
+      wr.clear();
+      if (t.ctxi >= 0) {
+        if (renum[t.ctxi] < 0) {
+          renum[t.ctxi] = (int)pcx.size();
+          pcx.push_back(ctxs[t.ctxi]);
+        }
+        use(u(cptr[t.ctxi].list), kTailListHdr + 2 * nf / es, true, false);
+      }
+      // the coarse level's length of a transfer
+      size_t nc = 0;
+      if (t.ctx)
+        for (const Level& l : h->lv)
+          if (l.tx == t.ctx && l.ty == t.cty) nc = std::max(nc, l.len * es);
+      if (t.kind == TAIL_SMOOTH) {
+        const CtxPtr& c = cptr[t.ctxi];
+        use(u(c.x), nf, true, true);
+        use(u(c.y), nf, true, true);
+        for (const void* q : {c.b, c.w, c.cE, c.cN}) use(u(q), nf, true, false);
+      } else if (t.kind >= OPK_RESTRICT0 && t.kind <= OPK_RESTRICT3) {
+        use(t.x, nf, false, false);
+        use(t.coef, nc, false, false);
+        use(t.y, nc, false, true);
+      } else if (t.kind >= OPK_PROLONG0 && t.kind <= OPK_PROLONG3) {
+        use(t.x, nc, false, false);
+        use(t.coef, nf, false, false);
+        use(t.y, nf, false, true);
+      } else if (t.kind == OPK_F32TO64 || t.kind == OPK_F64TO32) {
+        use(t.x, (size_t)t.n * (t.kind == OPK_F32TO64 ? 4 : 8), false, false);
+        use(t.y, (size_t)t.n * (t.kind == OPK_F32TO64 ? 8 : 4), false, true);
+      } else if (t.kind == OPK_ZERO || t.kind == OPK_FILL) {
+        use(t.y, nf, false, true);
+      } else {  // residual
+        for (unsigned long long q : {t.x, t.b, t.d, t.cE, t.cN}) use(q, nf, false, false);
+        use(t.m, (size_t)t.tx * t.ty * t.tz, false, false);
+        use(t.y, nf, false, true);
+      }
+      // no barrier before this operator when it meets none since the last one
+      // (a smoothing call has barriers of some warps inside: never left open)
+      const bool free_ = k > 0 && t.kind != TAIL_SMOOTH && po[k - 1].kind != TAIL_SMOOTH && !meet(wr, wr_all) &&
+                         !meet(wr, rd_all) && !meet(rd, wr_all);
+      if (free_) po[k - 1].nobar = 1;
+      else {
+        rd_all.clear();
+        wr_all.clear();
+      }
+      rd_all.insert(rd_all.end(), rd.begin(), rd.end());
+      wr_all.insert(wr_all.end(), wr.begin(), wr.end());
+    }
+    // the pieces of the arrays: their number before their place is known
+    size_t ncopy_max = 0;
+    for (const Arr& r : arr) ncopy_max += (tail_al(r.bytes) + kTailPiece - 1) / kTailPiece;
+    size_t at = tail_al(pcx.size() * sizeof(TailCtx) + ncopy_max * sizeof(TailCopy) + po.size() * sizeof(TailOp));
+    auto place = [&](Arr& r) {
+      r.off = (unsigned)at;
+      r.in = true;
+      at += tail_al(r.bytes);
+    };
+    for (Arr& r : arr)
+      if (r.hot) place(r);
+    if (at > kTailSmemMax) return CFMG_OK;
+    std::vector<size_t> ord(arr.size());
+    for (size_t k = 0; k < ord.size(); ++k) ord[k] = k;
+    std::stable_sort(ord.begin(), ord.end(), [&](size_t p, size_t q) { return arr[p].bytes < arr[q].bytes; });
+    for (size_t k : ord)
+      if (!arr[k].in && at + tail_al(arr[k].bytes) <= kTailSmemMax) place(arr[k]);
+    auto where = [&](unsigned long long g) -> unsigned long long {
+      for (const Arr& r : arr)
+        if (r.g == g && r.in) return kTailSmem | r.off;
+      return g;
+    };
+    for (size_t q = 0; q < ctxs.size(); ++q) {
+      if (renum[q] < 0) continue;
+      TailCtx& c = pcx[renum[q]];
+      const CtxPtr& p = cptr[q];
+      c.ox = (unsigned)where(u(p.x)); c.oy = (unsigned)where(u(p.y)); c.ob = (unsigned)where(u(p.b));
+      c.ow = (unsigned)where(u(p.w)); c.oE = (unsigned)where(u(p.cE)); c.oN = (unsigned)where(u(p.cN));
+      c.olist = (unsigned)where(u(p.list));
+    }
+    std::vector<TailCopy> cps;
+    int nstore = 0;
+    for (int written = 1; written >= 0; --written) {
+      for (const Arr& r : arr) {
+        if (!r.in || (int)r.written != written) continue;
+        for (size_t o = 0; o < tail_al(r.bytes); o += kTailPiece) {
+          TailCopy c;
+          std::memset(&c, 0, sizeof(c));
+          c.g = (void*)(uintptr_t)(r.g + o);
+          c.off = r.off + (unsigned)o;
+          c.bytes = (unsigned)std::min((size_t)kTailPiece, tail_al(r.bytes) - o);
+          cps.push_back(c);
+        }
+      }
+      if (written) nstore = (int)cps.size();
+    }
+    for (TailOp& t : po) {
+      if (t.ctxi >= 0) t.ctxi = renum[t.ctxi];
+      for (unsigned long long* q : {&t.x, &t.b, &t.d, &t.cE, &t.cN, &t.coef, &t.m, &t.y})
+        if (*q) *q = where(*q);
+    }
+    std::string key;
+    key.append((const char*)pcx.data(), pcx.size() * sizeof(TailCtx));
+    key.append((const char*)cps.data(), cps.size() * sizeof(TailCopy));
+    key.append((const char*)po.data(), po.size() * sizeof(TailOp));
+    const int bytes = (int)tail_al(key.size());
+    key.resize(bytes, 0);
+    size_t off;
+    auto it = h->tail_cache.find(key);
+    if (it != h->tail_cache.end()) {
+      off = it->second;
+    } else {
+      if (h->tail_used + bytes > h->tail_cap) return CFMG_OK;
+      // synchronous, and never over a program that a graph refers to (as in flush)
+      CUDA_OK(h, cudaMemcpy(h->tail_pool + h->tail_used, key.data(), bytes, cudaMemcpyHostToDevice));
+      off = h->tail_used;
+      h->tail_used += (bytes + 255) & ~(size_t)255;
+      h->tail_cache.emplace(std::move(key), off);
+    }
+    todo.push_back({off, bytes, (int)pcx.size(), nstore, (int)cps.size(), (int)po.size(), at});
+  }
+  for (const Launchable& q : todo) {
+    Launch k(h, CFMG_K_ENGINE, 0, P[0].prec ? CFMG_MIXED : CFMG_FP64);
+    launch_tail(h->tail_pool + q.off, q.bytes, q.nctx, q.nstore, q.ncopy, q.nops, q.smem, h->stream);
+  }
+  done = true;
+  return CFMG_OK;
+}
+
+// Remakes the levels' cell lists after a change of coefficients: called where
+// a smoothing call, a cycle or a solve begins, before any capture.
+int tail_lists(cfmg_handle* h) {
+  if ((!h->lists_dirty && !h->coef_exposed) || (h->tail_from[0] <= 0 && h->tail_from[1] <= 0)) return CFMG_OK;
+  TRY(flush(h));
+  TailListArgs a;
+  std::memset(&a, 0, sizeof(a));
+  int n = 0;
+  for (int lev = L(h); lev >= 1 && n < kTailMaxCtx; --lev) {
+    const Level& l = h->lv[lev - 1];
+    if (!l.tlist) break;
+    TailListLevel& q = a.lev[n++];
+    q.w = l.widiag; q.pc = l.Pcoef; q.m = l.msk; q.out = l.tlist;
+    q.len = (int)l.len; q.n1 = l.tx; q.nj = l.ty;
+    q.box = h->d.op == CFMG_LAPLACIAN9;
+    const int off = threed(h) ? l.tx * l.ty : l.tx;
+    q.lo = off; q.hi = (int)l.len - off;
+    q.ext = Box{l.nh, l.nx + l.nh + 1, l.nh, l.ny + l.nh + 1, threed(h) ? l.nh : 1, threed(h) ? l.nz + l.nh + 1 : l.nz};
+    q.in = interior(l);
+  }
+  launch_tail_lists(a, n, h->stream);
+  LAUNCH_OK(h);
+  h->lists_dirty = false;
+  return CFMG_OK;
+}
+
 int flush(cfmg_handle* h) {
   if (h->record || h->pending.empty()) return CFMG_OK;
   const int n = (int)h->pending.size();
+  // a single operator is a launch of its own; several on the tail's levels are a tail program
+  if (h->pending_tail && (n > 1 || h->pending[0].kind == OPK_FILL)) {
+    bool done = false;
+    TRY(flush_tail(h, done));
+    if (done) {
+      h->pending.clear();
+      LAUNCH_OK(h);
+      return CFMG_OK;
+    }
+  }
   std::string key((const char*)h->pending.data(), (size_t)n * sizeof(Op));
   auto it = h->prog_cache.find(key);
   int off = -1;
@@ -343,9 +675,21 @@ int flush(cfmg_handle* h) {
   return CFMG_OK;
 }
 
-// The engine's 8 SMs give about 1/19 of the GPU's FP64 rate, which suits
-// only small FP64 levels; FP32 levels up to engine_cells cells go there.
-long long engine_limit(const cfmg_handle* h, int prec) { return prec == 0 ? h->engine_cells / 16 : h->engine_cells; }
+// Whether a level's Ops are gathered instead of launched one by one: the
+// tail's levels, and levels within the cluster engine's threshold. FP32 2D
+// levels beyond the tail that have blocked passes are left to those: a
+// descent step is one launch there and 11 Ops of 2.3 us in the engine.
+bool blocked_form(const cfmg_handle* h, int lev) {
+  if (!h->tb_on || h->record || threed(h) || h->small_min <= 0 || h->tail_from[1] <= 0) return false;
+  if (h->d.op != CFMG_LAPLACIAN && h->d.op != CFMG_LAPLACIAN9) return false;
+  return !xperio(h) || (h->tb_version == 5 && h->d.op == CFMG_LAPLACIAN);
+}
+bool in_engine(const cfmg_handle* h, int lev, int prec) {
+  if (!h->engine_on) return false;
+  if (in_tail(h, lev, prec)) return true;
+  if ((long long)h->lv[lev - 1].len > engine_limit(h, prec)) return false;
+  return !(prec && blocked_form(h, lev));
+}
 
 int emit(cfmg_handle* h, const Op& op) {
   if (op.n <= 0) return CFMG_OK;
@@ -353,8 +697,10 @@ int emit(cfmg_handle* h, const Op& op) {
     h->pending.push_back(op);
     return CFMG_OK;
   }
-  const Level& l = h->lv[op.lev - 1];
-  if (h->engine_on && (long long)l.len <= engine_limit(h, op.prec)) {
+  if (in_engine(h, op.lev, op.prec)) {
+    const bool tail = in_tail(h, op.lev, op.prec);
+    if (!h->pending.empty() && h->pending_tail != tail) TRY(flush(h));
+    h->pending_tail = tail;
     h->pending.push_back(op);
     return CFMG_OK;
   }
@@ -417,8 +763,8 @@ bool tb_eligible(const cfmg_handle* h, int lev) {
   // four single-sweep kernels at 66 % of HBM
   if (threed(h) && (h->d.op != CFMG_LAPLACIAN || h->record || h->tb_version != 4)) return false;
   if (h->d.op != CFMG_LAPLACIAN && h->d.op != CFMG_LAPLACIAN9) return false;
-  const Level& l = h->lv[lev - 1];
-  return !(h->engine_on && (long long)l.len <= engine_limit(h, CFMG_MIXED));
+  if (h->record) return !(h->engine_on && (long long)h->lv[lev - 1].len <= engine_limit(h, CFMG_MIXED));
+  return !in_engine(h, lev, CFMG_MIXED);
 }
 
 // 3D 19-point FP32 level of a closed topology, standalone: its smoothing
@@ -429,7 +775,7 @@ bool tb3d19_ok(const cfmg_handle* h, int lev) {
     return false;
   const Level& l = h->lv[lev - 1];
   if (l.nh < 2) return false;
-  return !(h->engine_on && (long long)l.len <= engine_limit(h, CFMG_MIXED));
+  return !in_engine(h, lev, CFMG_MIXED);
 }
 
 // 3D 7-point: passes of up to 2 pairs (k_tb3d.cu), x -> partner buffer
@@ -525,6 +871,7 @@ template <class T>
 bool small_smooth_ok(const cfmg_handle* h, int lev, int nite) {
   if (h->record || xperio(h) || h->small_min <= 0 || nite < h->small_min) return false;
   if (!(h->d.op == CFMG_LAPLACIAN || (h->d.op == CFMG_LAPLACIAN9 && !threed(h)))) return false;
+  if (in_tail(h, lev, pc<T>())) return false;
   if (sizeof(T) == 4 && lev == 1 && h->x1_zero) return false;  // that sweep must not read x
   const Level& l = h->lv[lev - 1];
   if (l.xswap) return false;
@@ -686,7 +1033,7 @@ int prolong_t(cfmg_handle* h, int lev, bool onto_zero = false) {
   // FP32 cycles of a closed topology: parents whose children are all dry are skipped
   if (sizeof(T) == 4 && h->dry_on && !xperio(h)) op.m = f.msk;
   if (onto_zero) {
-    if (!h->record && !(h->engine_on && (long long)f.len <= engine_limit(h, pc<T>()))) op.assign = 1;
+    if (!h->record && !in_engine(h, lev, pc<T>())) op.assign = 1;
     else TRY(zero_t<T>(h, lev, CFMG_X));
   }
   TRY(emit(h, op));
@@ -709,10 +1056,6 @@ int coarsest_t(cfmg_handle* h, int nite);
 template <>
 int coarsest_t<double>(cfmg_handle* h, int nite) {
   return smooth_t<double>(h, L(h), nite);
-}
-bool coarsest_in_fp64(const cfmg_handle* h) {
-  return L(h) > 1 && (h->coarsest_fp64 > 0 ||
-                      (h->coarsest_fp64 < 0 && (long long)h->lv[L(h) - 1].len <= engine_limit(h, CFMG_FP64)));
 }
 template <>
 int coarsest_t<float>(cfmg_handle* h, int nite) {
@@ -787,7 +1130,7 @@ bool resid_restrict3d_ok(const cfmg_handle* h, int lev) {
       vertices(h) || !h->wq_on || !h->wq_ok)
     return false;
   const Level& f = h->lv[lev - 1];
-  if (h->engine_on && (long long)f.len <= engine_limit(h, CFMG_MIXED)) return false;
+  if (in_engine(h, lev, CFMG_MIXED)) return false;
   const Box fi = interior(f), ci = interior(h->lv[lev]);
   auto c2f = [](int i, int nh) { return (i - nh - 1) * 2 + nh + 1; };
   return c2f(ci.i0, f.nh) >= fi.i0 && c2f(ci.i1, f.nh) + 1 <= fi.i1 && c2f(ci.j0, f.nh) >= fi.j0 &&
@@ -1003,7 +1346,7 @@ int setup_operators_body(cfmg_handle* h) {
     launch_widiag(l.idiag, l.widiag, h->d.omega, l.len, s);
   }
   LAUNCH_OK(h);
-  h->mixed_dirty = true;
+  h->mixed_dirty = h->lists_dirty = true;
   return CFMG_OK;
 }
 
@@ -1319,7 +1662,7 @@ bool x1_zero_ok(const cfmg_handle* h, int kind) {
       !h->wq_ok || tb_eligible<float>(h, 1) || L(h) < 2)
     return false;
   const Level& l = h->lv[0];
-  if (h->engine_on && (long long)l.len <= engine_limit(h, CFMG_MIXED)) return false;
+  if (in_engine(h, 1, CFMG_MIXED)) return false;
   const View<float> v = view<float>(l);
   return l.xswap == 0 && sweep7_quad_ok(geom(l), v.x, v.y, v.b, l.wq);
 }
@@ -1688,7 +2031,10 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
   // coded omega*idiag: the 3D 7-point operator's standalone FP32 sweeps
   const bool coded = mixed && d->kase == CFMG_THREED && d->op == CFMG_LAPLACIAN;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  size_t total = al(kPartials * sizeof(double)) + al(S_COUNT * sizeof(double)) + al((size_t)pool_ops * sizeof(Op));
+  const size_t tail_bytes = shared ? 0 : kTailPoolBytes;
+  auto tailed = [&](const Level& l) { return tail_bytes && l.len <= (size_t)kTailMaxLen; };
+  size_t total = al(kPartials * sizeof(double)) + al(S_COUNT * sizeof(double)) + al((size_t)pool_ops * sizeof(Op)) +
+                 al(tail_bytes);
   for (const Level& l : h->lv) {
     size_t n = l.len;
     total += 8 * al(n * 8) + al(n);           // x y r b diag idiag widiag Rcoef Pcoef + msk (Pcoef counted below)
@@ -1697,6 +2043,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
     total += (mixed ? 8 : 0) * al(n * 4);     // x32 y32 r32 b32 widiag32 diag32 Rcoef32 Pcoef32
     total += (mixed && vc ? 2 : 0) * al(n * 4);
     total += coded ? al(n) : 0;               // wq
+    total += tailed(l) ? al(kTailListHdr + 2 * n) : 0;  // tlist
   }
   total += coded ? al(256 * sizeof(float)) : 0;  // wtab
   if (cudaMalloc(&h->arena, total) != cudaSuccess) {
@@ -1714,6 +2061,8 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
   h->partials = (double*)take(kPartials * sizeof(double));
   h->prog_pool = (Op*)take((size_t)pool_ops * sizeof(Op));
   h->pool_cap = pool_ops;
+  if (tail_bytes) h->tail_pool = (unsigned char*)take(tail_bytes);
+  h->tail_cap = tail_bytes;
   h->dscal = (double*)take(S_COUNT * sizeof(double));
   for (Level& l : h->lv) {
     size_t n = l.len;
@@ -1729,6 +2078,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
       if (vc) { l.cE32 = (float*)take(n * 4); l.cN32 = (float*)take(n * 4); }
     }
     if (coded) l.wq = (uint8_t*)take(n);
+    if (tailed(l)) l.tlist = (unsigned char*)take(kTailListHdr + 2 * n);
   }
   if (coded) h->wtab = (float*)take(256 * sizeof(float));
   // the fixed-point residual pass reads kResidIntReach elements beside level
@@ -1752,6 +2102,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
     return fail(nullptr, CFMG_ERR_ALLOC, "stream or pinned allocation failed");
   }
   h->stream = shared ? shared : h->own_stream;
+  plan_tail(h);
   if (cudaMemsetAsync(h->arena, 0, total, h->stream) != cudaSuccess) {
     cfmg_destroy(h);
     return fail(nullptr, CFMG_ERR_CUDA, "arena clear failed");
@@ -1845,6 +2196,7 @@ int cfmg_field_ptr(cfmg_handle* h, int lev, int field, void** dptr) {
   size_t elt;
   void* p = field_any(h->lv[lev - 1], field, &elt);
   if (!p || !dptr) return fail(h, CFMG_ERR_ARG, "unknown field (kappa exists only for the varcoef operator)");
+  if (field >= CFMG_DIAG) h->coef_exposed = true;
   *dptr = p;
   return CFMG_OK;
 }
@@ -1854,7 +2206,7 @@ static int refresh_derived(cfmg_handle* h, int lev, int field) {
   if (field == CFMG_IDIAG) launch_widiag(l.idiag, l.widiag, h->d.omega, l.len, h->stream);
   if (h->d.op == CFMG_VARCOEF && (field == CFMG_KAPPA || field == CFMG_MSK))
     launch_face_coef(l.kappa, l.msk, l.cE, l.cN, geom(l), h->stream);
-  if (field >= CFMG_DIAG) h->mixed_dirty = true;
+  if (field >= CFMG_DIAG) h->mixed_dirty = h->lists_dirty = true;
   LAUNCH_OK(h);
   return CFMG_OK;
 }
@@ -1894,7 +2246,7 @@ int cfmg_bind_level(cfmg_handle* h, int lev, const double* diag, const double* i
   if (msk) CUDA_OK(h, cudaMemcpyAsync(l.msk, msk, l.len, cudaMemcpyDefault, s));
   TRY(refresh_derived(h, lev, CFMG_IDIAG));
   if (msk) TRY(refresh_derived(h, lev, CFMG_MSK));
-  h->mixed_dirty = true;
+  h->mixed_dirty = h->lists_dirty = true;
   h->coef_set = true;
   h->solved = false;
   return sync(h);
@@ -1905,6 +2257,7 @@ int cfmg_set_default_msk(cfmg_handle* h) {
   Level& l = h->lv[0];
   launch_default_msk(DEFMSK_SET, l.msk, nullptr, 0.0, l, vertices(h), threed(h), xperio(h), h->stream);
   LAUNCH_OK(h);
+  h->lists_dirty = true;
   return sync(h);
 }
 
@@ -1921,6 +2274,7 @@ int cfmg_smooth(cfmg_handle* h, int lev, int nite) {
   TRY(check_lev(h, lev));
   TRY(need_setup(h));
   if (nite < 0) return fail(h, CFMG_ERR_ARG, "nite must be >= 0");
+  TRY(tail_lists(h));
   TRY(smooth_t<double>(h, lev, nite));
   return flush(h);
 }
@@ -1968,6 +2322,7 @@ int cfmg_fill(cfmg_handle* h, int lev, int field) {
   if (!p) return fail(h, CFMG_ERR_ARG, "unknown field");
   if (!xperio(h)) return CFMG_OK;
   TRY(flush(h));
+  if (field >= CFMG_DIAG) h->lists_dirty = true;
   if (elt == 1) launch_fill_xperio<uint8_t>((uint8_t*)p, geom(l), h->stream);
   else launch_fill_xperio<double>((double*)p, geom(l), h->stream);
   LAUNCH_OK(h);
@@ -2004,6 +2359,7 @@ int cfmg_normresidual(cfmg_handle* h, double normb, double* out) {
 int cfmg_cycle(cfmg_handle* h, int kind) {
   if (!h) return CFMG_ERR_ARG;
   TRY(need_setup(h));
+  TRY(tail_lists(h));
   return cycle_t<double>(h, kind);
 }
 
@@ -2038,6 +2394,7 @@ int cfmg_solve(cfmg_handle* h, double* res_out, int* nite_out, double* history) 
   if (prec == CFMG_MIXED && d.cycle != CFMG_CYCLE_V && d.cycle != CFMG_CYCLE_F && d.cycle != CFMG_CYCLE_VREC)
     return fail(h, CFMG_ERR_UNSUPPORTED, "the mixed-precision form runs V and F cycles");
   if (prec == CFMG_MIXED) TRY(prepare_mixed(h));
+  TRY(tail_lists(h));
   // normb = norm(mg, 1, :b) (src/gmg_solver.jl:22)
   const Level& l1 = h->lv[0];
   TRY(flush(h));
@@ -2851,6 +3208,7 @@ int cfmg_set_option(cfmg_handle* h, int option, long long value) {
   if (option == CFMG_OPT_COARSEST_FP64) {
     if (value < -1 || value > 1) return fail(h, CFMG_ERR_ARG, "coarsest_fp64 must be -1, 0 or 1");
     h->coarsest_fp64 = (int)value;
+    plan_tail(h);
     drop_graphs(h);
     return CFMG_OK;
   }
@@ -2884,6 +3242,7 @@ int cfmg_set_option(cfmg_handle* h, int option, long long value) {
   if (option == CFMG_OPT_SMALL_SMOOTH) {
     if (value < 0) return fail(h, CFMG_ERR_ARG, "small_smooth must be >= 0");
     h->small_min = (int)value;
+    plan_tail(h);
     drop_graphs(h);
     return CFMG_OK;
   }
@@ -2912,6 +3271,7 @@ int cfmg_set_option(cfmg_handle* h, int option, long long value) {
     if (value < 0) return fail(h, CFMG_ERR_ARG, "engine_cells must be >= 0");
     h->engine_cells = value;
     h->engine_on = value > 0;
+    plan_tail(h);
     drop_graphs(h);  // captured graphs embed the old split
     return CFMG_OK;
   }

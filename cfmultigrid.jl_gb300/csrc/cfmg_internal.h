@@ -67,6 +67,7 @@ struct Level {
   // the same levels, four-cell sweep: 1 for each (run of planes, quad of a
   // plane) holding a wet cell (launch_make_qact); dry quads are skipped
   uint8_t* qact;
+  unsigned char* tlist;  // the coarse tail's cell list (launch_tail_lists); null on levels too large for it
   int xswap;  // 1: the FP32 x currently lives in y32 (after a temporally blocked smoothing)
   int ic0, ic1, jc0, jc1, kc0, kc1;  // interior box (1-based inclusive)
 };
@@ -248,6 +249,52 @@ constexpr int kEngineCtas = 8;      // cluster size (portable)
 constexpr int kEngineThreads = 1024;
 void launch_op(const Op& op, cudaStream_t s);                   // one Op as a standalone kernel
 void launch_program(const Op* prog, int nops, double* red, cudaStream_t s);  // a device-resident program
+
+// ---- coarse tail in one block's shared memory (k_tail.cu)
+// A program: contexts (one level in one precision, as its smoothing calls
+// see it), copies (arrays staged in shared memory), operators. The host lays
+// it out as one blob: TailCtx[nctx], TailCopy[ncopy], TailOp[nops].
+constexpr int kTailThreads = 512;
+constexpr int kTailMaxCtx = 16;
+constexpr size_t kTailSmemMax = 224 * 1024;  // of the SM's 227 KB; the rest is static
+constexpr unsigned long long kTailSmem = 1ull << 63;  // operand in shared memory: offset in the low word
+constexpr int kTailMaxLen = 0x7fff;  // cells of a level: list entries keep bit 15 for a flag
+enum TailStencil { TAIL_5 = 0, TAIL_7, TAIL_9, TAIL_19, TAIL_VC };
+constexpr int TAIL_SMOOTH = 1000;  // TailOp kind: npairs pairs of sweeps of context ctxi
+constexpr int kTailListHdr = 16;  // bytes in front of a list: {listed cells, cells of the range}
+struct alignas(16) TailCtx {
+  int stencil, prec, n1, n2, lines, nh;  // lines: rows of the level (x-periodic fill)
+  unsigned ox, oy, ob, ow, oE, oN, olist;
+  double cff;
+};
+// a piece of an array, at most 16 bytes a thread; the pieces that are written back come first
+struct alignas(16) TailCopy {
+  void* g;
+  unsigned off, bytes;
+};
+constexpr unsigned kTailPiece = 16 * kTailThreads;
+struct alignas(16) TailOp {
+  int kind, prec, ctxi, npairs, fill;
+  int nobar;  // the next operator touches nothing that this one does: no barrier between them
+  int tx, ty, tz, nh, ctx, cty;
+  int n, lo, np_i, np_j, kf0;
+  Box box;
+  unsigned long long x, b, d, cE, cN, coef, m, y;
+};
+void launch_tail(const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops, size_t smem,
+                 cudaStream_t s);
+// the cell lists that its smoothing calls sweep, one per level
+struct TailListLevel {
+  const double *w, *pc;
+  const uint8_t* m;
+  unsigned char* out;  // kTailListHdr bytes, then one 16-bit entry a cell
+  int len, n1, nj, box, lo, hi;  // box != 0: the ranges are the boxes, else lo .. hi
+  Box ext, in;
+};
+struct TailListArgs {
+  TailListLevel lev[kTailMaxCtx];
+};
+void launch_tail_lists(const TailListArgs& a, int n, cudaStream_t s);
 
 // 3D 7-point streaming blocked passes (k_tb3d.cu): nite (1 or 2) pairs over U
 bool launch_smooth_tb3d(int nite, const float* x, float* xo, const float* b, const float* w, float cff, int tx,

@@ -97,7 +97,9 @@ extern "C" {
 /* options for cfmg_set_option */
 #define CFMG_OPT_ENGINE_CELLS 0 /* FP32 levels of at most this many cells (tx*ty*tz), FP64
                                    levels of at most 1/16 of it, run in the coarse-level
-                                   engine; 0 turns the engine off (default 20000) */
+                                   engine, or in the coarse tail where they fit it (see
+                                   CFMG_OPT_SMALL_SMOOTH); FP32 2D levels beyond the tail that have
+                                   blocked passes take those. 0 turns both off (default 20000) */
 #define CFMG_OPT_COARSEST_FP64 2 /* mixed form, coarsest-level smoothing in FP64: -1 (default) when the
                                     coarsest level holds at most 1/16 of CFMG_OPT_ENGINE_CELLS cells,
                                     0 never (FP32), 1 always */
@@ -134,7 +136,11 @@ extern "C" {
 #define CFMG_OPT_SMALL_SMOOTH 11 /* closed topology, 5-, 2D 9- and 3D 7-point operators: a smoothing
                                      call of at least this many pairs (default 4: the coarsest solve) on
                                      a level whose x, y, b and omega*idiag fit 200 KB runs as one block in
-                                     shared memory; 0 never (separate sweeps). The same bits. */
+                                     shared memory; 0 never (separate sweeps). The same bits. With a
+                                     value > 0 every operator of a cycle below the level whose arrays fit
+                                     one block's shared memory (all operators and topologies; FP64 levels
+                                     up to 6/5 of their engine threshold) runs in one launch there; with 0
+                                     they are Ops of the cluster engine. Same values either way. */
 #define CFMG_OPT_SKIP_DRY 10 /* mixed form, closed topology: 1 (default) passes skip groups of cells
                                that are all dry (their FP32 fields hold +0 and stay +0): the FP32
                                prolongation's parents, the strip residual's tasks; for the 3D 7-point
