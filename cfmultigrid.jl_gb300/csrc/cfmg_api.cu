@@ -1362,13 +1362,13 @@ int resid_kind(const cfmg_handle* h) {
 int prepare_int(cfmg_handle* h) {
   h->int_ok = false;
   const int kind = resid_kind(h);
-  if (!fused_ok(h) || kind == OPK_RESID19) return CFMG_OK;
+  if (!fused_ok(h)) return CFMG_OK;
   const Level& l1 = h->lv[0];
   if (!h->dq) CUDA_OK(h, cudaMalloc((void**)&h->dq, l1.len));
   int* ok = (int*)h->partials;  // scratch
   const int one = 1;
   CUDA_OK(h, cudaMemcpyAsync(ok, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
-  launch_make_dq(l1.diag, l1.msk, kind == OPK_RESID9 ? 4.0 : 1.0, h->dq, (long long)l1.len, ok, h->stream);
+  launch_make_dq(l1.diag, l1.msk, kind == OPK_RESID9 || kind == OPK_RESID19 ? 4.0 : 1.0, h->dq, (long long)l1.len, ok, h->stream);
   {
     const long long ns = resid_sflag_size(kind, geom(l1), interior(l1));
     if (ns > 0) {
@@ -1612,7 +1612,9 @@ int fused_residual(cfmg_handle* h) {
                       launch_resid_int3d(l1.x, l1.b, h->dqp, g, bx, h->dscal, l1.b32, r32, neumann, h->partials,
                                          h->stream, h->r3_rows, h->dry_on ? h->tcol : nullptr);
       h->r3_ran |= r3;
-      if (!r3 && !launch_resid_int2d(kind, l1.x, l1.b, h->dq, g, bx, h->dscal, l1.b32, r32, neumann, h->partials,
+      if (kind == OPK_RESID19)
+        launch_resid_int19(l1.x, l1.b, h->dq, g, bx, h->dscal, l1.b32, r32, neumann, h->partials, h->stream);
+      else if (!r3 && !launch_resid_int2d(kind, l1.x, l1.b, h->dq, g, bx, h->dscal, l1.b32, r32, neumann, h->partials,
                                      h->stream, h->dry_on ? h->sflag : nullptr))
         launch_resid_int(kind, l1.x, l1.b, h->dq, g, bx, lo, n, h->dscal, l1.b32, r32, neumann, h->partials,
                          h->stream);

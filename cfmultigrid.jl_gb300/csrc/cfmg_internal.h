@@ -441,7 +441,7 @@ void launch_fused_final(const double* partials, double* ds, const double* normb,
 void launch_rhs32_mean(const double* r, const uint8_t* m, const double* mean_scale, float* b32, float* r32,
                        long long n, cudaStream_t s);
 void launch_update_scaled(double* x, const float* e, const double* iscale, long long n, cudaStream_t s);
-// integer form of the fused pass (kinds 5-, 7- and 9-point)
+// integer form of the fused pass (kinds 5-, 7- and 9-point; 19-point: launch_resid_int19)
 void launch_resid_int(int kind, const double* x, const double* b, const int8_t* dq, const Geom& g, const Box& bx,
                       long long lo, long long n, const double* ds, float* b32, float* r32, bool neumann,
                       double* partials, cudaStream_t s);
@@ -459,6 +459,9 @@ bool launch_resid_int2d(int kind, const double* x, const double* b, const int8_t
                         const uint8_t* sflag = nullptr);
 long long resid_sflag_size(int kind, const Geom& g, const Box& bx);
 void launch_make_sflag(int kind, const uint8_t* m, uint8_t* sflag, const Geom& g, const Box& bx, cudaStream_t s);
+// 3D 19-point form (grid one bit coarser: see k_mixed.cu)
+void launch_resid_int19(const double* x, const double* b, const int8_t* dq, const Geom& g, const Box& bx,
+                        const double* ds, float* b32, float* r32, bool neumann, double* partials, cudaStream_t s);
 // 3D 7-point form with TMA-staged planes (k_resid3d.cu). dqp: dq with rows
 // padded to txp = dq_pitch(tx) bytes (launch_pad_dq). false: not applicable
 // (odd tx, misaligned arrays, no tensor-map encoder): use launch_resid_int2d.

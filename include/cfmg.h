@@ -109,8 +109,8 @@ extern "C" {
                                         packed form, 1 one column per thread; 4 as 3, plus streaming passes
                                         for 3D 7-point levels and the 3D 19-point pair in one pass; 0: one
                                         kernel per sweep. All give the same bits. */
-#define CFMG_OPT_INT_RESIDUAL 3 /* mixed form, closed topology, 5-, 7- and 2D 9-point operators: 1
-                                   (default) computes the level-1 residual exactly in 64-bit fixed point
+#define CFMG_OPT_INT_RESIDUAL 3 /* mixed form, closed topology, 5-, 7-, 2D 9- and 3D 19-point
+                                   operators: 1 (default) computes the level-1 residual exactly in 64-bit fixed point
                                    on the integer pipes; 0 in FP64 arithmetic */
 #define CFMG_OPT_HOST_LOOP 4 /* cfmg_solve: 0 (default) runs the whole loop as one graph launch (a
                                 `while` node); 1 launches one graph per iteration from the host, which
