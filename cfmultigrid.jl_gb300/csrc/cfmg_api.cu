@@ -23,6 +23,7 @@ struct cfmg_handle {
   std::vector<Level> lv;  // lv[0] is level 1
   int device = 0;
   cudaStream_t own_stream = nullptr;
+  cudaStream_t up_stream = nullptr;  // program uploads (upload_program)
   cudaStream_t stream = nullptr;
   void* arena = nullptr;
   size_t arena_bytes = 0;
@@ -364,6 +365,19 @@ bool in_tail(const cfmg_handle* h, int lev, int prec) {
   return !h->record && h->engine_on && h->tail_from[prec] > 0 && lev >= h->tail_from[prec];
 }
 
+// Copies a program into its device store, complete on return: allowed while
+// the handle's stream is being captured in relaxed mode, and never over a
+// program that a graph refers to. A plain cudaMemcpy from pageable memory may
+// return before its bytes are on the device, and nothing orders it before a
+// launch on the handle's non-blocking stream: a program then ran as the zeros
+// of the empty store.
+int upload_program(cfmg_handle* h, void* dst, const void* src, size_t bytes) {
+  if (!h->up_stream) CUDA_OK(h, cudaStreamCreateWithFlags(&h->up_stream, cudaStreamNonBlocking));
+  CUDA_OK(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->up_stream));
+  CUDA_OK(h, cudaStreamSynchronize(h->up_stream));
+  return CFMG_OK;
+}
+
 // Builds the pending Ops into tail programs and launches them: pairs of
 // sweeps become smoothing calls, every array they touch is staged in shared
 // memory, the smoothing arrays first, then the others while they fit (those
@@ -592,8 +606,7 @@ int flush_tail(cfmg_handle* h, bool& done) {
       off = it->second;
     } else {
       if (h->tail_used + bytes > h->tail_cap) return CFMG_OK;
-      // synchronous, and never over a program that a graph refers to (as in flush)
-      CUDA_OK(h, cudaMemcpy(h->tail_pool + h->tail_used, key.data(), bytes, cudaMemcpyHostToDevice));
+      TRY(upload_program(h, h->tail_pool + h->tail_used, key.data(), (size_t)bytes));
       off = h->tail_used;
       h->tail_used += (bytes + 255) & ~(size_t)255;
       h->tail_cache.emplace(std::move(key), off);
@@ -653,10 +666,7 @@ int flush(cfmg_handle* h) {
   if (it != h->prog_cache.end()) {
     off = it->second;
   } else if (h->pool_used + n <= h->pool_cap) {
-    // synchronous upload; allowed while the stream is being captured in
-    // relaxed mode, and never overwrites a program a graph refers to
-    CUDA_OK(h, cudaMemcpy(h->prog_pool + h->pool_used, h->pending.data(), (size_t)n * sizeof(Op),
-                          cudaMemcpyHostToDevice));
+    TRY(upload_program(h, h->prog_pool + h->pool_used, h->pending.data(), (size_t)n * sizeof(Op)));
     off = h->pool_used;
     h->pool_used += n;
     h->prog_cache.emplace(std::move(key), off);
@@ -2141,6 +2151,7 @@ int cfmg_destroy(cfmg_handle* h) {
   if (h->arena) cudaFree(h->arena);
   if (h->hscal) cudaFreeHost(h->hscal);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
+  if (h->up_stream) cudaStreamDestroy(h->up_stream);
   delete h;
   return CFMG_OK;
 }
