@@ -40,6 +40,7 @@ struct cfmg_handle {
   double* dhist = nullptr;  // device residual history (maxite + 1)
   long long launches = 0;      // kernels launched (graph replays count every kernel node)
   bool capturing = false;
+  const cfmg::LoopTest* loop = nullptr;  // set while the device loop's iteration is captured
   // device-time profile of one kernel class on one level (cfmg_profile)
   int prof_cls = -1, prof_lev = 0, prof_prec = 0;
   std::vector<cudaEvent_t> ev_pool;
@@ -1250,12 +1251,15 @@ int cycle_t(cfmg_handle* h, int kind, bool x1_zero = false) {
   return flush(h);
 }
 
+unsigned* norm_counter(cfmg_handle* h) { return reinterpret_cast<unsigned*>(h->dscal + S_CNT); }
+
 // norm of one FP64 field into dscal[S_NORM] (and dscal[S_RES] when normb given)
 int norm_dev(cfmg_handle* h, int lev, const double* x, const double* normb, int kind) {
   TRY(flush(h));
   const Level& l = h->lv[lev - 1];
-  Launch k(h, CFMG_K_NORM, lev, CFMG_FP64, 2);
-  launch_norm<double>(x, l.msk, l.len, h->partials, h->dscal + S_NORM, normb, kind, h->stream);
+  Launch k(h, CFMG_K_NORM, lev, CFMG_FP64);
+  launch_norm<double>(x, l.msk, l.len, h->partials, norm_counter(h), h->dscal + S_NORM, normb, kind, h->stream,
+                      normb ? h->loop : nullptr);
   LAUNCH_OK(h);
   return CFMG_OK;
 }
@@ -1452,7 +1456,8 @@ int prepare_mixed(cfmg_handle* h) {
   // number of wet cells of level 1 (for the residual scaling)
   const Level& l1 = h->lv[0];
   launch_fill_f64(l1.y, 1.0, l1.len, h->stream);
-  launch_norm<double>(l1.y, l1.msk, l1.len, h->partials, h->dscal + S_TMP0, nullptr, CFMG_NORM_L2, h->stream);
+  launch_norm<double>(l1.y, l1.msk, l1.len, h->partials, norm_counter(h), h->dscal + S_TMP0, nullptr, CFMG_NORM_L2,
+                      h->stream);
   CUDA_OK(h, cudaMemcpyAsync(h->dscal + S_NWET, h->dscal + S_TMP0, sizeof(double), cudaMemcpyDeviceToDevice,
                              h->stream));
   CUDA_OK(h, cudaMemsetAsync(l1.y, 0, l1.len * sizeof(double), h->stream));
@@ -1572,7 +1577,8 @@ __global__ void k_kappa_grad(const double* lam, const double* x, const uint8_t* 
 int count_wet(cfmg_handle* h) {
   const Level& l1 = h->lv[0];
   launch_fill_f64(l1.y, 1.0, l1.len, h->stream);
-  launch_norm<double>(l1.y, l1.msk, l1.len, h->partials, h->dscal + S_TMP0, nullptr, CFMG_NORM_L2, h->stream);
+  launch_norm<double>(l1.y, l1.msk, l1.len, h->partials, norm_counter(h), h->dscal + S_TMP0, nullptr, CFMG_NORM_L2,
+                      h->stream);
   CUDA_OK(h, cudaMemcpyAsync(h->dscal + S_NWET, h->dscal + S_TMP0, sizeof(double), cudaMemcpyDeviceToDevice,
                              h->stream));
   CUDA_OK(h, cudaMemsetAsync(l1.y, 0, l1.len * sizeof(double), h->stream));
@@ -1629,7 +1635,7 @@ int fused_residual(cfmg_handle* h) {
         launch_resid_int(kind, l1.x, l1.b, h->dq, g, bx, lo, n, h->dscal, l1.b32, r32, neumann, h->partials,
                          h->stream);
       launch_fused_final(h->partials, h->dscal, h->dscal + S_NORMB, neumann ? h->dscal + S_NWET : nullptr,
-                         h->d.norm_kind, h->stream);
+                         h->d.norm_kind, h->stream, h->loop);
     }
     if (neumann) {
       Launch k(h, CFMG_K_CONVERT, 1, CFMG_MIXED);
@@ -1644,7 +1650,7 @@ int fused_residual(cfmg_handle* h) {
     launch_resid_fused(kind, l1.r, l1.x, l1.b, l1.diag, l1.msk, g, bx, lo, n, h->dscal + S_NEXT, l1.b32, l1.r32,
                        neumann, h->partials, h->stream);
     launch_fused_final(h->partials, h->dscal, h->dscal + S_NORMB, neumann ? h->dscal + S_NWET : nullptr,
-                       h->d.norm_kind, h->stream);
+                       h->d.norm_kind, h->stream, h->loop);
   }
   if (neumann) {
     Launch k(h, CFMG_K_CONVERT, 1, CFMG_MIXED);
@@ -1740,7 +1746,9 @@ int iteration(cfmg_handle* h, int prec, int kind, int norm_kind) {
     TRY(cycle_t<double>(h, kind));
     TRY(normresidual_dev(h, norm_kind));
   }
-  CUDA_OK(h, cudaMemcpyAsync(h->hscal, h->dscal, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  // the device loop's host reads the scalars once, after the last iteration
+  if (!h->loop)
+    CUDA_OK(h, cudaMemcpyAsync(h->hscal, h->dscal, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   return CFMG_OK;
 }
 
@@ -1782,22 +1790,6 @@ void drop_graphs(cfmg_handle* h) {
         }
 }
 
-// The solve! loop on the device (src/gmg_solver.jl:29-39): hist[nite] = res
-// after every residual, and another iteration while res > tol and
-// nite < maxite (the count moves before the iteration runs).
-__global__ void k_loop_test(cudaGraphConditionalHandle hc, double* ds, double* hist, double tol, int maxite,
-                            int first) {
-  if (first) ds[S_NITE] = 0.0;
-  const double res = ds[S_RES];
-  const int nite = (int)ds[S_NITE];
-  hist[nite] = res;
-  // a NaN or Inf in b or in the residual ends the loop (reported as
-  // CFMG_ERR_NONFINITE): an infinite |b| would otherwise give res = 0
-  const bool more = isfinite(ds[S_NORMB]) && isfinite(res) && res > tol && nite < maxite;
-  if (more) ds[S_NITE] = (double)(nite + 1);
-  cudaGraphSetConditional(hc, more ? 1u : 0u);
-}
-
 int get_solve_graph(cfmg_handle* h, int prec, int kind, int norm_kind, cudaGraphExec_t* out) {
   cudaGraphExec_t& ge = h->sgraph[prec][kind];
   if (ge) {
@@ -1818,7 +1810,8 @@ int get_solve_graph(cfmg_handle* h, int prec, int kind, int norm_kind, cudaGraph
   if ((e = cudaStreamBeginCaptureToGraph(h->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed)) !=
       cudaSuccess)
     return bail("solve capture");
-  k_loop_test<<<1, 1, 0, h->stream>>>(hc, h->dscal, h->dhist, h->d.tol, h->d.maxite, 1);
+  const LoopTest lt{hc, h->dscal, h->dhist, h->d.tol, h->d.maxite, 1};
+  launch_loop_start(lt, h->stream);
   if ((e = cudaStreamEndCapture(h->stream, &g)) != cudaSuccess) return bail("solve capture");
   cudaGraphNode_t first = nullptr;
   size_t nn = 1;
@@ -1836,11 +1829,12 @@ int get_solve_graph(cfmg_handle* h, int prec, int kind, int norm_kind, cudaGraph
     return bail("solve capture");
   const long long before = h->launches;
   h->capturing = true;
+  h->loop = &lt;  // the iteration's norm tests the stopping rule
   int rc = iteration(h, prec, kind, norm_kind);
+  h->loop = nullptr;
   h->capturing = false;
   h->graph_launches[prec][kind] = h->launches - before;
   h->launches = before;
-  if (rc == CFMG_OK) k_loop_test<<<1, 1, 0, h->stream>>>(hc, h->dscal, h->dhist, h->d.tol, h->d.maxite, 0);
   e = cudaStreamEndCapture(h->stream, &body);
   if (rc != CFMG_OK) {
     cudaGraphDestroy(g);
@@ -2412,8 +2406,9 @@ int cfmg_solve(cfmg_handle* h, double* res_out, int* nite_out, double* history) 
   const Level& l1 = h->lv[0];
   TRY(flush(h));
   {
-    Launch k(h, CFMG_K_NORM, 1, CFMG_FP64, 2);
-    launch_norm<double>(l1.b, l1.msk, l1.len, h->partials, h->dscal + S_NORMB, nullptr, d.norm_kind, h->stream);
+    Launch k(h, CFMG_K_NORM, 1, CFMG_FP64);
+    launch_norm<double>(l1.b, l1.msk, l1.len, h->partials, norm_counter(h), h->dscal + S_NORMB, nullptr, d.norm_kind,
+                        h->stream);
   }
   LAUNCH_OK(h);
   if (prec == CFMG_MIXED && fused_ok(h)) {
@@ -2441,7 +2436,7 @@ int cfmg_solve(cfmg_handle* h, double* res_out, int* nite_out, double* history) 
     CUDA_OK(h, cudaMemcpyAsync(h->hscal, h->dscal, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     TRY(sync(h));
     const int nite = (int)h->hscal[S_NITE];
-    h->launches += 2 + (long long)nite * (h->graph_launches[prec][d.cycle] + 1);
+    h->launches += 1 + (long long)nite * h->graph_launches[prec][d.cycle];
     if (history)
       CUDA_OK(h, cudaMemcpy(history, h->dhist, sizeof(double) * (size_t)(nite + 1), cudaMemcpyDeviceToHost));
     *res_out = h->hscal[S_RES];

@@ -172,9 +172,18 @@ void launch_fill_xperio(T* x, const Geom& g, cudaStream_t s);
 // array into out[0], with 0 -> 1 for the reference rule
 // (src/operators_at_level.jl:21-23). When normb != nullptr, out[1] is the
 // residual ratio: sum/normb (CFMG_NORM_REF_SQUARED) or sqrt(sum/normb) (L2).
+// counter: one zeroed unsigned, 0 again afterwards. lt: the solve loop's test of the stopping rule.
+struct LoopTest {
+  cudaGraphConditionalHandle hc;
+  double *ds, *hist;  // the handle's device scalars, the residual history
+  double tol;
+  int maxite, on;
+};
 template <class T>
-void launch_norm(const T* x, const uint8_t* msk, size_t n, double* partials, double* out, const double* normb,
-                 int norm_kind, cudaStream_t s);
+void launch_norm(const T* x, const uint8_t* msk, size_t n, double* partials, unsigned* counter, double* out,
+                 const double* normb, int norm_kind, cudaStream_t s, const LoopTest* lt = nullptr);
+// before the loop: hist[0] and the test of the first residual (ds[S_RES])
+void launch_loop_start(const LoopTest& lt, cudaStream_t s);
 constexpr int kNormParts = 1024;
 // the handle's partial-sum scratch: two sums per block for the fused
 // residual pass of the mixed loop (k_mixed.cu), one for the norms
@@ -430,14 +439,16 @@ enum Scal { S_NORM = 0, S_RES = 1, S_NORMB = 2, S_NWET = 3, S_SCALE = 4, S_MEAN 
             S_NEXT = 8, S_CUR = 9, S_ICUR = 10, S_MEAN2 = 11, S_MAXX = 12, S_MAXB = 13, S_NITE = 14,
             S_SHIFT = 15, S_MAXO = 16,
             // 1 after a bounded wait in a kernel ran out (k_resid3d.cu); the solve reports it
-            S_FAULT = 17, S_COUNT = 18 };
+            S_FAULT = 17,
+            S_CNT = 18,  // launch_norm's block counter (an unsigned, 0 between launches)
+            S_COUNT = 19 };
 
 // fused FP64 steps of the mixed loop (k_mixed.cu)
 void launch_resid_fused(int kind, double* r, const double* x, const double* b, const double* d, const uint8_t* m,
                         const Geom& g, const Box& bx, long long lo, long long n, const double* scale, float* b32,
                         float* r32, bool neumann, double* partials, cudaStream_t s);
 void launch_fused_final(const double* partials, double* ds, const double* normb, const double* nwet, int norm_kind,
-                        cudaStream_t s);
+                        cudaStream_t s, const LoopTest* lt = nullptr);
 void launch_rhs32_mean(const double* r, const uint8_t* m, const double* mean_scale, float* b32, float* r32,
                        long long n, cudaStream_t s);
 void launch_update_scaled(double* x, const float* e, const double* iscale, long long n, cudaStream_t s);

@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_fused(double* __restrict__
 // applied (S_NEXT on entry) becomes S_CUR / S_ICUR, and the next scale
 // 2^-round(log2(rms)) goes to S_NEXT (powers of two, exact both ways).
 __global__ void __launch_bounds__(kMxParts) k_fused_final(const double* __restrict__ partials, double* ds,
-                                                          const double* normb, const double* nwet, int norm_kind) {
+                                                          const double* normb, const double* nwet, int norm_kind,
+                                                          LoopTest lt) {
   dep_wait();
   __shared__ double a[kMxParts], c[kMxParts];
   a[threadIdx.x] = partials[threadIdx.x];
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(kMxParts) k_fused_final(const double* __restri
     ds[S_MAXX] = ds[S_MAXO];  // the next update collects max |x| from max |x| outside U
     // the wet mean in units of the right-hand side, as an FP32 value
     *reinterpret_cast<float*>(ds + S_SHIFT) = (float)(ds[S_MEAN2] * used);
+    if (lt.on) loop_test(lt, ds[S_RES], *normb);
   }
 }
 
@@ -971,8 +973,8 @@ void launch_resid_fused(int kind, double* r, const double* x, const double* b, c
 }
 
 void launch_fused_final(const double* partials, double* ds, const double* normb, const double* nwet, int norm_kind,
-                        cudaStream_t s) {
-  launch_dep(k_fused_final, 1, kMxParts, 0, s, partials, ds, normb, nwet, norm_kind);
+                        cudaStream_t s, const LoopTest* lt) {
+  launch_dep(k_fused_final, 1, kMxParts, 0, s, partials, ds, normb, nwet, norm_kind, lt ? *lt : LoopTest{});
 }
 
 void launch_rhs32_mean(const double* r, const uint8_t* m, const double* mean_scale, float* b32, float* r32,

@@ -501,56 +501,82 @@ __global__ void __launch_bounds__(kThreads) k_fill_xperio(T* __restrict__ x, int
 }
 
 // ------------------------------------------------------------------- norm
-// Deterministic two-stage reduction: block b sums the elements b, b+P,
-// b+2P, ... strided by the whole grid (fixed grid of kNormParts blocks),
-// then one block adds the kNormParts partials in a fixed tree.
+// Deterministic two-stage reduction in one launch: block b of (up to)
+// kNormParts sums the elements b, b+P, b+2P, ... strided by the whole grid of
+// kNormParts blocks; the block that finishes last (a counter, back at 0 when
+// it is done) adds the kNormParts partials in a fixed tree, so the sum does
+// not depend on which block that is. Fields of fewer than kNormParts blocks'
+// cells launch only the blocks that hold some; the other partials are 0.
+// With `lt` (the solve loop's last kernel) it also tests the stopping rule.
+// As two launches and a test kernel these were 3 of the 18 nodes of a 64^2
+// FP64 solve's iteration (see launch_norm).
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_norm_partial(const T* __restrict__ x, const uint8_t* __restrict__ m,
-                                                           long long n, double* __restrict__ partials) {
+__global__ void __launch_bounds__(kThreads) k_norm(const T* __restrict__ x, const uint8_t* __restrict__ m, long long n,
+                                                   double* __restrict__ partials, unsigned* counter, double* out,
+                                                   const double* normb, int norm_kind, LoopTest lt) {
   dep_wait();
   double s = 0.0;
-  for (long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x; I < n; I += (long long)gridDim.x * blockDim.x) {
-    uint8_t mm = m[I];
+  const long long st = (long long)kNormParts * kThreads;
+  auto add = [&](uint8_t mm, T xv) {
     if (mm) {
-      double v = (double)x[I];
+      const double v = (double)xv;
       s = (mm == 1) ? __fma_rn(v, v, s) : __dadd_rn(s, __dmul_rn((double)mm, __dmul_rn(v, v)));
     }
+  };
+  long long I = (long long)blockIdx.x * kThreads + threadIdx.x;
+  for (; I + 3 * st < n; I += 4 * st) {  // four elements' loads in flight, added in their order
+    const uint8_t m0 = m[I], m1 = m[I + st], m2 = m[I + 2 * st], m3 = m[I + 3 * st];
+    const T x0 = x[I], x1 = x[I + st], x2 = x[I + 2 * st], x3 = x[I + 3 * st];
+    add(m0, x0);
+    add(m1, x1);
+    add(m2, x2);
+    add(m3, x3);
   }
+  for (; I < n; I += st) add(m[I], x[I]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_down_sync(0xffffffffu, s, o));
   __shared__ double ws[kThreads / 32];
+  __shared__ bool last;
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x < 32) {
     s = threadIdx.x < kThreads / 32 ? ws[threadIdx.x] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_down_sync(0xffffffffu, s, o));
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (threadIdx.x == 0) {
+      partials[blockIdx.x] = s;
+      __threadfence();
+      last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
+    }
   }
-}
-
-__global__ void __launch_bounds__(kNormParts) k_norm_final(const double* __restrict__ partials, double* out,
-                                                           const double* normb, int norm_kind) {
-  dep_wait();
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
   __shared__ double sh[kNormParts];
-  sh[threadIdx.x] = partials[threadIdx.x];
+  for (int t = threadIdx.x; t < kNormParts; t += kThreads) sh[t] = t < (int)gridDim.x ? __ldcg(partials + t) : 0.0;
   __syncthreads();
   for (int w = kNormParts / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) sh[threadIdx.x] = __dadd_rn(sh[threadIdx.x], sh[threadIdx.x + w]);
+    for (int t = threadIdx.x; t < w; t += kThreads) sh[t] = __dadd_rn(sh[t], sh[t + w]);
     __syncthreads();
   }
   if (threadIdx.x == 0) {
     double sum = sh[0];
-    if (norm_kind == CFMG_NORM_REF_SQUARED) {
-      if (sum == 0.0) sum = 1.0;
-      out[0] = sum;
-      if (normb) out[1] = (*normb > 0.0) ? sum / *normb : 0.0;
-    } else {
-      out[0] = sum;
-      if (normb) out[1] = (*normb > 0.0) ? sqrt(sum / *normb) : 0.0;
+    if (norm_kind == CFMG_NORM_REF_SQUARED && sum == 0.0) sum = 1.0;
+    out[0] = sum;
+    if (normb) {
+      const double nb = *normb;
+      const double q = nb > 0.0 ? sum / nb : 0.0;
+      const double res = norm_kind == CFMG_NORM_REF_SQUARED ? q : sqrt(q);
+      out[1] = res;
+      if (lt.on) loop_test(lt, res, nb);
     }
   }
 }
+__global__ void k_loop_start(LoopTest lt) {
+  lt.ds[S_NITE] = 0.0;
+  loop_test(lt, lt.ds[S_RES], lt.ds[S_NORMB]);
+}
+void launch_loop_start(const LoopTest& lt, cudaStream_t s) { k_loop_start<<<1, 1, 0, s>>>(lt); }
 
 // --------------------------------------------------------------- launchers
 template <class T>
@@ -891,10 +917,11 @@ void launch_fill_xperio(T* x, const Geom& g, cudaStream_t s) {
   launch_dep(k_fill_xperio<T>, nblocks(nlines), kThreads, 0, s, x, g.tx, g.nh, nlines);
 }
 template <class T>
-void launch_norm(const T* x, const uint8_t* m, size_t n, double* partials, double* out, const double* normb,
-                 int norm_kind, cudaStream_t s) {
-  launch_dep(k_norm_partial<T>, kNormParts, kThreads, 0, s, x, m, (long long)n, partials);
-  launch_dep(k_norm_final, 1, kNormParts, 0, s, partials, out, normb, norm_kind);
+void launch_norm(const T* x, const uint8_t* m, size_t n, double* partials, unsigned* counter, double* out,
+                 const double* normb, int norm_kind, cudaStream_t s, const LoopTest* lt) {
+  const long long nb = ((long long)n + kThreads - 1) / kThreads;
+  launch_dep(k_norm<T>, (unsigned)(nb < kNormParts ? nb : kNormParts), kThreads, 0, s, x, m, (long long)n, partials,
+             counter, out, normb, norm_kind, lt ? *lt : LoopTest{});
 }
 
 #define CFMG_INST(T)                                                                                             \
@@ -919,7 +946,8 @@ void launch_norm(const T* x, const uint8_t* m, size_t n, double* partials, doubl
   template void launch_prolong<T>(int, T*, const T*, const T*, const Geom&, const Geom&, int, int, int, int, int, \
                                   bool, cudaStream_t, const uint8_t*);                                           \
   template void launch_fill_xperio<T>(T*, const Geom&, cudaStream_t);                                            \
-  template void launch_norm<T>(const T*, const uint8_t*, size_t, double*, double*, const double*, int, cudaStream_t);
+  template void launch_norm<T>(const T*, const uint8_t*, size_t, double*, unsigned*, double*, const double*, int,    \
+                               cudaStream_t, const LoopTest*);
 
 CFMG_INST(double)
 CFMG_INST(float)

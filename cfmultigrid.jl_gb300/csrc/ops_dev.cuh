@@ -439,6 +439,19 @@ __device__ __forceinline__ int pow2_exponent(double v) {
   return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffULL) - 1023;
 }
 
+// The solve! loop's test (src/gmg_solver.jl:29-39): hist[nite] = res after
+// every residual, and another iteration while res > tol and nite < maxite
+// (the count moves before the iteration runs).
+__device__ __forceinline__ void loop_test(const LoopTest& lt, double res, double normb) {
+  const int nite = (int)lt.ds[S_NITE];
+  lt.hist[nite] = res;
+  // a NaN or Inf in b or in the residual ends the loop (reported as
+  // CFMG_ERR_NONFINITE): an infinite |b| would otherwise give res = 0
+  const bool more = isfinite(normb) && isfinite(res) && res > lt.tol && nite < lt.maxite;
+  if (more) lt.ds[S_NITE] = (double)(nite + 1);
+  cudaGraphSetConditional(lt.hc, more ? 1u : 0u);
+}
+
 // ------------------------------------------------------------------ halo
 // fill! for :xperio (src/halo.jl:6-9) on one (j,k) line. Each statement's
 // right-hand columns are read before any is written, as Julia's sliced
