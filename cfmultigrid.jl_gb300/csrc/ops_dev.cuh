@@ -215,6 +215,101 @@ __device__ __forceinline__ void d_residvc(T* r, const T* x, const T* b, const T*
   r[I] = v_residvc(x, b, d, cE, cN, m, n1, I);
 }
 
+// ------------------------------------------------ FP64 on zero operands
+// The FP64 pipe bounds every FP64 operator (one warp instruction in 76 clocks
+// per quarter of an SM), and over land and halo its operands are zeros. When
+// a whole warp's are, the standalone kernels take the result from the sign
+// bits instead: IEEE sums of zeros are +0 unless every term is -0. These
+// return false (the caller computes) unless every operand is a zero and the
+// coefficients are finite; zero_sweep also needs omega*idiag = +0 and
+// 1-omega >= +0, as dry cells have for omega <= 1.
+struct ZeroAcc {
+  unsigned o = 0, l = 0, a = ~0u;
+  __device__ __forceinline__ void add(double v) {
+    const unsigned h = (unsigned)__double2hiint(v);
+    o |= h;
+    l |= (unsigned)__double2loint(v);
+    a &= h;
+  }
+  __device__ __forceinline__ bool zero() const { return ((o << 1) | l) == 0u; }
+  __device__ __forceinline__ bool neg() const { return (a >> 31) != 0u; }  // the sum of the zeros is -0
+};
+__device__ __forceinline__ bool is_neg(double v) { return __double2hiint(v) < 0; }
+__device__ __forceinline__ bool is_fin(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+__device__ __forceinline__ double signed_zero(bool neg) { return neg ? -0.0 : 0.0; }
+enum ZeroStencil { ZS_5, ZS_7, ZS_9, ZS_19, ZS_VC };
+// faces (and for the 9- and 19-point operators diagonals) of cell I; false when a value is not a zero
+template <int ST>
+__device__ __forceinline__ bool zero_nb(const double* x, const double* cE, const double* cN, long long I, long long n1,
+                                        long long n2, bool& fneg, bool& dneg) {
+  ZeroAcc f, d;
+  f.add(x[I - 1]);
+  f.add(x[I + 1]);
+  f.add(x[I - n1]);
+  f.add(x[I + n1]);
+  bool ok = true;
+  if (ST == ZS_7 || ST == ZS_19) {
+    f.add(x[I - n2]);
+    f.add(x[I + n2]);
+  }
+  if (ST == ZS_9 || ST == ZS_19) {
+    d.add(x[I - 1 - n1]);
+    d.add(x[I + 1 - n1]);
+    d.add(x[I - 1 + n1]);
+    d.add(x[I + 1 + n1]);
+  }
+  if (ST == ZS_19) {
+    d.add(x[I - 1 - n2]);
+    d.add(x[I + 1 - n2]);
+    d.add(x[I - 1 + n2]);
+    d.add(x[I + 1 + n2]);
+    d.add(x[I - n1 - n2]);
+    d.add(x[I + n1 - n2]);
+    d.add(x[I - n1 + n2]);
+    d.add(x[I + n1 + n2]);
+  }
+  if (ST == ZS_VC) {  // products with face coefficients >= +0 keep the sign
+    const double c[4] = {cE[I - 1], cE[I], cN[I - n1], cN[I]};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ok = ok && !is_neg(c[q]) && is_fin(c[q]);
+  }
+  fneg = f.neg();
+  dneg = d.neg();
+  return ok && f.zero() && (ST == ZS_9 || ST == ZS_19 ? d.zero() : true);
+}
+template <int ST>
+__device__ __forceinline__ bool zero_sweep(const double* x, const double* b, const double* w, const double* cE,
+                                           const double* cN, double cff, long long n1, long long n2, long long I,
+                                           double& out) {
+  bool fneg, dneg;
+  ZeroAcc c;
+  const double xv = x[I], bv = b[I];
+  c.add(xv);
+  c.add(bv);
+  if (!zero_nb<ST>(x, cE, cN, I, n1, n2, fneg, dneg) || !c.zero() || __double_as_longlong(w[I]) != 0ll ||
+      !(cff >= 0.0) || is_neg(cff))
+    return false;
+  // b - faces (- diagonals) is -0 only from -0 minus sums that are all +0
+  bool tneg = is_neg(bv) && !fneg;
+  if (ST == ZS_9 || ST == ZS_19) tneg = tneg && !dneg;
+  out = signed_zero(is_neg(xv) && !tneg);
+  return true;
+}
+template <int ST>
+__device__ __forceinline__ bool zero_resid(const double* x, const double* b, const double* d, const double* cE,
+                                           const double* cN, long long n1, long long n2, long long I, double& out) {
+  bool fneg, dneg;
+  ZeroAcc c;
+  const double xv = x[I], bv = b[I], dv = d[I];
+  c.add(xv);
+  c.add(bv);
+  if (!zero_nb<ST>(x, cE, cN, I, n1, n2, fneg, dneg) || !c.zero() || !is_fin(dv)) return false;
+  bool v = (is_neg(dv) != is_neg(xv)) && is_neg(bv) && !fneg;  // (d x + b) - faces
+  if (ST == ZS_9 || ST == ZS_19) v = v && !dneg;
+  out = signed_zero(v);  // whatever the mask: it keeps the sign of a zero
+  return true;
+}
+
 // ---------------------------------------------------------- restriction
 // Coarse interior cell (ii, jj, kk) of kind 0 centres 2D (rcloop2d!,
 // src/RP_on_centers.jl:117-133), 1 centres 3D (rcloop3d!, :5-23),
@@ -279,6 +374,27 @@ __device__ __forceinline__ void d_restrict(const T* x, T* xc, const T* coef, con
   long long C;
   const T v = v_restrict<T, KIND>(x, coef, gf, gc, ii, jj, kk, C);
   xc[C] = v;
+}
+
+// the restriction of zeros under a finite Rcoef (see ZeroAcc): the fold is -0 only when every child is
+template <int KIND>
+__device__ __forceinline__ bool zero_restrict(const double* x, double coef, const Geom& gf, const Geom& gc, int ii,
+                                              int jj, int kk, double& out) {
+  const int nh = gc.nh;
+  const long long n1 = gf.n1, n2 = gf.n2;
+  const bool t3 = KIND == 1 || KIND == 3;
+  const long long F = lin(gf, c2f(ii, nh), c2f(jj, nh), t3 ? c2f(kk, nh) : kk);
+  ZeroAcc a;
+  constexpr int lo = KIND >= 2 ? -1 : 0;
+#pragma unroll
+  for (int dk = t3 ? lo : 0; dk <= (t3 ? 1 : 0); ++dk)
+#pragma unroll
+    for (int dj = lo; dj <= 1; ++dj)
+#pragma unroll
+      for (int di = lo; di <= 1; ++di) a.add(x[F + di + dj * n1 + dk * n2]);
+  if (!a.zero() || !is_fin(coef)) return false;
+  out = signed_zero(a.neg() != is_neg(coef));
+  return true;
 }
 
 // --------------------------------------------------------- prolongation
@@ -384,6 +500,36 @@ __device__ __forceinline__ void d_prolong(T* xf, const T* x, const T* coef, cons
     s = A::add(s, x111);
     upd(F + 1 + f1 + f2, s);
   }
+}
+
+// FP64 parent whose update changes nothing: its children's Pcoef and fine x
+// are all +0, and every coarse value it reads is finite with room for the
+// weights (below 2^1009), so +0 + 0*v = +0
+template <int KIND>
+__device__ __forceinline__ bool zero_prolong(const double* xf, const double* x, const double* coef, const Geom& gf,
+                                             const Geom& gc, int p, int q, int qk, int kf0) {
+  const int nh = gf.nh;
+  const int i = nh + 1 + 2 * p, j = nh + 1 + 2 * q;
+  const bool t3 = KIND == 1 || KIND == 3;
+  const int k = t3 ? nh + 1 + 2 * qk : kf0 + qk;
+  const long long F = lin(gf, i, j, k), f1 = gf.n1, f2 = gf.n2;
+  unsigned long long o = 0;
+#pragma unroll
+  for (int c = 0; c < (t3 ? 8 : 4); ++c) {
+    const long long Fi = F + (c & 1) + ((c >> 1) & 1) * f1 + (c >> 2) * f2;
+    o |= (unsigned long long)__double_as_longlong(coef[Fi]) | (unsigned long long)__double_as_longlong(xf[Fi]);
+  }
+  if (o) return false;
+  const long long C = lin(gc, f2c(i, nh), f2c(j, nh), t3 ? f2c(k, nh) : k), c1 = gc.n1, c2 = gc.n2;
+  constexpr int lo = KIND < 2 ? -1 : 0;
+  int big = 0;
+#pragma unroll
+  for (int dk = t3 ? lo : 0; dk <= (t3 ? 1 : 0); ++dk)
+#pragma unroll
+    for (int dj = lo; dj <= 1; ++dj)
+#pragma unroll
+      for (int di = lo; di <= 1; ++di) big = max(big, __double2hiint(x[C + di + dj * c1 + dk * c2]) & 0x7fffffff);
+  return big < 0x7f000000;
 }
 
 // ------------------------------------------------------- fixed point
