@@ -698,22 +698,30 @@ __global__ void __launch_bounds__(256) k_sweep7_3d_q(const float* __restrict__ x
 // qact (optional): a quad whose cells are dry in every plane of the run is
 // skipped. In the mixed form's FP32 fields a dry cell holds +0 in x, y and b
 // and has omega*idiag = 0, so the sweep would write +0 over +0 there.
+//
+// run: planes a thread sweeps, kQRun or 1. A run reads each plane once instead
+// of three times but takes its planes one after the other; a level that gives
+// fewer than kQBlocks blocks in runs is bound by that chain of loads, and
+// takes a plane a thread (70 x 70 x 38 and below of a 512 x 512 x 256 solve:
+// 7.4-7.9 -> 4.3-5.1 us a sweep).
 constexpr int kQRun = kQRunPlanes;
+constexpr long long kQBlocks = 4 * 152;
 template <bool ZERO>
 __global__ void __launch_bounds__(256) k_sweep7_3d_q4(const float* __restrict__ x, float* __restrict__ y,
                                                       const float* __restrict__ b, const uint8_t* __restrict__ wq,
                                                       const float* __restrict__ wtab, float cff, long long n1,
-                                                      long long n2, int tz, const uint8_t* __restrict__ qact) {
+                                                      long long n2, int tz, const uint8_t* __restrict__ qact,
+                                                      int run) {
   __shared__ float tab[256];
   dep_wait();
   const long long t = (long long)blockIdx.x * 256 + threadIdx.x;  // quad of the plane
-  const int k0 = 1 + blockIdx.y * kQRun;
-  const bool live = 4 * t < n2 && k0 <= tz - 2 && (!qact || qact[(long long)blockIdx.y * (n2 >> 2) + t]);
+  const int k0 = 1 + blockIdx.y * run;
+  const bool live = 4 * t < n2 && k0 <= tz - 2 && (!qact || qact[(long long)((k0 - 1) / kQRun) * (n2 >> 2) + t]);
   if (!__syncthreads_or(live)) return;  // a block of dry quads reads nothing more
   tab[threadIdx.x] = wtab[threadIdx.x];
   __syncthreads();
   if (!live) return;
-  const int k1 = min(k0 + kQRun, tz - 1);
+  const int k1 = min(k0 + run, tz - 1);
   typedef Ar<float> A;
   long long I = 4 * t + n2 * k0;
   const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -751,11 +759,13 @@ void launch_sweep7_3d_q(const float* x, float* y, const float* b, const uint8_t*
                         const Geom& g, cudaStream_t s, bool x_zero, const uint8_t* qact) {
   if (g.tz < 3) return;
   if (sweep7_quad_ok(g, x, y, b, wq)) {
-    const dim3 grid((unsigned)((g.n2 / 4 + 255) / 256), (unsigned)((g.tz - 2 + kQRun - 1) / kQRun));
+    const long long nb = (g.n2 / 4 + 255) / 256;
+    const int run = nb * ((g.tz - 2 + kQRun - 1) / kQRun) < kQBlocks ? 1 : kQRun;
+    const dim3 grid((unsigned)nb, (unsigned)((g.tz - 2 + run - 1) / run));
     if (x_zero)
-      launch_dep(k_sweep7_3d_q4<true>, grid, 256, 0, s, x, y, b, wq, wtab, cff, g.n1, g.n2, g.tz, qact);
+      launch_dep(k_sweep7_3d_q4<true>, grid, 256, 0, s, x, y, b, wq, wtab, cff, g.n1, g.n2, g.tz, qact, run);
     else
-      launch_dep(k_sweep7_3d_q4<false>, grid, 256, 0, s, x, y, b, wq, wtab, cff, g.n1, g.n2, g.tz, qact);
+      launch_dep(k_sweep7_3d_q4<false>, grid, 256, 0, s, x, y, b, wq, wtab, cff, g.n1, g.n2, g.tz, qact, run);
     return;
   }
   if (x_zero) cudaMemsetAsync(const_cast<float*>(x), 0, (size_t)g.len * sizeof(float), s);  // the one-cell form reads x
@@ -798,12 +808,12 @@ __device__ __forceinline__ float q4at(const float4& v, int c) { return c == 0 ? 
 __global__ void __launch_bounds__(256) k_sweep19_3d_q4(const float* __restrict__ x, float* __restrict__ y,
                                                        const float* __restrict__ b, const float* __restrict__ w,
                                                        float cff, long long n1, long long n2, Box bx, long long q0,
-                                                       long long nq) {
+                                                       long long nq, int run) {
   dep_wait();
   const long long qi = q0 + (long long)blockIdx.x * 256 + threadIdx.x;  // quad of the plane
-  const int k0 = (bx.k0 - 1) + (int)blockIdx.y * kQ19Run;               // 0-based planes k0 .. k1-1
+  const int k0 = (bx.k0 - 1) + (int)blockIdx.y * run;                   // 0-based planes k0 .. k1-1
   if (qi >= q0 + nq || k0 > bx.k1 - 1) return;
-  const int k1 = min(k0 + kQ19Run, bx.k1);
+  const int k1 = min(k0 + run, bx.k1);
   const long long Lp = 4 * qi;
   const int jq = (int)(Lp / n1), iq = (int)(Lp - (long long)jq * n1);
   bool inb[4];
@@ -867,8 +877,10 @@ bool launch_sweep19_3d_q4(const float* x, float* y, const float* b, const float*
   if (box_empty(bx)) return true;
   const long long q0 = (g.n1 * (bx.j0 - 1)) / 4, qe = (g.n1 * bx.j1 + 3) / 4;  // quads covering rows j0 .. j1
   const long long nq = qe - q0;
-  const dim3 grid((unsigned)((nq + 255) / 256), (unsigned)((bx.k1 - bx.k0 + kQ19Run) / kQ19Run));
-  launch_dep(k_sweep19_3d_q4, grid, 256, 0, s, x, y, b, w, cff, g.n1, g.n2, bx, q0, nq);
+  const long long nb = (nq + 255) / 256;
+  const int nk = bx.k1 - bx.k0 + 1, run = nb * ((nk + kQ19Run - 1) / kQ19Run) < kQBlocks ? 1 : kQ19Run;  // see kQBlocks
+  const dim3 grid((unsigned)nb, (unsigned)((nk + run - 1) / run));
+  launch_dep(k_sweep19_3d_q4, grid, 256, 0, s, x, y, b, w, cff, g.n1, g.n2, bx, q0, nq, run);
   return true;
 }
 
