@@ -1720,7 +1720,7 @@ int mixed_iteration(cfmg_handle* h, int kind) {
   TRY(flush(h));
   {
     Launch k(h, CFMG_K_CONVERT, 1, CFMG_MIXED, remove_mean ? 3 : 2);
-    if (remove_mean) launch_dep(k_mean_partial, kNormParts, 256, 0, h->stream, l1.r, l1.msk, n, h->partials);
+    if (remove_mean) launch_mean_fix(l1.r, l1.msk, n, h->dscal, h->partials, h->stream);
     launch_dep(k_scale_from_norm, 1, kNormParts, 0, h->stream, h->dscal, h->partials, kNormParts, remove_mean);
     launch_dep(k_rhs32, nb, 256, 0, h->stream, l1.r, l1.msk, h->dscal, l1.b32, l1.r32, n);
   }

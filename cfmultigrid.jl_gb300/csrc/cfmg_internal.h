@@ -452,6 +452,9 @@ void launch_fused_final(const double* partials, double* ds, const double* normb,
 void launch_rhs32_mean(const double* r, const uint8_t* m, const double* mean_scale, float* b32, float* r32,
                        long long n, cudaStream_t s);
 void launch_update_scaled(double* x, const float* e, const double* iscale, long long n, cudaStream_t s);
+// wet sum of r in fixed point, kNormParts partials; ds[S_NORM] = sum r^2 bounds it
+void launch_mean_fix(const double* r, const uint8_t* m, long long n, const double* ds, double* partials,
+                     cudaStream_t s);
 // integer form of the fused pass (kinds 5-, 7- and 9-point; 19-point: launch_resid_int19)
 void launch_resid_int(int kind, const double* x, const double* b, const int8_t* dq, const Geom& g, const Box& bx,
                       long long lo, long long n, const double* ds, float* b32, float* r32, bool neumann,

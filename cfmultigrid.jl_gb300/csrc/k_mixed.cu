@@ -494,6 +494,48 @@ bool launch_resid_int2d(int kind, const double* x, const double* b, const int8_t
   return false;
 }
 
+// ---- wet sum of r for the operators without a fused pass (variable
+// coefficient, x-periodic), per block into partials[kNormParts]. Each r is
+// taken to 64-bit fixed point, 2^58 steps for the bound |r| <= sqrt(sum r^2)
+// that the norm just gave (ds[S_NORM]), and added exactly in 128-bit integers:
+// rounding below 2^-59 of the bound a cell, against the bound's sqrt(n) times
+// smaller rms of r. The compensated FP64 sum it replaces issued six FP64
+// operations a cell: 66 us at 2048^2 against 13.7.
+__global__ void __launch_bounds__(256) k_mean_fix(const double* __restrict__ r, const uint8_t* __restrict__ m,
+                                                  long long n, const double* __restrict__ ds,
+                                                  double* __restrict__ partials) {
+  dep_wait();
+  int e2 = 0;
+  const double sq = ds[S_NORM];
+  if (sq > 0 && isfinite(sq)) frexp(sq, &e2);  // sum r^2 < 2^e2
+  const int k = 58 - ((e2 + 1) >> 1);
+  __int128 s = 0;
+  const long long st = (long long)kNormParts * 256;
+  long long I = (long long)blockIdx.x * 256 + threadIdx.x;
+  for (; I + 3 * st < n; I += 4 * st) {  // four cells' loads in flight
+    const double v0 = r[I], v1 = r[I + st], v2 = r[I + 2 * st], v3 = r[I + 3 * st];
+    const uint8_t m0 = m[I], m1 = m[I + st], m2 = m[I + 2 * st], m3 = m[I + 3 * st];
+    s += (__int128)((m0 ? to_fix(v0, k) : 0LL)) + (m1 ? to_fix(v1, k) : 0LL);
+    s += (__int128)((m2 ? to_fix(v2, k) : 0LL)) + (m3 ? to_fix(v3, k) : 0LL);
+  }
+  for (; I < n; I += st) s += m[I] ? to_fix(r[I], k) : 0LL;
+  double v = __dadd_rn(__dmul_rn((double)(long long)(s >> 64), 18446744073709551616.0), (double)(unsigned long long)s);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  __shared__ double sh[8];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double a = 0.0;
+    for (int w = 0; w < 8; ++w) a += sh[w];
+    partials[blockIdx.x] = ldexp(a, -k);
+  }
+}
+void launch_mean_fix(const double* r, const uint8_t* m, long long n, const double* ds, double* partials,
+                     cudaStream_t s) {
+  launch_dep(k_mean_fix, kNormParts, 256, 0, s, r, m, n, ds, partials);
+}
+
 // ---- 3D 19-point form. A block owns a 32 x 8 column tile of the interior box
 // and marches along k. Each x of the tile and its one-cell rim is converted
 // once into shared memory (340 conversions for 256 cells); a thread reads its
