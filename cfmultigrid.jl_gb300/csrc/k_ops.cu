@@ -568,6 +568,12 @@ __global__ void __launch_bounds__(kThreads) k_fill_xperio(T* __restrict__ x, int
 // With `lt` (the solve loop's last kernel) it also tests the stopping rule.
 // As two launches and a test kernel these were 3 of the 18 nodes of a 64^2
 // FP64 solve's iteration (see launch_norm).
+// msk*v^2 for a mask that is neither 0 nor 1: out of line, since inline the
+// compiler issued its conversion and three operations for every cell, five on
+// the FP64 pipe instead of the one FMA (39 us against 16 at 2048^2)
+static __device__ __noinline__ double weighted_square(uint8_t mm, double v, double s) {
+  return __dadd_rn(s, __dmul_rn((double)mm, __dmul_rn(v, v)));
+}
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_norm(const T* __restrict__ x, const uint8_t* __restrict__ m, long long n,
                                                    double* __restrict__ partials, unsigned* counter, double* out,
@@ -578,7 +584,8 @@ __global__ void __launch_bounds__(kThreads) k_norm(const T* __restrict__ x, cons
   auto add = [&](uint8_t mm, T xv) {
     if (mm) {
       const double v = (double)xv;
-      s = (mm == 1) ? __fma_rn(v, v, s) : __dadd_rn(s, __dmul_rn((double)mm, __dmul_rn(v, v)));
+      if (mm == 1) s = __fma_rn(v, v, s);
+      else s = weighted_square(mm, v, s);
     }
   };
   long long I = (long long)blockIdx.x * kThreads + threadIdx.x;
