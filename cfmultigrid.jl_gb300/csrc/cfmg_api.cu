@@ -144,6 +144,8 @@ struct cfmg_batch {
   BSmall* ssm = nullptr;       // small-level smoothing descriptors (device)
   int2* rent = nullptr;        // coarse-run entries {0, Op} / {1, BSmall} (device)
   int4* runs = nullptr;        // coarse runs {instance, first entry, end entry, 0} (device)
+  unsigned char* tstore = nullptr;  // coarse runs as tail programs (device) and their table
+  TailProg* tprogs = nullptr;
   bool host_loop = false;      // CFMG_BOPT_HOST_LOOP
   bool coarse_runs = true;     // CFMG_BOPT_COARSE_RUNS
   bool interleave = true;      // CFMG_BOPT_INTERLEAVE
@@ -155,8 +157,8 @@ struct cfmg_batch {
   bool neumann = false;
   struct Step {
     int tb, stencil, nite;     // tb: OPK_TB Ops of one (stencil, nite), 1 scalar tiles, 4 lean packed
-                               // tiles; 2: BSmall blocks; 3: coarse runs
-    long long tab0;            // offset into stab (or ssm, or runs)
+                               // tiles; 2: BSmall blocks; 3: coarse runs; 5: coarse runs as tail programs
+    long long tab0;            // offset into stab (or ssm, runs, tprogs)
     long long nchunks;         // table entries (or BSmall blocks, or runs)
     int smem;                  // BSmall, coarse runs: shared memory bytes
   };
@@ -350,7 +352,7 @@ size_t tail_hot_bytes(const cfmg_handle* h, const Level& l, int prec) {
 void plan_tail(cfmg_handle* h) {
   for (int prec = 0; prec < 2; ++prec) {
     h->tail_from[prec] = 0;
-    if (!h->engine_on || h->small_min <= 0 || !h->tail_pool || (prec == 1 && h->d.precision != CFMG_MIXED)) continue;
+    if (!h->engine_on || h->small_min <= 0 || (prec == 1 && h->d.precision != CFMG_MIXED)) continue;
     const long long cap = prec == 0 ? engine_limit(h, 0) * 6 / 5 : engine_limit(h, 1);
     size_t used = kTailBlobReserve;
     if (prec == 1 && coarsest_in_fp64(h)) used += tail_hot_bytes(h, h->lv.back(), 0);
@@ -363,7 +365,7 @@ void plan_tail(cfmg_handle* h) {
   }
 }
 bool in_tail(const cfmg_handle* h, int lev, int prec) {
-  return !h->record && h->engine_on && h->tail_from[prec] > 0 && lev >= h->tail_from[prec];
+  return !h->record && h->tail_pool && h->engine_on && h->tail_from[prec] > 0 && lev >= h->tail_from[prec];
 }
 
 // Copies a program into its device store, complete on return: allowed while
@@ -379,14 +381,17 @@ int upload_program(cfmg_handle* h, void* dst, const void* src, size_t bytes) {
   return CFMG_OK;
 }
 
-// Builds the pending Ops into tail programs and launches them: pairs of
+// A tail program: its bytes on the device, and what the launch needs to know.
+struct TailBuild {
+  std::string bytes;
+  int nctx, nstore, ncopy, nops;
+  size_t smem;
+};
+// Builds Ops into tail programs, to be run one after the other: pairs of
 // sweeps become smoothing calls, every array they touch is staged in shared
 // memory, the smoothing arrays first, then the others while they fit (those
-// left out are used in place). done = false: the Ops do not form such a
-// program (or the store is full), nothing was launched.
-int flush_tail(cfmg_handle* h, bool& done) {
-  done = false;
-  const std::vector<Op>& P = h->pending;
+// left out are used in place). false: the Ops do not form such programs.
+bool build_tail(const cfmg_handle* h, const std::vector<Op>& P, std::vector<TailBuild>& out) {
   std::vector<TailOp> ops;
   std::vector<TailCtx> ctxs;
   struct CtxPtr { const void *x, *y, *b, *w, *cE, *cN, *list; int lev; };
@@ -413,11 +418,11 @@ int flush_tail(cfmg_handle* h, bool& done) {
         k += 2 + f;
         ++pairs;
       }
-      if (!pairs) return CFMG_OK;
+      if (!pairs) return false;
       int q = 0;
       while (q < (int)ctxs.size() && !(cptr[q].x == a.x && cptr[q].w == a.w)) ++q;
       if (q == (int)ctxs.size()) {
-        if (q == kTailMaxCtx) return CFMG_OK;
+        if (q == kTailMaxCtx) return false;
         const Level& l = h->lv[a.lev - 1];
         TailCtx c;
         std::memset(&c, 0, sizeof(c));
@@ -438,7 +443,7 @@ int flush_tail(cfmg_handle* h, bool& done) {
       i = k;
     } else {
       const bool pro = a.kind >= OPK_PROLONG0 && a.kind <= OPK_PROLONG3;
-      if (!(a.kind >= OPK_RESID5 && a.kind <= OPK_F64TO32) || a.n > 0x7fffffff || a.assign) return CFMG_OK;
+      if (!(a.kind >= OPK_RESID5 && a.kind <= OPK_F64TO32) || a.n > 0x7fffffff || a.assign) return false;
       t.kind = a.kind;
       t.n = (int)a.n;
       t.lo = (int)a.lo;
@@ -462,8 +467,6 @@ int flush_tail(cfmg_handle* h, bool& done) {
       if (lev > 1 && cptr[q].lev == lev && ctxs[q].prec == t.prec && u(cptr[q].x) == t.x) t.ctxi = q;
   }
   // program pieces that fit the reserve
-  struct Launchable { size_t off; int bytes, nctx, nstore, ncopy, nops; size_t smem; };
-  std::vector<Launchable> todo;
   constexpr size_t kPiece = 100;
   for (size_t o0 = 0; o0 < ops.size(); o0 += kPiece) {
     std::vector<TailOp> po(ops.begin() + o0, ops.begin() + std::min(ops.size(), o0 + kPiece));
@@ -555,7 +558,7 @@ int flush_tail(cfmg_handle* h, bool& done) {
     };
     for (Arr& r : arr)
       if (r.hot) place(r);
-    if (at > kTailSmemMax) return CFMG_OK;
+    if (at > kTailSmemMax) return false;
     std::vector<size_t> ord(arr.size());
     for (size_t k = 0; k < ord.size(); ++k) ord[k] = k;
     std::stable_sort(ord.begin(), ord.end(), [&](size_t p, size_t q) { return arr[p].bytes < arr[q].bytes; });
@@ -599,24 +602,33 @@ int flush_tail(cfmg_handle* h, bool& done) {
     key.append((const char*)pcx.data(), pcx.size() * sizeof(TailCtx));
     key.append((const char*)cps.data(), cps.size() * sizeof(TailCopy));
     key.append((const char*)po.data(), po.size() * sizeof(TailOp));
-    const int bytes = (int)tail_al(key.size());
-    key.resize(bytes, 0);
-    size_t off;
-    auto it = h->tail_cache.find(key);
-    if (it != h->tail_cache.end()) {
-      off = it->second;
-    } else {
-      if (h->tail_used + bytes > h->tail_cap) return CFMG_OK;
-      TRY(upload_program(h, h->tail_pool + h->tail_used, key.data(), (size_t)bytes));
-      off = h->tail_used;
-      h->tail_used += (bytes + 255) & ~(size_t)255;
-      h->tail_cache.emplace(std::move(key), off);
-    }
-    todo.push_back({off, bytes, (int)pcx.size(), nstore, (int)cps.size(), (int)po.size(), at});
+    key.resize(tail_al(key.size()), 0);
+    out.push_back({std::move(key), (int)pcx.size(), nstore, (int)cps.size(), (int)po.size(), at});
   }
-  for (const Launchable& q : todo) {
-    Launch k(h, CFMG_K_ENGINE, 0, P[0].prec ? CFMG_MIXED : CFMG_FP64);
-    launch_tail(h->tail_pool + q.off, q.bytes, q.nctx, q.nstore, q.ncopy, q.nops, q.smem, h->stream);
+  return true;
+}
+
+// Runs the pending Ops as tail programs. done = false: they do not form any
+// (or the store is full), and nothing was launched.
+int flush_tail(cfmg_handle* h, bool& done) {
+  done = false;
+  std::vector<TailBuild> built;
+  if (!build_tail(h, h->pending, built)) return CFMG_OK;
+  std::vector<size_t> at;
+  for (const TailBuild& q : built) {
+    auto it = h->tail_cache.find(q.bytes);
+    if (it == h->tail_cache.end()) {
+      if (h->tail_used + q.bytes.size() > h->tail_cap) return CFMG_OK;
+      TRY(upload_program(h, h->tail_pool + h->tail_used, q.bytes.data(), q.bytes.size()));
+      it = h->tail_cache.emplace(q.bytes, h->tail_used).first;
+      h->tail_used += (q.bytes.size() + 255) & ~(size_t)255;
+    }
+    at.push_back(it->second);
+  }
+  for (size_t i = 0; i < built.size(); ++i) {
+    const TailBuild& q = built[i];
+    Launch k(h, CFMG_K_ENGINE, 0, h->pending[0].prec ? CFMG_MIXED : CFMG_FP64);
+    launch_tail(h->tail_pool + at[i], (int)q.bytes.size(), q.nctx, q.nstore, q.ncopy, q.nops, q.smem, h->stream);
   }
   done = true;
   return CFMG_OK;
@@ -691,7 +703,7 @@ int flush(cfmg_handle* h) {
 // levels beyond the tail that have blocked passes are left to those: a
 // descent step is one launch there and 11 Ops of 2.3 us in the engine.
 bool blocked_form(const cfmg_handle* h, int lev) {
-  if (!h->tb_on || h->record || threed(h) || h->small_min <= 0 || h->tail_from[1] <= 0) return false;
+  if (!h->tb_on || h->record || threed(h) || !h->tail_pool || h->tail_from[1] <= 0) return false;
   if (h->d.op != CFMG_LAPLACIAN && h->d.op != CFMG_LAPLACIAN9) return false;
   return !xperio(h) || (h->tb_version == 5 && h->d.op == CFMG_LAPLACIAN);
 }
@@ -762,6 +774,17 @@ int sweep(cfmg_handle* h, int lev, int kind, const T* x, T* y, const Box* bx, bo
   return emit(h, op);
 }
 
+// A batched instance's coarse levels, whose steps run as one block per run of
+// steps: those of the coarse tail, else (small_smooth = 0) those that a
+// single handle would run in the cluster engine. Larger ones take part in
+// the steps launched for all instances: at 134^2 cells an Op takes one block
+// 10 us and more.
+bool batch_coarse(const cfmg_handle* h, int lev) {
+  if (!h->engine_on) return false;
+  if (h->tail_from[1] > 0) return lev >= h->tail_from[1];
+  return (long long)h->lv[lev - 1].len <= engine_limit(h, CFMG_MIXED);
+}
+
 // FP32 smoothing of a fine level in temporally blocked passes (closed
 // topology, 2D 5- and 9-point): the result goes to the partner buffer.
 template <class T>
@@ -774,7 +797,7 @@ bool tb_eligible(const cfmg_handle* h, int lev) {
   // four single-sweep kernels at 66 % of HBM
   if (threed(h) && (h->d.op != CFMG_LAPLACIAN || h->record || h->tb_version != 4)) return false;
   if (h->d.op != CFMG_LAPLACIAN && h->d.op != CFMG_LAPLACIAN9) return false;
-  if (h->record) return !(h->engine_on && (long long)h->lv[lev - 1].len <= engine_limit(h, CFMG_MIXED));
+  if (h->record) return !batch_coarse(h, lev);
   return !in_engine(h, lev, CFMG_MIXED);
 }
 
@@ -2038,7 +2061,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
   const bool coded = mixed && d->kase == CFMG_THREED && d->op == CFMG_LAPLACIAN;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t tail_bytes = shared ? 0 : kTailPoolBytes;
-  auto tailed = [&](const Level& l) { return tail_bytes && l.len <= (size_t)kTailMaxLen; };
+  auto tailed = [&](const Level& l) { return l.len <= (size_t)kTailMaxLen; };
   size_t total = al(kPartials * sizeof(double)) + al(S_COUNT * sizeof(double)) + al((size_t)pool_ops * sizeof(Op)) +
                  al(tail_bytes);
   for (const Level& l : h->lv) {
@@ -2604,6 +2627,7 @@ int batch_build(cfmg_batch* b) {
   BCUDA(b, cudaMemcpy(b->ptrs, ptrs.data(), sizeof(Op*) * (size_t)ninst, cudaMemcpyHostToDevice));
   BCUDA(b, cudaMalloc((void**)&b->nops, sizeof(int) * (size_t)ninst));
   BCUDA(b, cudaMemcpy(b->nops, cnt.data(), sizeof(int) * (size_t)ninst, cudaMemcpyHostToDevice));
+  BCUDA(b, cudaStreamSynchronize(cudaStreamLegacy));  // the uploads above are from pageable memory
   b->nclusters = engine_max_clusters();
   if (b->nclusters > ninst) b->nclusters = ninst;
   BCUDA(b, cudaMalloc((void**)&b->counter, sizeof(int) * (size_t)(1 + b->nclusters)));
@@ -2730,7 +2754,9 @@ int lockstep_body(cfmg_batch* b) {
     if (b->neumann) launch_brhs(b->bi, b->l1tab, b->l1chunks, b->active, b->stream);
   }
   for (const cfmg_batch::Step& st : b->steps) {
-    if (st.tb == 3) {
+    if (st.tb == 5) {
+      launch_tail_batch(b->tstore, b->tprogs + st.tab0, (int)st.nchunks, (size_t)st.smem, b->active, b->stream);
+    } else if (st.tb == 3) {
       launch_brun(b->sops, b->ssm, b->rent, b->runs + st.tab0, (int)st.nchunks, st.smem, b->active, b->stream);
     } else if (st.tb == 2) {
       launch_bsmall(b->ssm + st.tab0, (int)st.nchunks, st.smem, b->active, b->stream);
@@ -2791,10 +2817,10 @@ int lockstep_build(cfmg_batch* b) {
         if (k == 0) v.depth = L(h);
         if (L(h) == 1 && v.op != V_ZERO && v.op != V_COARSEST) continue;
         part[i][k] = 1;
-        const Level& lv = h->lv[L(h) - v.depth];  // the step's level (the finer one of a transfer)
-        coarse[i][k] = b->coarse_runs && h->engine_on && (long long)lv.len <= engine_limit(h, CFMG_MIXED);
+        // the step's level (the finer one of a transfer)
+        coarse[i][k] = b->coarse_runs && batch_coarse(h, L(h) - v.depth + 1);
         BSmall sm;
-        if (L(h) > 1 && small_smooth(h, v, sm)) {
+        if (!(coarse[i][k] && h->tail_from[1] > 0) && L(h) > 1 && small_smooth(h, v, sm)) {
           sm.inst = i;
           smalls[k].push_back(sm);
           continue;
@@ -2848,13 +2874,52 @@ int lockstep_build(cfmg_batch* b) {
   // Instances are independent, so only each instance's own order matters.
   std::vector<int2> rent;
   std::vector<int4> runs;
+  // With the coarse tail (k_tail.cu) a run is a program of it.
   std::vector<std::vector<int2>> pend(ninst);
   std::vector<int> pend_smem(ninst, 0);
+  std::string tstore;
+  std::vector<TailProg> tprogs;
   auto small_bytes = [](const BSmall& q) { return (int)(4 * q.g.len * (q.prec == 0 ? 8 : 4)); };
   auto flush_runs = [&]() {
     cfmg_batch::Step st;
     st.tb = 3; st.stencil = 0; st.nite = 0; st.smem = 0;
     st.tab0 = (long long)runs.size();
+    cfmg_batch::Step tt = st;  // the tail's programs: piece q of every run, then piece q + 1
+    std::vector<std::vector<TailProg>> piece;
+    for (int i = 0; i < ninst; ++i) {
+      if (pend[i].empty() || b->inst[i]->tail_from[1] <= 0) continue;
+      std::vector<Op> ops;
+      bool plain = true;
+      for (const int2& e : pend[i]) {
+        plain = plain && e.x == 0;
+        if (e.x == 0) ops.push_back(all[e.y]);
+      }
+      std::vector<TailBuild> built;
+      if (!plain || !build_tail(b->inst[i], ops, built)) continue;  // stays a run of k_brun
+      for (size_t q = 0; q < built.size(); ++q) {
+        if (q == piece.size()) piece.emplace_back();
+        TailProg p;
+        std::memset(&p, 0, sizeof(p));
+        p.off = (long long)tstore.size();
+        p.bytes = (int)built[q].bytes.size();
+        p.nctx = built[q].nctx; p.nstore = built[q].nstore; p.ncopy = built[q].ncopy; p.nops = built[q].nops;
+        p.inst = i;
+        tstore += built[q].bytes;
+        tstore.resize((tstore.size() + 15) & ~(size_t)15, 0);
+        tt.smem = std::max(tt.smem, (int)built[q].smem);
+        piece[q].push_back(p);
+      }
+      pend[i].clear();
+      pend_smem[i] = 0;
+    }
+    for (const auto& pc : piece) {
+      cfmg_batch::Step t = tt;
+      t.tb = 5;
+      t.tab0 = (long long)tprogs.size();
+      t.nchunks = (long long)pc.size();
+      tprogs.insert(tprogs.end(), pc.begin(), pc.end());
+      b->steps.push_back(t);
+    }
     for (int i = 0; i < ninst; ++i) {
       if (pend[i].empty()) continue;
       runs.push_back(make_int4(i, (int)rent.size(), (int)(rent.size() + pend[i].size()), 0));
@@ -3011,6 +3076,12 @@ int lockstep_build(cfmg_batch* b) {
     BCUDA(b, cudaMalloc((void**)&b->runs, sizeof(int4) * runs.size()));
     BCUDA(b, cudaMemcpy(b->runs, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice));
   }
+  if (!tprogs.empty()) {
+    BCUDA(b, cudaMalloc((void**)&b->tstore, tstore.size()));
+    BCUDA(b, cudaMemcpy(b->tstore, tstore.data(), tstore.size(), cudaMemcpyHostToDevice));
+    BCUDA(b, cudaMalloc((void**)&b->tprogs, sizeof(TailProg) * tprogs.size()));
+    BCUDA(b, cudaMemcpy(b->tprogs, tprogs.data(), sizeof(TailProg) * tprogs.size(), cudaMemcpyHostToDevice));
+  }
   if (!all.empty()) {
     BCUDA(b, cudaMalloc((void**)&b->sops, sizeof(Op) * all.size()));
     BCUDA(b, cudaMemcpy(b->sops, all.data(), sizeof(Op) * all.size(), cudaMemcpyHostToDevice));
@@ -3019,6 +3090,7 @@ int lockstep_build(cfmg_batch* b) {
     BCUDA(b, cudaMalloc((void**)&b->stab, sizeof(int4) * tab.size()));
     BCUDA(b, cudaMemcpy(b->stab, tab.data(), sizeof(int4) * tab.size(), cudaMemcpyHostToDevice));
   }
+  BCUDA(b, cudaStreamSynchronize(cudaStreamLegacy));  // the uploads above are from pageable memory
   b->kind = hb[0].kind;
   b->neumann = hb[0].neumann != 0;
   for (int i = 1; i < ninst; ++i)
@@ -3109,7 +3181,8 @@ int cfmg_batch_destroy(cfmg_batch* b) {
   for (void* p : {(void*)b->progs, (void*)b->ptrs, (void*)b->nops, (void*)b->counter, (void*)b->red, (void*)b->sc,
                   (void*)b->nwet, (void*)b->bi, (void*)b->l1start, (void*)b->l1tab, (void*)b->bpart,
                   (void*)b->active, (void*)b->nactive, (void*)b->sops, (void*)b->stab, (void*)b->ssm,
-                  (void*)b->ttab, (void*)b->tstart, (void*)b->rent, (void*)b->runs})
+                  (void*)b->ttab, (void*)b->tstart, (void*)b->rent, (void*)b->runs, (void*)b->tstore,
+                  (void*)b->tprogs})
     if (p) cudaFree(p);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
@@ -3161,7 +3234,7 @@ int cfmg_batch_solve(cfmg_batch* b, int zero_x, double* res, int* nite, double* 
                      (void**)&b->sc, (void**)&b->nwet, (void**)&b->bi, (void**)&b->l1start, (void**)&b->l1tab,
                      (void**)&b->bpart, (void**)&b->active, (void**)&b->nactive, (void**)&b->sops,
                      (void**)&b->stab, (void**)&b->ssm, (void**)&b->ttab, (void**)&b->tstart, (void**)&b->rent,
-                     (void**)&b->runs})
+                     (void**)&b->runs, (void**)&b->tstore, (void**)&b->tprogs})
       if (*p) {
         cudaFree(*p);
         *p = nullptr;
@@ -3170,6 +3243,8 @@ int cfmg_batch_solve(cfmg_batch* b, int zero_x, double* res, int* nite, double* 
     TRY(b->lockstep ? lockstep_build(b) : batch_build(b));
   }
   const int ninst = (int)b->inst.size();
+  for (cfmg_handle* h : b->inst)
+    if (tail_lists(h) != CFMG_OK) return bfail(b, CFMG_ERR_CUDA, h->err);
   if (b->lockstep && b->host_loop) {
     launch_binit(b->bi, ninst, zero_x ? 1 : 0, b->active, b->nactive, b->stream);
     for (;;) {

@@ -343,8 +343,9 @@ __device__ __forceinline__ void tail_exec(const TailOp* op) {
 
 }  // namespace
 
-__global__ void __launch_bounds__(kTT, 1) k_tail(const unsigned char* __restrict__ blob, int blob_bytes, int nctx,
-                                                 int nstore, int ncopy, int nops) {
+// one program, run by one block
+__device__ __forceinline__ void tail_run(const unsigned char* __restrict__ blob, int blob_bytes, int nctx, int nstore,
+                                         int ncopy, int nops) {
   __shared__ int full[kTailMaxCtx];  // -1: not looked at in this launch; 1: the context sweeps its whole range
   const int tid = threadIdx.x;
   // the program was uploaded before the launch: no kernel writes it
@@ -404,6 +405,21 @@ __global__ void __launch_bounds__(kTT, 1) k_tail(const unsigned char* __restrict
     if (tid * 16 < (int)cp[q].bytes)
       *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(cp[q].g) + tid * 16) =
           *reinterpret_cast<const uint4*>(sm + cp[q].off + tid * 16);
+}
+
+__global__ void __launch_bounds__(kTT, 1) k_tail(const unsigned char* __restrict__ blob, int blob_bytes, int nctx,
+                                                 int nstore, int ncopy, int nops) {
+  tail_run(blob, blob_bytes, nctx, nstore, ncopy, nops);
+}
+
+// batched solver: a block per program of the table, for instances still iterating
+__global__ void __launch_bounds__(kTT, 1) k_tail_batch(const unsigned char* __restrict__ store,
+                                                       const TailProg* __restrict__ tab,
+                                                       const int* __restrict__ active) {
+  const TailProg p = tab[blockIdx.x];  // uploaded before the launch
+  dep_wait();
+  if (!active[p.inst]) return;
+  tail_run(store + p.off, p.bytes, p.nctx, p.nstore, p.ncopy, p.nops);
 }
 
 // The cell lists of the levels, one block a level: {live cells, cells of the
@@ -469,6 +485,13 @@ __global__ void __launch_bounds__(1024) k_tail_lists(TailListArgs a) {
     hdr[0] = tl;
     hdr[1] = tl + td;
   }
+}
+
+void launch_tail_batch(const void* store, const TailProg* tab, int n, size_t smem, const int* active, cudaStream_t s) {
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(k_tail_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmemMax);
+  (void)attr;
+  if (n > 0) launch_dep(k_tail_batch, (unsigned)n, kTT, smem, s, (const unsigned char*)store, tab, active);
 }
 
 void launch_tail_lists(const TailListArgs& a, int n, cudaStream_t s) {

@@ -278,8 +278,9 @@ CFMG_API int cfmg_adjoint_solve(cfmg_handle* h, const double* cot, double* grad_
  * profilers that do not descend into conditional graph nodes). */
 #define CFMG_BOPT_HOST_LOOP 0
 /* cfmg_batch_set_option(b, CFMG_BOPT_COARSE_RUNS, 0/1): with 1 (default) the
- * steps of an iteration on an instance's coarse levels (those its engine
- * threshold, CFMG_OPT_ENGINE_CELLS, would put in the program engine) run as
+ * steps of an iteration on an instance's coarse levels (the coarse tail's,
+ * see CFMG_OPT_SMALL_SMOOTH; with small_smooth 0 those its engine threshold,
+ * CFMG_OPT_ENGINE_CELLS, would put in the program engine) run as
  * one block per instance, a run of consecutive steps per launch, instead of
  * one launch per step; 0 launches every step for all instances. Same
  * values either way. */
