@@ -71,19 +71,6 @@ __device__ __forceinline__ double bsum(double v, double* sh) {
   return t;
 }
 
-// block maximum (kBThreads threads); valid in thread 0
-__device__ __forceinline__ double bmax(double v, double* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < kBThreads / 32; ++w) t = fmax(t, sh[w]);
-  return t;
-}
-
 // ------------------------------------------------------------ cycle steps
 // Generic step: the active chunks (kBStageChunk items) of a list of Ops
 // (tab[c] = {op, chunk of the op, instance}), each executed with the
@@ -118,28 +105,100 @@ static_assert(sizeof(Op) / sizeof(int) <= kBThreads, "one thread per word of an 
 
 // ------------------------------------------------------- FP64 loop steps
 // start of a solve: zero x when asked, normb = sum msk b^2 (0 -> 1 for the
-// reference rule), the first right-hand-side scale from |b|, counters.
-// One block per instance.
-__global__ void __launch_bounds__(kBThreads) k_binit(const BInst* __restrict__ bi, int zero_x, int* active,
-                                                     int* nactive) {
+// reference rule), the first right-hand-side scale from |b|, counters. A
+// cluster of kInitCtas blocks per instance: with one block the largest
+// instance of a batch (1024^2) set the launch's 1.4 ms, 4100 rounds of loads
+// and five FP64-pipe instructions each. Here a thread loads four cells ahead,
+// the maxima are of bit patterns, and the blocks' results meet in block 0's
+// shared memory, added in rank order: 173 us.
+constexpr int kInitCtas = 8;
+static __device__ __noinline__ double weighted_sq(uint8_t mm, double v, double s) {
+  return __dadd_rn(s, __dmul_rn((double)mm, __dmul_rn(v, v)));
+}
+// |v| as bits, 0 for a NaN (as fmax ignores it)
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFULL;
+  return u > 0x7FF0000000000000ULL ? 0ULL : u;
+}
+__device__ __forceinline__ unsigned long long bmax_bits(unsigned long long v, unsigned long long* sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long u = __shfl_down_sync(0xffffffffu, v, o);
+    v = u > v ? u : v;
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  unsigned long long t = 0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kBThreads / 32; ++w) t = sh[w] > t ? sh[w] : t;
+  return t;
+}
+__global__ void __cluster_dims__(kInitCtas, 1, 1) __launch_bounds__(kBThreads)
+    k_binit(const BInst* __restrict__ bi, int zero_x, int* active, int* nactive) {
   dep_wait();
   __shared__ double sh[kBThreads / 32];
-  const BInst& B = bi[blockIdx.x];
-  double* sc = B.sc;
+  __shared__ unsigned long long shu[kBThreads / 32];
+  __shared__ double part[kInitCtas][3];  // block 0's copy collects every block's results
+  const int inst = blockIdx.x / kInitCtas, rank = blockIdx.x % kInitCtas;
+  const BInst& B = bi[inst];
   const bool zx = zero_x != 0;
-  double v = 0.0, mx = 0.0, mb = 0.0;
-  for (long long t = threadIdx.x; t < B.len; t += kBThreads) {
-    if (zx) B.x[t] = 0.0;
-    const uint8_t mm = B.m[t];
-    const double bb = B.b[t];
-    if (mm) v = (mm == 1) ? __fma_rn(bb, bb, v) : __dadd_rn(v, __dmul_rn((double)mm, __dmul_rn(bb, bb)));
-    mx = fmax(mx, fabs(B.x[t]));
-    mb = fmax(mb, fabs(bb));
+  double v = 0.0;
+  unsigned long long mx = 0, mb = 0;
+  constexpr long long st = (long long)kInitCtas * kBThreads;
+  auto cell = [&](uint8_t mm, double bb, double xx) {
+    if (mm) {
+      if (mm == 1) v = __fma_rn(bb, bb, v);
+      else v = weighted_sq(mm, bb, v);
+    }
+    const unsigned long long ux = abs_bits(xx), ub = abs_bits(bb);
+    mx = ux > mx ? ux : mx;
+    mb = ub > mb ? ub : mb;
+  };
+  const uint8_t* __restrict__ m = B.m;
+  const double* __restrict__ b = B.b;
+  double* x = B.x;
+  long long t = (long long)rank * kBThreads + threadIdx.x;
+  for (; t + 3 * st < B.len; t += 4 * st) {
+    uint8_t mm[4];
+    double bb[4], xx[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      mm[u] = m[t + u * st];
+      bb[u] = b[t + u * st];
+      xx[u] = zx ? 0.0 : x[t + u * st];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (zx) x[t + u * st] = 0.0;
+      cell(mm[u], bb[u], xx[u]);
+    }
   }
-  double tot = bsum(v, sh);
-  __syncthreads();
-  const double tmx = bmax(mx, sh), tmb = bmax(mb, sh);
+  for (; t < B.len; t += st) {
+    const double xx = zx ? 0.0 : x[t];
+    if (zx) x[t] = 0.0;
+    cell(m[t], b[t], xx);
+  }
+  const double s0 = bsum(v, sh);
+  const unsigned long long m0 = bmax_bits(mx, shu), m1 = bmax_bits(mb, shu);
   if (threadIdx.x == 0) {
+    const double res[3] = {s0, __longlong_as_double((long long)m0), __longlong_as_double((long long)m1)};
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      unsigned a = (unsigned)__cvta_generic_to_shared(&part[rank][q]), ra;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ra) : "r"(a));
+      asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(res[q]) : "memory");
+    }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank == 0 && threadIdx.x == 0) {
+    double* sc = B.sc;
+    double tot = 0.0, tmx = 0.0, tmb = 0.0;
+    for (int r = 0; r < kInitCtas; ++r) {
+      tot = __dadd_rn(tot, part[r][0]);
+      tmx = fmax(tmx, part[r][1]);
+      tmb = fmax(tmb, part[r][2]);
+    }
     sc[BS_MAXX] = tmx;
     sc[BS_MAXB] = tmb;
     if (B.norm_kind == CFMG_NORM_REF_SQUARED && tot == 0.0) tot = 1.0;
@@ -151,8 +210,8 @@ __global__ void __launch_bounds__(kBThreads) k_binit(const BInst* __restrict__ b
     if (rms > 0 && isfinite(rms)) frexp(rms, &e);
     sc[BS_NEXT] = ldexp(1.0, -e);
     sc[BS_T0] = (double)gtimer();
-    active[blockIdx.x] = 1;
-    if (blockIdx.x == 0) *nactive = 0;
+    active[inst] = 1;
+    if (inst == 0) *nactive = 0;
   }
 }
 
@@ -630,7 +689,7 @@ void launch_bstage(const Op* ops, const int4* tab, long long nchunks, const int*
 }
 
 void launch_binit(const BInst* bi, int ninst, int zero_x, int* active, int* nactive, cudaStream_t s) {
-  launch_dep(k_binit, ninst, kBThreads, 0, s, bi, zero_x, active, nactive);
+  launch_dep(k_binit, ninst * kInitCtas, kBThreads, 0, s, bi, zero_x, active, nactive);
 }
 
 void launch_bres(int kind, bool neumann, const BInst* bi, const int4* tab, long long nchunks, const int* active,
