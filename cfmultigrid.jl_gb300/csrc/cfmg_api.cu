@@ -105,6 +105,7 @@ struct cfmg_handle {
   float* wtab = nullptr;  // 256 entries
   bool record = false;  // emit() records every Op (whole-solve programs) instead of running it
   bool record_tb = false;  // while recording: temporally blocked smoothing is recorded as OPK_TB Ops
+  bool record_epi = false;  // while recording: the last such pass takes its descent step's epilogue
 };
 
 constexpr int kProgPoolOps = 8192;  // device store of engine programs (~1.9 MB)
@@ -157,7 +158,8 @@ struct cfmg_batch {
   bool neumann = false;
   struct Step {
     int tb, stencil, nite;     // tb: OPK_TB Ops of one (stencil, nite), 1 scalar tiles, 4 lean packed
-                               // tiles; 2: BSmall blocks; 3: coarse runs; 5: coarse runs as tail programs
+                               // tiles; 2: BSmall blocks; 3: coarse runs; 5: coarse runs as tail programs;
+                               // 6: as 4 with a descent step's epilogue
     long long tab0;            // offset into stab (or ssm, runs, tprogs)
     long long nchunks;         // table entries (or BSmall blocks, or runs)
     int smem;                  // BSmall, coarse runs: shared memory bytes
@@ -867,7 +869,15 @@ int smooth_tb(cfmg_handle* h, int lev, int nite) {
       op.np_i = n;
       op.np_j = stencil;
       op.form = h->tb_version >= 5 ? 5 : 1;  // the tile form of the standalone passes
-      if (op.form == 5) tb5_tiles(n, op.box.i0, op.box.i1, op.box.j0, op.box.j1, &op.kf0, &op.kf1);
+      if (h->record_epi && left == n) {  // the descent step's last pass: residual, restriction, coarse x zeroed
+        const Level& c = h->lv[lev];
+        const View<float> vc = view<float>(c);
+        op.form = 6;
+        op.d = v.diag; op.m = l.msk; op.coef = vc.Rcoef; op.y2 = vc.b; op.cE = vc.x;
+        op.gc = geom(c);
+        op.s0 = vertices(h) ? 2 : 0;
+      }
+      if (op.form >= 5) tb5_tiles(n, op.form == 6, op.box.i0, op.box.i1, op.box.j0, op.box.j1, &op.kf0, &op.kf1);
       else tb_tiles(n, op.box.i0, op.box.i1, op.box.j0, op.box.j1, &op.kf0, &op.kf1);
       op.n = (long long)op.kf0 * op.kf1 * l.tz;
       h->pending.push_back(op);
@@ -2741,6 +2751,22 @@ int record_vstep(cfmg_handle* h, const VStep& v, std::vector<Op>& out) {
   return rc;
 }
 
+// A descent step (smoothing, residual, restriction of r, coarse x zeroed) that
+// an instance records as one blocked pass with that epilogue: the conditions
+// of fused_descent_ok, on a level that takes blocked passes
+bool batch_fused_descent(const cfmg_handle* h, const std::vector<VStep>& vs, size_t k) {
+  const VStep& v = vs[k];
+  if (v.op != V_SMOOTH || v.arg < 1 || k + 3 >= vs.size() || !h->fuse_on || h->tb_version != 5 || !h->record_tb)
+    return false;
+  if (vs[k + 1].op != V_RESID || vs[k + 1].depth != v.depth || vs[k + 2].op != V_RESTRICT ||
+      vs[k + 2].depth != v.depth || vs[k + 2].arg != CFMG_R || vs[k + 3].op != V_ZERO ||
+      vs[k + 3].depth != v.depth - 1)
+    return false;
+  const int lev = L(h) - v.depth + 1;
+  if (lev >= L(h) || h->lv[lev - 1].tz != 1 || !h->tb_on) return false;
+  return !batch_coarse(h, lev);
+}
+
 // One lockstep iteration of every active instance (see k_batch.cu).
 int lockstep_body(cfmg_batch* b) {
   const int ninst = (int)b->inst.size();
@@ -2760,8 +2786,8 @@ int lockstep_body(cfmg_batch* b) {
       launch_brun(b->sops, b->ssm, b->rent, b->runs + st.tab0, (int)st.nchunks, st.smem, b->active, b->stream);
     } else if (st.tb == 2) {
       launch_bsmall(b->ssm + st.tab0, (int)st.nchunks, st.smem, b->active, b->stream);
-    } else if (st.tb == 4) {
-      if (!launch_btb5(st.stencil, st.nite, b->sops, b->stab + st.tab0, st.nchunks, b->active, b->stream))
+    } else if (st.tb == 4 || st.tb == 6) {
+      if (!launch_btb5(st.stencil, st.nite, st.tb == 6, b->sops, b->stab + st.tab0, st.nchunks, b->active, b->stream))
         return bfail(b, CFMG_ERR_UNSUPPORTED, "blocked pass shape");
     } else if (st.tb) {
       if (!launch_btb(st.stencil, st.nite, b->sops, b->stab + st.tab0, st.nchunks, b->active, b->stream))
@@ -2811,9 +2837,10 @@ int lockstep_build(cfmg_batch* b) {
       coarse[i].assign(vs.size(), 0);
       for (auto& sm : smalls)
         sm.erase(std::remove_if(sm.begin(), sm.end(), [&](const BSmall& q) { return q.inst == i; }), sm.end());
+      size_t skip_to = 0;  // steps that the fused descent before them holds
       for (size_t k = 0; k < vs.size(); ++k) {
         VStep v = vs[k];
-        if (L(h) < v.need) continue;
+        if (L(h) < v.need || k < skip_to) continue;
         if (k == 0) v.depth = L(h);
         if (L(h) == 1 && v.op != V_ZERO && v.op != V_COARSEST) continue;
         part[i][k] = 1;
@@ -2825,7 +2852,10 @@ int lockstep_build(cfmg_batch* b) {
           smalls[k].push_back(sm);
           continue;
         }
+        h->record_epi = batch_fused_descent(h, vs, k);
+        if (h->record_epi) skip_to = k + 4;
         int rc = record_vstep(h, v, rec[i][k]);
+        h->record_epi = false;
         if (rc != CFMG_OK) return bfail(b, rc, "instance " + std::to_string(i) + ": " + h->err);
         for (Op& op : rec[i][k]) {
           op.inst = i;
@@ -2967,14 +2997,14 @@ int lockstep_build(cfmg_batch* b) {
       if (!coarse[i][k]) depth = std::max(depth, rec[i][k].size());
     for (size_t q = 0; q < depth; ++q) {
       std::vector<Op> gen;
-      std::vector<std::vector<Op>> tbs(16);  // [lean packed form?][stencil 9?][pairs]
+      std::vector<std::vector<Op>> tbs(24);  // [scalar, lean packed, lean packed with epilogue][stencil 9?][pairs]
       for (int i = 0; i < ninst; ++i) {
         if (coarse[i][k] || q >= rec[i][k].size()) continue;
         const Op& op = rec[i][k][q];
-        if (op.kind == OPK_TB) tbs[(op.form == 5 ? 8 : 0) + (op.np_j == 9 ? 4 : 0) + op.np_i].push_back(op);
+        if (op.kind == OPK_TB) tbs[(op.form >= 5 ? 8 * (op.form - 4) : 0) + (op.np_j == 9 ? 4 : 0) + op.np_i].push_back(op);
         else gen.push_back(op);
       }
-      for (int t = 0; t < 16; ++t) add_step(tbs[t], t >= 8 ? 4 : 1, (t & 4) ? 9 : 5, t & 3);
+      for (int t = 0; t < 24; ++t) add_step(tbs[t], t >= 16 ? 6 : (t >= 8 ? 4 : 1), (t & 4) ? 9 : 5, t & 3);
       add_step(gen, 0, 0, 0);
     }
   }

@@ -246,7 +246,7 @@ struct Op {
   const uint8_t* wq;
   const float* wtab;
   const uint8_t* qact;  // the level's quad activity flags (see Level), or null: every quad swept
-  int form;  // OPK_TB: 5 the lean packed tiles (k_btb5), else the scalar tiles (k_btb)
+  int form;  // OPK_TB: 5 the lean packed tiles (k_btb5), 6 those with a descent step's epilogue, else the scalar tiles (k_btb)
 };
 // scalar block of a whole-solve program
 enum SolveSlot { SS_NORMB = 0, SS_NR, SS_RES, SS_NITE, SS_NWET, SS_MEAN, SS_SCALE, SS_ISCALE, SS_T0, SS_T1,
@@ -422,8 +422,9 @@ void tb_tiles(int nite, int ui0, int ui1, int uj0, int uj1, int* ntx, int* nty);
 bool launch_btb(int stencil, int nite, const Op* ops, const int4* tab, long long ntiles, const int* active,
                 cudaStream_t s);
 // the same for the lean packed pass (OPK_TB Ops of form 5)
-void tb5_tiles(int nite, int ui0, int ui1, int uj0, int uj1, int* ntx, int* nty);
-bool launch_btb5(int stencil, int nite, const Op* ops, const int4* tab, long long ntiles, const int* active,
+// epi: with the descent step's residual and restriction (see k_btb5)
+void tb5_tiles(int nite, bool epi, int ui0, int ui1, int uj0, int uj1, int* ntx, int* nty);
+bool launch_btb5(int stencil, int nite, bool epi, const Op* ops, const int4* tab, long long ntiles, const int* active,
                  cudaStream_t s);
 void launch_binit(const BInst* bi, int ninst, int zero_x, int* active, int* nactive, cudaStream_t s);
 void launch_bres(int kind, bool neumann, const BInst* bi, const int4* tab, long long nchunks, const int* active,

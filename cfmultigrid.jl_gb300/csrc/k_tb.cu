@@ -777,7 +777,12 @@ __global__ void __launch_bounds__(kTbW * kTbTy, 1) k_btb(const Op* __restrict__ 
 // standalone pass): the same windowed walk over a tile table as k_btb, each
 // active tile run by tb5_tile; the barrier after a tile keeps the next
 // tile's loads behind this tile's last shared-memory reads.
-template <int ST, int NITE>
+//
+// EPI: the Ops carry a descent step's residual and restriction too (np_i
+// pairs, then OPK_TB fields d, m, coef, gc, y2 = coarse b, cE = coarse x): one
+// launch instead of four for the instances that have such a step (128
+// instances of 64^2..1024^2: 30.0 -> 25.8 ms).
+template <int ST, int NITE, bool EPI>
 __global__ void __launch_bounds__(kT5Tx * 8, 2) k_btb5(const Op* __restrict__ ops, const int4* __restrict__ tab,
                                                        long long ntiles, int win, const int* __restrict__ active) {
   dep_wait();
@@ -813,10 +818,20 @@ __global__ void __launch_bounds__(kT5Tx * 8, 2) k_btb5(const Op* __restrict__ op
       const long long per_layer = (long long)op.kf0 * op.kf1;
       const int bz = (int)(en.y / per_layer);
       const int rem = (int)(en.y - (long long)bz * per_layer);
-      tb5_tile<ST, NITE, 8, 6, false, false, false>((const float*)op.x, (float*)op.y, (const float*)op.b,
-                                                    (const float*)op.w, (float)op.cff, op.g.tx, op.g.ty, op.box.i0,
-                                                    op.box.i1, op.box.j0, op.box.j1, TbEpi{}, rem % op.kf0,
-                                                    rem / op.kf0, bz, smem);
+      TbEpi ep{};
+      if constexpr (EPI) {
+        const int nh = op.g.nh;
+        ep.d = (const float*)op.d; ep.m = op.m; ep.rcoef = (const float*)op.coef;
+        ep.bc = (float*)op.y2; ep.xc = (float*)const_cast<void*>(op.cE);
+        ep.ri0 = nh + 1; ep.ri1 = op.g.tx - nh; ep.rj0 = nh + 1; ep.rj1 = op.g.ty - nh;
+        ep.nh = nh; ep.ctx = op.gc.tx;
+        ep.ci0 = nh + 1; ep.ci1 = op.gc.tx - nh; ep.cj0 = nh + 1; ep.cj1 = op.gc.ty - nh;
+        ep.pkind = op.s0;
+      }
+      tb5_tile<ST, NITE, 8, 6, EPI, false, false>((const float*)op.x, (float*)op.y, (const float*)op.b,
+                                                  (const float*)op.w, (float)op.cff, op.g.tx, op.g.ty, op.box.i0,
+                                                  op.box.i1, op.box.j0, op.box.j1, ep, rem % op.kf0, rem / op.kf0, bz,
+                                                  smem);
       __syncthreads();
     }
     __syncthreads();  // list is rewritten by the next window
@@ -949,19 +964,20 @@ void tb_tiles(int nite, int ui0, int ui1, int uj0, int uj1, int* ntx, int* nty) 
 }
 
 // tile counts of one lean packed pass (8 x 6 rows) over the box U
-void tb5_tiles(int nite, int ui0, int ui1, int uj0, int uj1, int* ntx, int* nty) {
-  const int H = 2 * nite, CW = kT5W - 2 * H, CH = 8 * 6 - 2 * H;
+void tb5_tiles(int nite, bool epi, int ui0, int ui1, int uj0, int uj1, int* ntx, int* nty) {
+  const int H = 2 * nite + (epi ? 2 : 0), CW = kT5W - 2 * H, CH = 8 * 6 - 2 * H;
   *ntx = (ui1 - ui0 + CW) / CW;
   *nty = (uj1 - uj0 + CH) / CH;
 }
 
-template <int ST, int NITE>
+template <int ST, int NITE, bool EPI>
 static void launch_btb5_n(const Op* ops, const int4* tab, long long ntiles, const int* active, cudaStream_t s) {
-  const size_t smem = 2 * (size_t)t5_plane<8, 6>() * sizeof(float);
+  const size_t smem = 2 * (size_t)t5_plane<8, 6>() * sizeof(float) +
+                      (EPI ? (size_t)48 * kT5Tx * (sizeof(float2) + sizeof(ushort)) : 0);
   static bool attr = false;
   static int nsm = 0;
   if (!attr) {
-    cudaFuncSetAttribute(k_btb5<ST, NITE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_btb5<ST, NITE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -973,15 +989,16 @@ static void launch_btb5_n(const Op* ops, const int4* tab, long long ntiles, cons
   if (win > kT5Tx * 8) win = kT5Tx * 8;
   const long long windows = (ntiles + win - 1) / win;
   const long long grid = windows < g ? windows : g;
-  launch_dep(k_btb5<ST, NITE>, (unsigned)grid, dim3(kT5Tx, 8, 1), smem, s, ops, tab, ntiles, (int)win, active);
+  launch_dep(k_btb5<ST, NITE, EPI>, (unsigned)grid, dim3(kT5Tx, 8, 1), smem, s, ops, tab, ntiles, (int)win, active);
 }
 
-bool launch_btb5(int stencil, int nite, const Op* ops, const int4* tab, long long ntiles, const int* active,
+bool launch_btb5(int stencil, int nite, bool epi, const Op* ops, const int4* tab, long long ntiles, const int* active,
                  cudaStream_t s) {
   if (ntiles <= 0) return true;
 #define CFMG_BTB5(ST, N)                                             \
   if (stencil == ST && nite == N) {                                  \
-    launch_btb5_n<ST, N>(ops, tab, ntiles, active, s);               \
+    if (epi) launch_btb5_n<ST, N, true>(ops, tab, ntiles, active, s); \
+    else launch_btb5_n<ST, N, false>(ops, tab, ntiles, active, s);   \
     return true;                                                     \
   }
   CFMG_BTB5(5, 1) CFMG_BTB5(5, 2) CFMG_BTB5(5, 3)
