@@ -63,6 +63,12 @@ struct cfmg_handle {
   // the levels' cell lists need remaking; coef_exposed: a coefficient's device
   // address was handed out, so they are remade at every call that uses them
   bool lists_dirty = true, coef_exposed = false;
+  // the coefficients are as cfmg_setup_operators left them; dirt[lev - 1]: the
+  // fields (bit per CFMG_X .. CFMG_Y) of a level that may hold values outside
+  // its wet interior (written by the caller or by the setup, not zeroed since)
+  bool coef_setup = false;
+  std::vector<unsigned> dirt;
+  bool graph_steps = false;  // whether the captured graphs were made with steps_clean (see step_ok)
   std::unordered_map<std::string, size_t> tail_cache;
   bool tb_on = true;  // temporally blocked FP32 smoothing on fine levels
   bool fuse_on = true;  // V-cycle descent: residual and restriction in the last pre-smoothing pass
@@ -108,6 +114,7 @@ struct cfmg_handle {
   bool record_epi = false;  // while recording: the last such pass takes its descent step's epilogue
 };
 
+constexpr unsigned kDirtExposed = 1u << 31;  // dirt: a coarse field's device address was handed out
 constexpr int kProgPoolOps = 8192;  // device store of engine programs (~1.9 MB)
 constexpr size_t kTailPoolBytes = 1 << 21;  // device store of coarse-tail programs
 
@@ -1195,8 +1202,51 @@ int resid_restrict3d(cfmg_handle* h, int lev) {
   return CFMG_OK;
 }
 
+// FP64 2D levels below the first whose descent and ascent steps run as one
+// launch each (k_tbg.cu): the coefficients are the setup's, every field of
+// levels 2.. holds +0 outside the wet interior, omega <= 1, and the level is
+// small enough that its launches cost more than its work. At 262^2 a 5-point
+// step with 2 pairs takes 10 us against 18 us for its 7 launches; at 518^2 the
+// halo's extra FP64 work uses the gain up.
+constexpr long long kStepCells = 150000;
+bool steps_clean(const cfmg_handle* h) {
+  if (!h->coef_setup || h->coef_exposed) return false;
+  for (int k = 2; k <= L(h); ++k)
+    if (h->dirt[k - 1]) return false;
+  return true;
+}
+bool step_ok(const cfmg_handle* h, int lev) {
+  if (!h->fuse_on || h->record || threed(h) || xperio(h) || lev < 2 || lev >= L(h) || h->d.omega > 1.0) return false;
+  if (h->d.npre < 1 || h->d.npre > kTbgMaxPairs || h->d.npost < 1 || h->d.npost > kTbgMaxPairs) return false;
+  const Level& l = h->lv[lev - 1];
+  return l.s64 && !in_engine(h, lev, CFMG_FP64) && steps_clean(h);
+}
+
+int step2d(cfmg_handle* h, int lev, int mode, int np) {
+  const Level& l = h->lv[lev - 1];
+  const Level& c = h->lv[lev];
+  TRY(flush(h));
+  TbgArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.xs = l.s64; a.b = l.b; a.w = l.widiag; a.cE = l.cE; a.cN = l.cN; a.d = l.diag; a.pc = l.Pcoef;
+  a.xc = c.x; a.rc = c.Rcoef; a.m = l.msk;
+  a.x = l.x; a.y = l.y; a.r = l.r; a.s = l.s64; a.bc = c.b; a.xcz = c.x;
+  a.cff = 1.0 - h->d.omega;
+  a.np = np;
+  a.tx = l.tx; a.ty = l.ty; a.nh = l.nh; a.ctx = c.tx; a.cty = c.ty;
+  a.np_i = (l.nx + 1) / 2; a.np_j = (l.ny + 1) / 2;
+  {
+    Launch k(h, mode == 2 ? CFMG_K_SWEEP : CFMG_K_DESCENT, lev, CFMG_FP64);
+    launch_step2d(a, h->d.op == CFMG_LAPLACIAN9 ? TAIL_9 : h->d.op == CFMG_VARCOEF ? TAIL_VC : TAIL_5, mode,
+                  vertices(h), h->stream);
+  }
+  LAUNCH_OK(h);
+  return CFMG_OK;
+}
+
+// zero_coarse = false: nothing reads the coarse x before it is written
 template <class T>
-int descend_t(cfmg_handle* h, int lev, int nite) {
+int descend_t(cfmg_handle* h, int lev, int nite, bool zero_coarse = true) {
   if (sizeof(T) == 4 && fused_descent_ok(h, lev)) return smooth_tb_epi(h, lev, nite);
   if (sizeof(T) == 4 && resid_restrict3d_ok(h, lev)) {
     TRY(smooth_t<T>(h, lev, nite));
@@ -1206,17 +1256,26 @@ int descend_t(cfmg_handle* h, int lev, int nite) {
   TRY(smooth_t<T>(h, lev, nite));
   TRY(residual_t<T>(h, lev));
   TRY(restrict_t<T>(h, lev, CFMG_R));
-  return zero_t<T>(h, lev + 1, CFMG_X);
+  return zero_coarse ? zero_t<T>(h, lev + 1, CFMG_X) : CFMG_OK;
 }
 
-// vcycle! (src/gmg_cycles.jl:67-83)
+// vcycle! (src/gmg_cycles.jl:67-83). prolonged: level lev0 takes its one-launch
+// steps, the first of which does the prolongation that the F-cycle left out
 template <class T>
-int vcycle_t(cfmg_handle* h, int lev0) {
+int vcycle_t(cfmg_handle* h, int lev0, bool prolonged = false) {
   const cfmg_desc& d = h->d;
   const int nl = L(h);
-  for (int lev = lev0; lev <= nl - 1; ++lev) TRY(descend_t<T>(h, lev, d.npre));
+  auto step = [&](int lev) { return sizeof(T) == 8 && (lev > lev0 || prolonged) && step_ok(h, lev); };
+  for (int lev = lev0; lev <= nl - 1; ++lev) {
+    if (step(lev)) TRY(step2d(h, lev, lev > lev0 ? 0 : 1, d.npre));
+    else TRY(descend_t<T>(h, lev, d.npre, !(lev + 1 < nl && step(lev + 1))));
+  }
   TRY(coarsest_t<T>(h, d.ndeepest));
   for (int lev = nl - 1; lev >= lev0; --lev) {
+    if (step(lev)) {
+      TRY(step2d(h, lev, 2, d.npost));
+      continue;
+    }
     TRY(prolong_t<T>(h, lev));
     // level 1's post-smoothing is the cycle's last step: with upd_req its
     // last pass may also apply the FP64 solution update
@@ -1241,12 +1300,14 @@ int fcycle_t(cfmg_handle* h, bool x1_zero = false) {
   const bool lazy = sizeof(T) == 4 && !xperio(h);
   for (int lev = 1; lev <= nl - 1; ++lev) {
     TRY(restrict_t<T>(h, lev, lev > 1 ? CFMG_B : CFMG_R));
-    if (!lazy || lev + 1 == nl) TRY(zero_t<T>(h, lev + 1, CFMG_X));  // the coarsest solve reads it
+    const bool step = sizeof(T) == 8 && step_ok(h, lev + 1);  // its first step assigns x
+    if ((!lazy && !step) || lev + 1 == nl) TRY(zero_t<T>(h, lev + 1, CFMG_X));  // the coarsest solve reads it
   }
   TRY(coarsest_t<T>(h, h->d.ndeepest));
   for (int lev = nl - 1; lev >= 1; --lev) {
-    TRY(prolong_t<T>(h, lev, lev >= 2 ? lazy : x1_zero));
-    TRY(vcycle_t<T>(h, lev));
+    const bool step = sizeof(T) == 8 && step_ok(h, lev);
+    if (!step) TRY(prolong_t<T>(h, lev, lev >= 2 ? lazy : x1_zero));
+    TRY(vcycle_t<T>(h, lev, step));
   }
   return CFMG_OK;
 }
@@ -2060,6 +2121,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
   cfmg_handle* h = new cfmg_handle();
   h->d = *d;
   h->lv = create_levels(*d);
+  h->dirt.assign(h->lv.size(), 0u);
   if (cudaGetDevice(&h->device) != cudaSuccess) {
     delete h;
     return fail(nullptr, CFMG_ERR_CUDA, "no CUDA device");
@@ -2071,6 +2133,9 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
   const bool coded = mixed && d->kase == CFMG_THREED && d->op == CFMG_LAPLACIAN;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t tail_bytes = shared ? 0 : kTailPoolBytes;
+  auto stepped = [&](const Level& l) {
+    return !shared && !l.threed && l.tz == 1 && (long long)l.len <= kStepCells && &l != &h->lv[0];
+  };
   auto tailed = [&](const Level& l) { return l.len <= (size_t)kTailMaxLen; };
   size_t total = al(kPartials * sizeof(double)) + al(S_COUNT * sizeof(double)) + al((size_t)pool_ops * sizeof(Op)) +
                  al(tail_bytes);
@@ -2083,6 +2148,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
     total += (mixed && vc ? 2 : 0) * al(n * 4);
     total += coded ? al(n) : 0;               // wq
     total += tailed(l) ? al(kTailListHdr + 2 * n) : 0;  // tlist
+    total += stepped(l) ? al(n * 8) : 0;                // s64
   }
   total += coded ? al(256 * sizeof(float)) : 0;  // wtab
   if (cudaMalloc(&h->arena, total) != cudaSuccess) {
@@ -2118,6 +2184,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
     }
     if (coded) l.wq = (uint8_t*)take(n);
     if (tailed(l)) l.tlist = (unsigned char*)take(kTailListHdr + 2 * n);
+    if (stepped(l)) l.s64 = (double*)take(n * 8);
   }
   if (coded) h->wtab = (float*)take(256 * sizeof(float));
   // the fixed-point residual pass reads kResidIntReach elements beside level
@@ -2237,6 +2304,7 @@ int cfmg_field_ptr(cfmg_handle* h, int lev, int field, void** dptr) {
   void* p = field_any(h->lv[lev - 1], field, &elt);
   if (!p || !dptr) return fail(h, CFMG_ERR_ARG, "unknown field (kappa exists only for the varcoef operator)");
   if (field >= CFMG_DIAG) h->coef_exposed = true;
+  else if (lev > 1) h->dirt[lev - 1] |= kDirtExposed;
   *dptr = p;
   return CFMG_OK;
 }
@@ -2246,7 +2314,10 @@ static int refresh_derived(cfmg_handle* h, int lev, int field) {
   if (field == CFMG_IDIAG) launch_widiag(l.idiag, l.widiag, h->d.omega, l.len, h->stream);
   if (h->d.op == CFMG_VARCOEF && (field == CFMG_KAPPA || field == CFMG_MSK))
     launch_face_coef(l.kappa, l.msk, l.cE, l.cN, geom(l), h->stream);
-  if (field >= CFMG_DIAG) h->mixed_dirty = h->lists_dirty = true;
+  if (field >= CFMG_DIAG) {
+    h->mixed_dirty = h->lists_dirty = true;
+    h->coef_setup = false;
+  }
   LAUNCH_OK(h);
   return CFMG_OK;
 }
@@ -2259,6 +2330,7 @@ int cfmg_upload(cfmg_handle* h, int lev, int field, const void* src) {
   if (!p || !src) return fail(h, CFMG_ERR_ARG, "unknown field or null source");
   CUDA_OK(h, cudaMemcpyAsync(p, src, l.len * elt, cudaMemcpyDefault, h->stream));
   TRY(refresh_derived(h, lev, field));
+  if (field < CFMG_DIAG) h->dirt[lev - 1] |= 1u << field;
   if (field >= CFMG_DIAG && field != CFMG_MSK && field != CFMG_KAPPA) h->coef_set = true;
   h->solved = false;
   return sync(h);
@@ -2288,6 +2360,7 @@ int cfmg_bind_level(cfmg_handle* h, int lev, const double* diag, const double* i
   if (msk) TRY(refresh_derived(h, lev, CFMG_MSK));
   h->mixed_dirty = h->lists_dirty = true;
   h->coef_set = true;
+  h->coef_setup = false;
   h->solved = false;
   return sync(h);
 }
@@ -2298,6 +2371,7 @@ int cfmg_set_default_msk(cfmg_handle* h) {
   launch_default_msk(DEFMSK_SET, l.msk, nullptr, 0.0, l, vertices(h), threed(h), xperio(h), h->stream);
   LAUNCH_OK(h);
   h->lists_dirty = true;
+  h->coef_setup = false;
   return sync(h);
 }
 
@@ -2306,6 +2380,8 @@ int cfmg_setup_operators(cfmg_handle* h) {
   TRY(setup_operators(h));
   TRY(sync(h));
   h->coef_set = true;
+  h->coef_setup = true;
+  for (unsigned& q : h->dirt) q |= 1u << CFMG_X | 1u << CFMG_R | 1u << CFMG_B | 1u << CFMG_Y;  // its scratch
   h->solved = false;
   return CFMG_OK;
 }
@@ -2350,6 +2426,7 @@ int cfmg_zero(cfmg_handle* h, int lev, int field) {
   void* p = field_any(l, field, &elt);
   if (!p) return fail(h, CFMG_ERR_ARG, "unknown field");
   CUDA_OK(h, cudaMemsetAsync(p, 0, l.len * elt, h->stream));
+  if (field < CFMG_DIAG) h->dirt[lev - 1] &= ~(1u << field);
   if (field >= CFMG_DIAG) TRY(refresh_derived(h, lev, field));
   return CFMG_OK;
 }
@@ -2362,7 +2439,10 @@ int cfmg_fill(cfmg_handle* h, int lev, int field) {
   if (!p) return fail(h, CFMG_ERR_ARG, "unknown field");
   if (!xperio(h)) return CFMG_OK;
   TRY(flush(h));
-  if (field >= CFMG_DIAG) h->lists_dirty = true;
+  if (field >= CFMG_DIAG) {
+    h->lists_dirty = true;
+    h->coef_setup = false;
+  }
   if (elt == 1) launch_fill_xperio<uint8_t>((uint8_t*)p, geom(l), h->stream);
   else launch_fill_xperio<double>((double*)p, geom(l), h->stream);
   LAUNCH_OK(h);
@@ -2435,6 +2515,11 @@ int cfmg_solve(cfmg_handle* h, double* res_out, int* nite_out, double* history) 
     return fail(h, CFMG_ERR_UNSUPPORTED, "the mixed-precision form runs V and F cycles");
   if (prec == CFMG_MIXED) TRY(prepare_mixed(h));
   TRY(tail_lists(h));
+  if (steps_clean(h) != h->graph_steps) {  // the captured iterations took the other route
+    TRY(sync(h));
+    drop_graphs(h);
+    h->graph_steps = steps_clean(h);
+  }
   // normb = norm(mg, 1, :b) (src/gmg_solver.jl:22)
   const Level& l1 = h->lv[0];
   TRY(flush(h));

@@ -257,44 +257,8 @@ __device__ __noinline__ void tail_restrict(const TailOp* opp) {
   }
 }
 
-// d_prolong's value of one child before its Pcoef: a thread per child instead
-// of per parent, since a parent's 29 FP64 instructions in one warp took 1.1 us
-// on a level of 16 parents; each child's sum is formed in d_prolong's order.
-template <class T, int K>
-__device__ __forceinline__ T tail_child(const T* x, long long C, long long c1, long long c2, int ch) {
-  typedef Ar<T> A;
-  const int di = ch & 1, dj = (ch >> 1) & 1, dk = ch >> 2;
-  if (K == 0) return A::add(square3(x, C, (long long)(2 * di - 1), (2 * dj - 1) * c1, 0LL), A::mul(x[C], T(9)));
-  if (K == 1) {
-    const long long ddi = 2 * di - 1, ddj = (2 * dj - 1) * c1;
-    const T bb = A::mul(square3(x, C, ddi, ddj, 0LL), T(3));
-    return A::add(A::add(bb, square3(x, C, ddi, ddj, dk ? c2 : -c2)), A::mul(x[C], T(28)));
-  }
-  T v = x[C];
-  if (K == 2) {
-    if (di) v = A::add(v, x[C + 1]);
-    if (dj) v = A::add(v, x[C + c1]);
-    return di && dj ? A::add(v, x[C + 1 + c1]) : v;
-  }
-  const T x100 = x[C + 1], x010 = x[C + c1], x001 = x[C + c2];
-  switch (ch) {
-    case 0: return v;
-    case 1: return A::add(v, x100);
-    case 2: return A::add(v, x010);
-    case 4: return A::add(v, x001);
-    case 3: return A::add(A::add(A::add(v, x100), x010), x[C + 1 + c1]);
-    case 5: return A::add(A::add(A::add(v, x100), x001), x[C + 1 + c2]);
-    case 6: return A::add(A::add(A::add(v, x001), x010), x[C + c1 + c2]);
-    default: break;
-  }
-  v = A::add(v, x100);
-  v = A::add(v, x001);
-  v = A::add(v, x[C + 1 + c2]);
-  v = A::add(v, x010);
-  v = A::add(v, x[C + 1 + c1]);
-  v = A::add(v, x[C + c1 + c2]);
-  return A::add(v, x[C + 1 + c1 + c2]);
-}
+// a thread per child instead of per parent: a parent's 29 FP64 instructions in
+// one warp took 1.1 us on a level of 16 parents
 template <class T, int K>
 __device__ __noinline__ void tail_prolong(const TailOp* opp) {
   const TailOp& op = *opp;
@@ -312,7 +276,7 @@ __device__ __noinline__ void tail_prolong(const TailOp* opp) {
     const int k = t3 ? nh + 1 + 2 * (int)r : op.kf0 + (int)r;
     const long long C = lin(gc, f2c(i, nh), f2c(j, nh), t3 ? f2c(k, nh) : k);
     const long long F = lin(g, i + (int)(ch & 1), j + (int)((ch >> 1) & 1), k + (int)(ch >> 2));
-    y[F] = Ar<T>::add(y[F], Ar<T>::mul(coef[F], tail_child<T, K>(x, C, gc.n1, gc.n2, (int)ch)));
+    y[F] = Ar<T>::add(y[F], Ar<T>::mul(coef[F], prolong_child<T, K>(x, C, gc.n1, gc.n2, (int)ch)));
   }
 }
 

@@ -502,6 +502,43 @@ __device__ __forceinline__ void d_prolong(T* xf, const T* x, const T* coef, cons
   }
 }
 
+// d_prolong's value of one child (di = ch & 1, dj = ch >> 1 & 1, dk = ch >> 2)
+// of coarse cell C before its Pcoef, in d_prolong's order.
+template <class T, int K>
+__device__ __forceinline__ T prolong_child(const T* x, long long C, long long c1, long long c2, int ch) {
+  typedef Ar<T> A;
+  const int di = ch & 1, dj = (ch >> 1) & 1, dk = ch >> 2;
+  if (K == 0) return A::add(square3(x, C, (long long)(2 * di - 1), (2 * dj - 1) * c1, 0LL), A::mul(x[C], T(9)));
+  if (K == 1) {
+    const long long ddi = 2 * di - 1, ddj = (2 * dj - 1) * c1;
+    const T bb = A::mul(square3(x, C, ddi, ddj, 0LL), T(3));
+    return A::add(A::add(bb, square3(x, C, ddi, ddj, dk ? c2 : -c2)), A::mul(x[C], T(28)));
+  }
+  T v = x[C];
+  if (K == 2) {
+    if (di) v = A::add(v, x[C + 1]);
+    if (dj) v = A::add(v, x[C + c1]);
+    return di && dj ? A::add(v, x[C + 1 + c1]) : v;
+  }
+  const T x100 = x[C + 1], x010 = x[C + c1], x001 = x[C + c2];
+  switch (ch) {
+    case 0: return v;
+    case 1: return A::add(v, x100);
+    case 2: return A::add(v, x010);
+    case 4: return A::add(v, x001);
+    case 3: return A::add(A::add(A::add(v, x100), x010), x[C + 1 + c1]);
+    case 5: return A::add(A::add(A::add(v, x100), x001), x[C + 1 + c2]);
+    case 6: return A::add(A::add(A::add(v, x001), x010), x[C + c1 + c2]);
+    default: break;
+  }
+  v = A::add(v, x100);
+  v = A::add(v, x001);
+  v = A::add(v, x[C + 1 + c2]);
+  v = A::add(v, x010);
+  v = A::add(v, x[C + 1 + c1]);
+  v = A::add(v, x[C + c1 + c2]);
+  return A::add(v, x[C + 1 + c1 + c2]);
+}
 // FP64 parent whose update changes nothing: its children's Pcoef and fine x
 // are all +0, and every coarse value it reads is finite with room for the
 // weights (below 2^1009), so +0 + 0*v = +0

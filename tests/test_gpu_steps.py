@@ -1,0 +1,81 @@
+"""The one-launch descent and ascent steps of FP64 2D levels (k_tbg.cu) against
+the separate kernels (option fused_descent = 0): every field of every level
+after cycles, bit for bit: the same operations in the same order, tolerance
+zero. Sizes put tile edges inside, at and beyond the array, on levels through
+odd extents."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+cfmg = pytest.importorskip("cfmg")
+
+
+def _make(fused, nx, ny, seed, upload=None, **p):
+    rng = np.random.default_rng(seed)
+    mg = cfmg.get_gmg(cfmg.Param(nx=nx, ny=ny, nz=1, case="twod", verbose=False, **p))
+    mg.set_option("fused_descent", fused)
+    shape = mg.shape(1)
+    i, j = np.arange(shape[0])[:, None, None] / shape[0], np.arange(shape[1])[None, :, None] / shape[1]
+    wet = ((i - 0.5) ** 2 + (j - 0.45) ** 2 < 0.18) & (rng.random(shape) > 0.002)
+    mg.oper[1].msk = np.asfortranarray(wet.astype(np.uint8))
+    if p.get("operator") == "varcoef":
+        mg.oper[1].kappa = np.exp(0.5 * rng.standard_normal(shape))
+    cfmg.setup_operators(mg)
+    for lev in range(1, mg.nlevels + 1):
+        for f in ("x", "y", "r", "b"):
+            cfmg.set_to_zero(mg, lev, f)
+    m = mg.download(1, "msk").astype(np.float64)
+    b = rng.standard_normal(shape) * m
+    mg.data[1].b = b - m * (b.sum() / m.sum())
+    if upload:
+        mg.upload(2, upload, rng.standard_normal(mg.shape(2)))
+    return mg
+
+
+def _run(fused, *a, cycles=2, **p):
+    mg = _make(fused, *a, **p)
+    for _ in range(cycles):
+        cfmg.normresidual(mg, 1.0)
+        cfmg.cycle(mg)
+    out = {(lev, f): mg.download(lev, f) for lev in range(1, mg.nlevels + 1) for f in ("x", "y", "r", "b")}
+    res, nite, hist = cfmg.solve(mg, history=True, maxite=3, tol=0.0)
+    out["hist"], out["x"] = hist, mg.data[1].x
+    mg.close()
+    return out
+
+
+OPS = {
+    "5": dict(operator="laplacian"),
+    "5-vertices": dict(operator="laplacian", location="vertices"),
+    "9-vertices": dict(operator="laplacian9", location="vertices"),
+    "9": dict(operator="laplacian9"),
+    "varcoef": dict(operator="varcoef"),
+}
+
+
+@pytest.mark.parametrize("cycle", ["v", "f"])
+@pytest.mark.parametrize("name", list(OPS))
+@pytest.mark.parametrize("size,pairs", [((224, 160), (2, 2)), ((333, 270), (1, 3)), ((514, 390), (3, 1))])
+def test_steps_are_bit_identical(name, cycle, size, pairs):
+    p = dict(cycle=cycle, npre=pairs[0], npost=pairs[1], omega=0.8, nlevels=6, **OPS[name])
+    a, b = (_run(fused, *size, 7, **p) for fused in (1, 0))
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("upload", ["x", "b"])
+def test_values_outside_the_wet_interior_take_the_separate_kernels(upload):
+    """A caller's values in a coarse field (halo and land included) are what the reference's cycle sees; a solve
+    captured before them is captured again."""
+    p = dict(cycle="v", npre=2, npost=2, omega=0.8, nlevels=6)
+    out = []
+    for fused in (1, 0):
+        mg = _make(fused, 300, 220, 3, **p)
+        cfmg.solve(mg, maxite=2, tol=0.0)
+        mg.upload(2, upload, np.random.default_rng(1).standard_normal(mg.shape(2)))
+        cfmg.solve(mg, maxite=2, tol=0.0)
+        out.append([mg.download(lev, f) for lev in (1, 2, 3) for f in ("x", "y", "r", "b")])
+        mg.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
