@@ -351,18 +351,25 @@ bool coarsest_in_fp64(const cfmg_handle* h) {
 // levels of more than 6/5 of the engine's FP64 threshold (1500 cells by
 // default) stay out, because one SM's FP64 pipe then takes longer for a sweep
 // than a launch on all SMs does: a 38^2 level with every cell wet takes
-// 2.1 us a sweep in the tail and 2.2 us as a launch.
+// 2.1 us a sweep in the tail and 2.2 us as a launch. Where the level's steps
+// can be one launch each (k_tbg.cu) the line lies at 2/5 of that, 600 cells: a
+// 38^2 disk level takes 21 us a cycle in the tail and 10 us as two steps.
 constexpr size_t kTailBlobReserve = 24 * 1024;
 constexpr size_t tail_al(size_t b) { return (b + 15) & ~(size_t)15; }
 size_t tail_hot_bytes(const cfmg_handle* h, const Level& l, int prec) {
   const size_t n = l.len, es = prec ? 4 : 8;
   return (h->d.op == CFMG_VARCOEF ? 6 : 4) * tail_al(n * es) + tail_al(kTailListHdr + 2 * n);
 }
+// whether the handle's FP64 levels can take one-launch steps (see step_ok)
+bool steps_form(const cfmg_handle* h) {
+  return !threed(h) && !xperio(h) && h->lv[0].tz == 1 && h->fuse_on && h->d.omega <= 1.0;
+}
 void plan_tail(cfmg_handle* h) {
+  h->lists_dirty = true;  // the levels that need lists may change
   for (int prec = 0; prec < 2; ++prec) {
     h->tail_from[prec] = 0;
     if (!h->engine_on || h->small_min <= 0 || (prec == 1 && h->d.precision != CFMG_MIXED)) continue;
-    const long long cap = prec == 0 ? engine_limit(h, 0) * 6 / 5 : engine_limit(h, 1);
+    const long long cap = prec == 0 ? engine_limit(h, 0) * 6 / 5 * 2 / (steps_form(h) ? 5 : 2) : engine_limit(h, 1);
     size_t used = kTailBlobReserve;
     if (prec == 1 && coarsest_in_fp64(h)) used += tail_hot_bytes(h, h->lv.back(), 0);
     for (int lev = L(h); lev >= 1 && L(h) - lev < kTailMaxCtx - 2; --lev) {
@@ -653,7 +660,8 @@ int tail_lists(cfmg_handle* h) {
   int n = 0;
   for (int lev = L(h); lev >= 1 && n < kTailMaxCtx; --lev) {
     const Level& l = h->lv[lev - 1];
-    if (!l.tlist) break;
+    if (!l.tlist || !((h->tail_from[0] > 0 && lev >= h->tail_from[0]) || (h->tail_from[1] > 0 && lev >= h->tail_from[1])))
+      break;
     TailListLevel& q = a.lev[n++];
     q.w = l.widiag; q.pc = l.Pcoef; q.m = l.msk; q.out = l.tlist;
     q.len = (int)l.len; q.n1 = l.tx; q.nj = l.ty;
@@ -720,7 +728,8 @@ bool in_engine(const cfmg_handle* h, int lev, int prec) {
   if (!h->engine_on) return false;
   if (in_tail(h, lev, prec)) return true;
   if ((long long)h->lv[lev - 1].len > engine_limit(h, prec)) return false;
-  return !(prec && blocked_form(h, lev));
+  // FP64 levels between the tail and the threshold take one-launch steps
+  return !(prec ? blocked_form(h, lev) : h->tail_pool && h->tail_from[0] > 0 && steps_form(h));
 }
 
 int emit(cfmg_handle* h, const Op& op) {
@@ -1202,13 +1211,16 @@ int resid_restrict3d(cfmg_handle* h, int lev) {
   return CFMG_OK;
 }
 
-// FP64 2D levels below the first whose descent and ascent steps run as one
-// launch each (k_tbg.cu): the coefficients are the setup's, every field of
-// levels 2.. holds +0 outside the wet interior, omega <= 1, and the level is
-// small enough that its launches cost more than its work. At 262^2 a 5-point
-// step with 2 pairs takes 10 us against 18 us for its 7 launches; at 518^2 the
-// halo's extra FP64 work uses the gain up.
-constexpr long long kStepCells = 150000;
+// FP64 2D levels whose descent and ascent steps run as one launch each
+// (k_tbg.cu): the coefficients are the setup's, every field of levels 2..
+// holds +0 outside the wet interior, omega <= 1, and the level is small enough
+// that its launches cost more than the halo's extra FP64 work. The line is
+// drawn in FP64 operations a sweep (7 a cell for the 5-point operator, 11 for
+// the others): 800 000, as 262^2 9-point cells (a 2048^2 F-cycle solve takes 8 %
+// less with that level in steps); 400 000 on level 1, where a 262^2 5-point
+// level lost 1.5 % of its solve and a 390 x 294 variable-coefficient one 10 %.
+constexpr long long kStepCells = 150000;  // levels that get the scratch array
+constexpr long long kStepWork = 800000, kStepWork1 = 400000;
 bool steps_clean(const cfmg_handle* h) {
   if (!h->coef_setup || h->coef_exposed) return false;
   for (int k = 2; k <= L(h); ++k)
@@ -1216,9 +1228,10 @@ bool steps_clean(const cfmg_handle* h) {
   return true;
 }
 bool step_ok(const cfmg_handle* h, int lev) {
-  if (!h->fuse_on || h->record || threed(h) || xperio(h) || lev < 2 || lev >= L(h) || h->d.omega > 1.0) return false;
+  if (h->record || !steps_form(h) || lev >= L(h)) return false;
   if (h->d.npre < 1 || h->d.npre > kTbgMaxPairs || h->d.npost < 1 || h->d.npost > kTbgMaxPairs) return false;
   const Level& l = h->lv[lev - 1];
+  if ((long long)l.len * (h->d.op == CFMG_LAPLACIAN ? 7 : 11) > (lev == 1 ? kStepWork1 : kStepWork)) return false;
   return l.s64 && !in_engine(h, lev, CFMG_FP64) && steps_clean(h);
 }
 
@@ -1228,9 +1241,11 @@ int step2d(cfmg_handle* h, int lev, int mode, int np) {
   TRY(flush(h));
   TbgArgs a;
   std::memset(&a, 0, sizeof(a));
-  a.xs = l.s64; a.b = l.b; a.w = l.widiag; a.cE = l.cE; a.cN = l.cN; a.d = l.diag; a.pc = l.Pcoef;
+  const bool first = lev == 1 && mode != 2;  // the descent of level 1 starts from x and leaves x and y alone
+  a.xs = mode == 2 ? l.s64 : first ? l.x : nullptr;
+  a.b = l.b; a.w = l.widiag; a.cE = l.cE; a.cN = l.cN; a.d = l.diag; a.pc = l.Pcoef;
   a.xc = c.x; a.rc = c.Rcoef; a.m = l.msk;
-  a.x = l.x; a.y = l.y; a.r = l.r; a.s = l.s64; a.bc = c.b; a.xcz = c.x;
+  a.x = first ? nullptr : l.x; a.y = first ? nullptr : l.y; a.r = l.r; a.s = l.s64; a.bc = c.b; a.xcz = c.x;
   a.cff = 1.0 - h->d.omega;
   a.np = np;
   a.tx = l.tx; a.ty = l.ty; a.nh = l.nh; a.ctx = c.tx; a.cty = c.ty;
@@ -1259,15 +1274,15 @@ int descend_t(cfmg_handle* h, int lev, int nite, bool zero_coarse = true) {
   return zero_coarse ? zero_t<T>(h, lev + 1, CFMG_X) : CFMG_OK;
 }
 
-// vcycle! (src/gmg_cycles.jl:67-83). prolonged: level lev0 takes its one-launch
-// steps, the first of which does the prolongation that the F-cycle left out
+// vcycle! (src/gmg_cycles.jl:67-83). prolonged: the F-cycle left the
+// prolongation onto lev0 to the one-launch step that starts here
 template <class T>
 int vcycle_t(cfmg_handle* h, int lev0, bool prolonged = false) {
   const cfmg_desc& d = h->d;
   const int nl = L(h);
-  auto step = [&](int lev) { return sizeof(T) == 8 && (lev > lev0 || prolonged) && step_ok(h, lev); };
+  auto step = [&](int lev) { return sizeof(T) == 8 && (lev > lev0 || lev == 1 || prolonged) && step_ok(h, lev); };
   for (int lev = lev0; lev <= nl - 1; ++lev) {
-    if (step(lev)) TRY(step2d(h, lev, lev > lev0 ? 0 : 1, d.npre));
+    if (step(lev)) TRY(step2d(h, lev, lev == lev0 && prolonged ? 1 : 0, d.npre));
     else TRY(descend_t<T>(h, lev, d.npre, !(lev + 1 < nl && step(lev + 1))));
   }
   TRY(coarsest_t<T>(h, d.ndeepest));
@@ -2134,7 +2149,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t tail_bytes = shared ? 0 : kTailPoolBytes;
   auto stepped = [&](const Level& l) {
-    return !shared && !l.threed && l.tz == 1 && (long long)l.len <= kStepCells && &l != &h->lv[0];
+    return !shared && !l.threed && l.tz == 1 && (long long)l.len <= kStepCells;
   };
   auto tailed = [&](const Level& l) { return l.len <= (size_t)kTailMaxLen; };
   size_t total = al(kPartials * sizeof(double)) + al(S_COUNT * sizeof(double)) + al((size_t)pool_ops * sizeof(Op)) +
@@ -3429,6 +3444,7 @@ int cfmg_set_option(cfmg_handle* h, int option, long long value) {
   }
   if (option == CFMG_OPT_FUSED_DESCENT) {
     h->fuse_on = value != 0;
+    plan_tail(h);
     drop_graphs(h);
     return CFMG_OK;
   }

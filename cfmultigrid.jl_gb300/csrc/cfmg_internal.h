@@ -315,7 +315,8 @@ void launch_tail_lists(const TailListArgs& a, int n, cudaStream_t s);
 // ---- a descent or ascent step of an FP64 2D level in one launch (k_tbg.cu)
 constexpr int kTbgMaxPairs = 3;
 struct TbgArgs {
-  const double *xs;                          // ascent: the descent's result (the level's scratch)
+  const double *xs;                          // ascent: the descent's result (the level's scratch); descent
+                                             // of level 1: its x (x and y null: only s is written)
   const double *b, *w, *cE, *cN, *d, *pc;    // pc: the level's Pcoef
   const double *xc, *rc;                     // coarse x (prolonged), coarse Rcoef
   const uint8_t* m;
@@ -323,8 +324,8 @@ struct TbgArgs {
   double cff;
   int np, tx, ty, nh, ctx, cty, np_i, np_j;  // np: pairs of sweeps; np_i x np_j prolongation parents
 };
-// stencil TAIL_5 / TAIL_9 / TAIL_VC; mode 0: descent from x = +0, 1: descent
-// from x = Pcoef P(coarse x), 2: ascent
+// stencil TAIL_5 / TAIL_9 / TAIL_VC; mode 0: descent from x = +0 (or xs), 1:
+// descent from x = +0 (or xs) + Pcoef P(coarse x), 2: ascent
 void launch_step2d(const TbgArgs& a, int stencil, int mode, bool vertices, cudaStream_t s);
 
 // 3D 7-point streaming blocked passes (k_tb3d.cu): nite (1 or 2) pairs over U

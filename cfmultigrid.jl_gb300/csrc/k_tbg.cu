@@ -13,12 +13,17 @@
 // Each sweep covers the tile's cells that later ones need: sweep s leaves a
 // margin of s + 1 cells. The tiles overlap, so a step must not read what it
 // writes: a descent reads no x at all, and leaves a copy of its result in the
-// level's scratch array, which is what the ascent reads.
+// level's scratch array, which is what the ascent reads. Level 1 starts from
+// the caller's x; its descent writes the scratch only, and the ascent x and y.
 //
 // Every cell of the tile is updated by the same formula, which rests on the
 // coefficients that setup_operators made (the caller checks that they are)
 // and on omega <= 1: outside the wet interior x, y and the coarse levels' x
-// hold +0 and omega*idiag, Pcoef are +0, so the formula leaves +0 there. The
+// hold +0 and omega*idiag, Pcoef are +0, so the formula leaves +0 there. (On
+// level 1 x may hold anything there: with omega*idiag = +0 the formula is the
+// reference's (1-omega) x in its sweep range, and cells out of range matter to
+// no cell with omega*idiag != 0; the 9-point operator's second sweep, over the
+// interior only, leaves the others alone.) The
 // arithmetic per cell is that of the separate kernels, and x, y, r and the
 // coarse b and x receive what those would leave: the same bits.
 //
@@ -106,7 +111,7 @@ __global__ void __launch_bounds__(kGThreads) k_step2d(TbgArgs a, int S, int core
     const bool in = gi >= 1 && gi <= tx && gj >= 1 && gj <= ty;
     const long long I = in ? (long long)(gi - 1) + (long long)tx * (gj - 1) : 0;
     double xv = 0.0;
-    if (MODE == 2 && in) xv = a.xs[I];
+    if ((MODE == 2 || a.xs) && in) xv = a.xs[I];
     B[t] = in ? a.b[I] : 0.0;
     W[t] = in ? a.w[I] : 0.0;
     if (ST == TAIL_VC) {
@@ -139,6 +144,10 @@ __global__ void __launch_bounds__(kGThreads) k_step2d(TbgArgs a, int S, int core
       sq.at(t, i, j);
       const int L = (j + s + 1) * S + i + s + 1;
       const double b = B[L], w = W[L];
+      if (ST == TAIL_9 && (s & 1)) {  // the interior only
+        const int gi = i0 + i + s + 1, gj = j0 + j + s + 1;
+        if (gi <= nh || gi > tx - nh || gj <= nh || gj > ty - nh) continue;
+      }
       double v = 0.0;
       if (!__all_sync(__activemask(), g_land<ST>(src, L, S, b, w))) v = g_cell<ST>(src, L, S, b, w, a.cff, E, N);
       dst[L] = v;
@@ -157,11 +166,9 @@ __global__ void __launch_bounds__(kGThreads) k_step2d(TbgArgs a, int S, int core
     const bool r1 = ST == TAIL_9 ? gi >= nh && gi <= tx - nh + 1 && gj >= nh && gj <= ty - nh + 1
                                  : gj >= 2 && gj <= ty - 1;
     const bool r2 = ST == TAIL_9 ? gi > nh && gi <= tx - nh && gj > nh && gj <= ty - nh : r1;
-    if (r1) a.y[I] = Y[L];
-    if (r2) {
-      a.x[I] = X[L];
-      if (MODE != 2) a.s[I] = X[L];
-    }
+    if (r1 && a.y) a.y[I] = Y[L];
+    if (r2 && a.x) a.x[I] = X[L];
+    if (MODE != 2 && (r2 || a.xs)) a.s[I] = X[L];  // level 1's x out of range counts too
   }
   if (MODE == 2) return;
   __syncthreads();

@@ -64,6 +64,23 @@ def test_steps_are_bit_identical(name, cycle, size, pairs):
         assert np.array_equal(a[k], b[k]), k
 
 
+@pytest.mark.parametrize("cycle", ["v", "f"])
+@pytest.mark.parametrize("name", list(OPS))
+def test_first_level_step_of_any_x(name, cycle):
+    """Level 1 in the steps: the caller's x holds values in land and halo cells."""
+    p = dict(cycle=cycle, npre=2, npost=2, omega=0.8, nlevels=4, **OPS[name])
+    out = []
+    for fused in (1, 0):
+        mg = _make(fused, 150, 118, 5, **p)
+        mg.data[1].x = np.random.default_rng(2).standard_normal(mg.shape(1))
+        cfmg.normresidual(mg, 1.0)
+        cfmg.cycle(mg)
+        out.append([mg.download(lev, f) for lev in range(1, mg.nlevels + 1) for f in ("x", "y", "r", "b")])
+        mg.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("upload", ["x", "b"])
 def test_values_outside_the_wet_interior_take_the_separate_kernels(upload):
     """A caller's values in a coarse field (halo and land included) are what the reference's cycle sees; a solve
