@@ -446,7 +446,7 @@ bool build_tail(const cfmg_handle* h, const std::vector<Op>& P, std::vector<Tail
                     : a.kind == OPK_SWEEP19 ? TAIL_19 : TAIL_VC;
         c.prec = a.prec;
         c.n1 = (int)a.g.n1; c.n2 = (int)a.g.n2;
-        c.lines = l.ty * l.tz; c.nh = l.nh;
+        c.lines = l.ty * l.tz; c.nh = l.nh; c.nx = l.nx;
         c.cff = a.cff;
         ctxs.push_back(c);
         const bool vc = a.kind == OPK_SWEEPVC;
@@ -866,7 +866,7 @@ int smooth_tb(cfmg_handle* h, int lev, int nite) {
       }
       l.xswap ^= 1;
       left -= n;
-      TRY(fill_if<float>(h, lev, view<float>(l).x));
+      if (l.nx < l.nh) TRY(fill_if<float>(h, lev, view<float>(l).x));  // else the pass wrote the halo columns
     }
     LAUNCH_OK(h);
     return CFMG_OK;
@@ -1034,6 +1034,8 @@ int residual_t(cfmg_handle* h, int lev) {
   }
   TRY(emit(h, op));
   if (h->d.op == CFMG_LAPLACIAN9 && threed(h)) return CFMG_OK;  // residual_laplacian9!: no fill!
+  // the FP32 r of a cycle is only restricted, and a cell-centred restriction reads the interior
+  if (sizeof(T) == 4 && !vertices(h)) return CFMG_OK;
   return fill_if<T>(h, lev, v.r);
 }
 
@@ -1053,6 +1055,9 @@ int restrict_t(cfmg_handle* h, int lev, int field) {
   op.box = interior(c);
   op.n = box_count(op.box);
   TRY(emit(h, op));
+  // an FP32 level in periodic blocked passes reads the interior columns of b only
+  // (its residual's halo columns, where b is read too, are not used: see residual_t)
+  if (sizeof(T) == 4 && !vertices(h) && xperio(h) && lev + 1 < L(h) && tb_eligible<T>(h, lev + 1)) return CFMG_OK;
   return fill_if<T>(h, lev + 1, vc.b);
 }
 
@@ -1064,8 +1069,10 @@ int zero_t(cfmg_handle* h, int lev, int field);
 // so a standalone launch writes x = +0 + P x_coarse without reading it; the
 // caller then skips zeroing it. A level of the program engine is zeroed here
 // and prolonged as usual.
+// smoothed: a smoothing call of this level follows; in periodic blocked passes
+// that reads the interior columns only, so the halo columns are not filled.
 template <class T>
-int prolong_t(cfmg_handle* h, int lev, bool onto_zero = false) {
+int prolong_t(cfmg_handle* h, int lev, bool onto_zero = false, bool smoothed = false) {
   const Level& f = h->lv[lev - 1];
   const Level& c = h->lv[lev];
   View<T> vf = view<T>(f);
@@ -1097,6 +1104,7 @@ int prolong_t(cfmg_handle* h, int lev, bool onto_zero = false) {
     else TRY(zero_t<T>(h, lev, CFMG_X));
   }
   TRY(emit(h, op));
+  if (sizeof(T) == 4 && smoothed && xperio(h) && tb_eligible<T>(h, lev)) return CFMG_OK;
   return fill_if<T>(h, lev, vf.x);
 }
 
@@ -1291,7 +1299,7 @@ int vcycle_t(cfmg_handle* h, int lev0, bool prolonged = false) {
       TRY(step2d(h, lev, 2, d.npost));
       continue;
     }
-    TRY(prolong_t<T>(h, lev));
+    TRY(prolong_t<T>(h, lev, false, d.npost > 0));
     // level 1's post-smoothing is the cycle's last step: with upd_req its
     // last pass may also apply the FP64 solution update
     h->upd_now = sizeof(T) == 4 && lev == 1 && h->upd_req;
@@ -1321,7 +1329,7 @@ int fcycle_t(cfmg_handle* h, bool x1_zero = false) {
   TRY(coarsest_t<T>(h, h->d.ndeepest));
   for (int lev = nl - 1; lev >= 1; --lev) {
     const bool step = sizeof(T) == 8 && step_ok(h, lev);
-    if (!step) TRY(prolong_t<T>(h, lev, lev >= 2 ? lazy : x1_zero));
+    if (!step) TRY(prolong_t<T>(h, lev, lev >= 2 ? lazy : x1_zero, h->d.npre > 0));
     TRY(vcycle_t<T>(h, lev, step));
   }
   return CFMG_OK;

@@ -273,7 +273,7 @@ enum TailStencil { TAIL_5 = 0, TAIL_7, TAIL_9, TAIL_19, TAIL_VC };
 constexpr int TAIL_SMOOTH = 1000;  // TailOp kind: npairs pairs of sweeps of context ctxi
 constexpr int kTailListHdr = 16;  // bytes in front of a list: {listed cells, cells of the range}
 struct alignas(16) TailCtx {
-  int stencil, prec, n1, n2, lines, nh;  // lines: rows of the level (x-periodic fill)
+  int stencil, prec, n1, n2, lines, nh, nx;  // lines: rows of the level (x-periodic fill)
   unsigned ox, oy, ob, ow, oE, oN, olist;
   double cff;
 };
@@ -345,8 +345,9 @@ constexpr int kTbMaxPairs = 10;
 bool launch_smooth_tb(int version, int stencil, int nite, const float* x, float* xo, const float* b, const float* w,
                       float cff, int tx, int ty, int nz, int ui0, int ui1, int uj0, int uj1, cudaStream_t s);
 // the lean packed passes for the x-periodic topology, 5-point operator: the
-// tiles cover the interior columns [ui0, ui1] and read the periodic images
-// of the columns beside them; the caller fills the halo columns afterwards
+// tiles cover the interior columns [ui0, ui1], read the periodic images of
+// the columns beside them and write the images of the end columns (the caller
+// fills the halo columns of a level with nx < nh)
 bool launch_smooth_tb_periodic(int nite, const float* x, float* xo, const float* b, const float* w, float cff,
                                int tx, int ty, int nz, int ui0, int ui1, int uj0, int uj1, cudaStream_t s);
 // The last pass of a V-cycle's pre-smoothing with the step that follows it

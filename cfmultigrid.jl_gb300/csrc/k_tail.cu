@@ -72,9 +72,14 @@ __device__ __forceinline__ void bar_warps(int nw) {
   else asm volatile("bar.sync 1, %0;" ::"r"(nw * 32) : "memory");
 }
 
-// npairs pairs of sweeps over the listed cells
+// npairs pairs of sweeps over the listed cells. fill (x-periodic): fill! after
+// each pair, as the second sweep's writers of the nh columns at either end
+// writing their images in the halo (whose own cells are not swept then); a
+// fill of every line in a step of its own, with its barrier, took as long as
+// the two sweeps of a small level. whole: the list is the whole range (or
+// nx < nh): fills as the reference does.
 template <class T, int ST>
-__device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, int nact) {
+__device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, bool whole, int nact) {
   const TailCtx& c = reinterpret_cast<const TailCtx*>(sm)[ctxi];
   T* x = reinterpret_cast<T*>(sm + c.ox);
   T* y = reinterpret_cast<T*>(sm + c.oy);
@@ -85,8 +90,23 @@ __device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, int na
   const unsigned short* list = reinterpret_cast<const unsigned short*>(sm + c.olist + kTailListHdr);
   const T cff = (T)c.cff;
   const int n1 = c.n1, n2 = c.n2, tid = threadIdx.x;
-  if (nact <= 0) return;
-  if (!fill && nact <= kTT) {  // one cell a thread, the warps that hold cells only
+  if (nact <= 0 && !fill) return;
+  const bool img = fill && !whole && c.nx >= c.nh;
+  const int nx = c.nx, nh = c.nh;
+  // stores the second sweep's value: its own cell, or (img) an interior cell and its images
+  auto put = [&](int I, T v) {
+    if (img) {
+      const int col = (int)((unsigned)I % (unsigned)n1);
+      if (col < nh || col >= nh + nx) return;
+      if (col < 2 * nh) x[I + nx] = v;
+      if (col >= nx) x[I - nx] = v;
+    }
+    x[I] = v;
+  };
+  auto fill_lines = [&]() {
+    for (int t = tid; t < c.lines; t += kTT) d_fill_line(x + t * c.n1, c.n1, c.nh);
+  };
+  if ((!fill || img) && nact <= kTT) {  // one cell a thread, the warps that hold cells only
     const int nw = (nact + 31) >> 5;
     if ((tid >> 5) < nw) {
       const bool on = tid < nact;
@@ -99,9 +119,13 @@ __device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, int na
         if (on) y[I] = v;
         bar_warps(nw);
         v = tail_cell<T, ST>(y, I, n1, n2, bI, wI, cff, cE, cN);
-        if (on2) x[I] = v;
+        if (on2) put(I, v);
         bar_warps(nw);
       }
+    }
+    if (fill) {  // the lines out of the sweeps' range
+      __syncthreads();
+      fill_lines();
     }
     return;
   }
@@ -115,24 +139,24 @@ __device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, int na
       const unsigned e = list[t];
       if (e & kOut2) continue;
       const int I = (int)e;
-      x[I] = tail_cell<T, ST>(y, I, n1, n2, b[I], w[I], cff, cE, cN);
+      put(I, tail_cell<T, ST>(y, I, n1, n2, b[I], w[I], cff, cE, cN));
     }
     __syncthreads();
-    if (fill) {
-      for (int t = tid; t < c.lines; t += kTT) d_fill_line(x + t * c.n1, c.n1, c.nh);
+    if (fill && (!img || p == npairs - 1)) {
+      fill_lines();
       __syncthreads();
     }
   }
 }
 
 template <class T>
-__device__ __forceinline__ void tail_smooth_any(int st, int ctxi, int npairs, bool fill, int nact) {
+__device__ __forceinline__ void tail_smooth_any(int st, int ctxi, int npairs, bool fill, bool whole, int nact) {
   switch (st) {
-    case TAIL_5: tail_smooth<T, TAIL_5>(ctxi, npairs, fill, nact); break;
-    case TAIL_7: tail_smooth<T, TAIL_7>(ctxi, npairs, fill, nact); break;
-    case TAIL_9: tail_smooth<T, TAIL_9>(ctxi, npairs, fill, nact); break;
-    case TAIL_19: tail_smooth<T, TAIL_19>(ctxi, npairs, fill, nact); break;
-    default: tail_smooth<T, TAIL_VC>(ctxi, npairs, fill, nact); break;
+    case TAIL_5: tail_smooth<T, TAIL_5>(ctxi, npairs, fill, whole, nact); break;
+    case TAIL_7: tail_smooth<T, TAIL_7>(ctxi, npairs, fill, whole, nact); break;
+    case TAIL_9: tail_smooth<T, TAIL_9>(ctxi, npairs, fill, whole, nact); break;
+    case TAIL_19: tail_smooth<T, TAIL_19>(ctxi, npairs, fill, whole, nact); break;
+    default: tail_smooth<T, TAIL_VC>(ctxi, npairs, fill, whole, nact); break;
   }
 }
 
@@ -345,8 +369,8 @@ __device__ __forceinline__ void tail_run(const unsigned char* __restrict__ blob,
         if (tid == 0) full[q] = fl;
       }
       const int n = fl ? nrange : nact;
-      if (c.prec) tail_smooth_any<float>(c.stencil, q, op.npairs, op.fill != 0, n);
-      else tail_smooth_any<double>(c.stencil, q, op.npairs, op.fill != 0, n);
+      if (c.prec) tail_smooth_any<float>(c.stencil, q, op.npairs, op.fill != 0, fl != 0, n);
+      else tail_smooth_any<double>(c.stencil, q, op.npairs, op.fill != 0, fl != 0, n);
     } else if (op.kind == OPK_F32TO64) {
       const float* x = tail_ptr<const float>(op.x);
       double* y = tail_ptr<double>(op.y);

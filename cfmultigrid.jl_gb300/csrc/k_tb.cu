@@ -428,7 +428,9 @@ __device__ __forceinline__ void tb5_resid(const float* __restrict__ src, float* 
 // [ui0, ui1] = [nh+1, nx+nh], and a tile column outside them reads its
 // periodic image, so the sweeps see the periodic domain. With nh >= 2 that
 // is what the reference's interior gets from its linear-range sweeps with a
-// fill! after each pair; the caller fills the halo columns after the pass.
+// fill! after each pair; the output phase writes the nh = ui0 - 1 columns at
+// either end to their images in the halo too, as fill! would in a launch of
+// its own (2 us of a 240 us cycle, 8 times; nx < nh: the caller fills).
 //
 // UPD (the last post-smoothing pass of a mixed-precision cycle on level 1):
 // the smoothed FP32 correction e is not stored; the pass applies the FP64
@@ -462,7 +464,8 @@ __device__ __forceinline__ void tb5_tile(const float* __restrict__ x, float* __r
   const bool cols_in = ti0 >= ui0 && ti0 + kT5W - 1 <= ui1, rows_in = tj0 >= uj0 && tj0 + TH - 1 <= uj1;
   const bool tile_in_u = rows_in && (PER || cols_in);  // periodic: every column is updated
   // the parity of I0 is the same for every thread of the tile
-  const bool fast = rows_in && cols_in && ((I0 | tx) & 1) == 0;
+  const bool fast = rows_in && cols_in && ((I0 | tx) & 1) == 0 &&
+                    (!PER || (ti0 + H >= 2 * ui0 - 1 && ti0 + H + CW - 1 <= ui1 - ui0 + 1));  // core has no images
   float2 B[ROWS], WT[ROWS];
   unsigned inU = ~0u;  // bit 2r + e: cell in U
   float* prow = P0 + (r0 + 1) * kT5Row + lx;  // padded row r0 + 1 = tile row r0
@@ -693,8 +696,18 @@ __device__ __forceinline__ void tb5_tile(const float* __restrict__ x, float* __r
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int lc = 2 * lx + e;
-      if (lc >= H && lc < kT5W - H && (inU >> (2 * r + e) & 1u) && (!PER || gi0 + e <= ui1))
-        xo[I0 + (long long)r * tx + e] = prow[r * kT5Row + e * kT5Half + 1];
+      if (lc >= H && lc < kT5W - H && (inU >> (2 * r + e) & 1u) && (!PER || gi0 + e <= ui1)) {
+        const long long I = I0 + (long long)r * tx + e;
+        const float v = prow[r * kT5Row + e * kT5Half + 1];
+        xo[I] = v;
+        if (PER) {
+          const int nx = ui1 - ui0 + 1, hw = ui0 - 1, gi = gi0 + e;
+          if (nx >= hw) {
+            if (gi < ui0 + hw) xo[I + nx] = v;
+            if (gi > ui1 - hw) xo[I - nx] = v;
+          }
+        }
+      }
     }
   }
 }
