@@ -397,6 +397,13 @@ int upload_program(cfmg_handle* h, void* dst, const void* src, size_t bytes) {
   return CFMG_OK;
 }
 
+int rp_kind(const cfmg_handle* h) { return (vertices(h) ? 2 : 0) + (threed(h) ? 1 : 0); }
+int tail_stencil(const cfmg_handle* h) {
+  if (h->d.op == CFMG_VARCOEF) return TAIL_VC;
+  if (h->d.op == CFMG_LAPLACIAN9) return threed(h) ? TAIL_19 : TAIL_9;
+  return threed(h) ? TAIL_7 : TAIL_5;
+}
+
 // A tail program: its bytes on the device, and what the launch needs to know.
 struct TailBuild {
   std::string bytes;
@@ -644,7 +651,7 @@ int flush_tail(cfmg_handle* h, bool& done) {
   for (size_t i = 0; i < built.size(); ++i) {
     const TailBuild& q = built[i];
     Launch k(h, CFMG_K_ENGINE, 0, h->pending[0].prec ? CFMG_MIXED : CFMG_FP64);
-    launch_tail(h->tail_pool + at[i], (int)q.bytes.size(), q.nctx, q.nstore, q.ncopy, q.nops, q.smem, h->stream);
+    launch_tail(tail_stencil(h), rp_kind(h), h->tail_pool + at[i], (int)q.bytes.size(), q.nctx, q.nstore, q.ncopy, q.nops, q.smem, h->stream);
   }
   done = true;
   return CFMG_OK;
@@ -1038,8 +1045,6 @@ int residual_t(cfmg_handle* h, int lev) {
   if (sizeof(T) == 4 && !vertices(h)) return CFMG_OK;
   return fill_if<T>(h, lev, v.r);
 }
-
-int rp_kind(const cfmg_handle* h) { return (vertices(h) ? 2 : 0) + (threed(h) ? 1 : 0); }
 
 // mg.restriction[lev]: field of lev -> b of lev+1, then fill!
 template <class T>
@@ -2889,7 +2894,7 @@ int lockstep_body(cfmg_batch* b) {
   }
   for (const cfmg_batch::Step& st : b->steps) {
     if (st.tb == 5) {
-      launch_tail_batch(b->tstore, b->tprogs + st.tab0, (int)st.nchunks, (size_t)st.smem, b->active, b->stream);
+      launch_tail_batch(tail_stencil(b->inst[0]), rp_kind(b->inst[0]), b->tstore, b->tprogs + st.tab0, (int)st.nchunks, (size_t)st.smem, b->active, b->stream);
     } else if (st.tb == 3) {
       launch_brun(b->sops, b->ssm, b->rent, b->runs + st.tab0, (int)st.nchunks, st.smem, b->active, b->stream);
     } else if (st.tb == 2) {

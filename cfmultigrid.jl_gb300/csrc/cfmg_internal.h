@@ -291,14 +291,16 @@ struct alignas(16) TailOp {
   Box box;
   unsigned long long x, b, d, cE, cN, coef, m, y;
 };
-void launch_tail(const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops, size_t smem,
-                 cudaStream_t s);
+// stencil: the operator (TailStencil); kind: its restriction and prolongation, 0 .. 3 as in launch_restrict
+void launch_tail(int stencil, int kind, const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops,
+                 size_t smem, cudaStream_t s);
 // batched solver: programs of many instances in one launch, a block each
 struct TailProg {
   long long off;  // into the store
   int bytes, nctx, nstore, ncopy, nops, inst;
 };
-void launch_tail_batch(const void* store, const TailProg* tab, int n, size_t smem, const int* active, cudaStream_t s);
+void launch_tail_batch(int stencil, int kind, const void* store, const TailProg* tab, int n, size_t smem,
+                       const int* active, cudaStream_t s);
 // the cell lists that its smoothing calls sweep, one per level
 struct TailListLevel {
   const double *w, *pc;

@@ -42,9 +42,7 @@ constexpr int kTT = kTailThreads;
 // list entries: cell index, bit 15 set when the cell is outside the second
 // sweep's box (9- and 19-point operators)
 constexpr unsigned kOut2 = 0x8000u;
-// the block's dynamic shared memory: named here so that the functions below,
-// compiled out of line (one inlined body needed 1.8 KB of spills), still
-// address it as shared memory
+// the block's dynamic shared memory
 extern __shared__ __align__(16) unsigned char sm[];
 
 // the value of one sweep at I; b and omega*idiag of the cell come in registers
@@ -79,7 +77,7 @@ __device__ __forceinline__ void bar_warps(int nw) {
 // the two sweeps of a small level. whole: the list is the whole range (or
 // nx < nh): fills as the reference does.
 template <class T, int ST>
-__device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, bool whole, int nact) {
+__device__ __forceinline__ void tail_smooth(int ctxi, int npairs, bool fill, bool whole, int nact) {
   const TailCtx& c = reinterpret_cast<const TailCtx*>(sm)[ctxi];
   T* x = reinterpret_cast<T*>(sm + c.ox);
   T* y = reinterpret_cast<T*>(sm + c.oy);
@@ -93,15 +91,17 @@ __device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, bool w
   if (nact <= 0 && !fill) return;
   const bool img = fill && !whole && c.nx >= c.nh;
   const int nx = c.nx, nh = c.nh;
-  // stores the second sweep's value: its own cell, or (img) an interior cell and its images
-  auto put = [&](int I, T v) {
-    if (img) {
-      const int col = (int)((unsigned)I % (unsigned)n1);
-      if (col < nh || col >= nh + nx) return;
-      if (col < 2 * nh) x[I + nx] = v;
-      if (col >= nx) x[I - nx] = v;
-    }
-    x[I] = v;
+  // where the second sweep's value of cell I goes: bit 0 itself, 1 its image at I + nx, 2 at I - nx
+  auto dest = [&](int I) -> unsigned {
+    if (!img) return 1u;
+    const int col = (int)((unsigned)I % (unsigned)n1);
+    if (col < nh || col >= nh + nx) return 0u;
+    return 1u | (col < 2 * nh ? 2u : 0u) | (col >= nx ? 4u : 0u);
+  };
+  auto put = [&](int I, T v, unsigned d) {
+    if (d & 1u) x[I] = v;
+    if (d & 2u) x[I + nx] = v;
+    if (d & 4u) x[I - nx] = v;
   };
   auto fill_lines = [&]() {
     for (int t = tid; t < c.lines; t += kTT) d_fill_line(x + t * c.n1, c.n1, c.nh);
@@ -114,12 +114,13 @@ __device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, bool w
       const int I = (int)(e & (kOut2 - 1));
       const bool on2 = on && !(e & kOut2);
       const T bI = b[I], wI = w[I];
+      const unsigned d2 = on2 ? dest(I) : 0u;
       for (int p = 0; p < npairs; ++p) {
         T v = tail_cell<T, ST>(x, I, n1, n2, bI, wI, cff, cE, cN);
         if (on) y[I] = v;
         bar_warps(nw);
         v = tail_cell<T, ST>(y, I, n1, n2, bI, wI, cff, cE, cN);
-        if (on2) put(I, v);
+        put(I, v, d2);
         bar_warps(nw);
       }
     }
@@ -139,24 +140,13 @@ __device__ __noinline__ void tail_smooth(int ctxi, int npairs, bool fill, bool w
       const unsigned e = list[t];
       if (e & kOut2) continue;
       const int I = (int)e;
-      put(I, tail_cell<T, ST>(y, I, n1, n2, b[I], w[I], cff, cE, cN));
+      put(I, tail_cell<T, ST>(y, I, n1, n2, b[I], w[I], cff, cE, cN), dest(I));
     }
     __syncthreads();
     if (fill && (!img || p == npairs - 1)) {
       fill_lines();
       __syncthreads();
     }
-  }
-}
-
-template <class T>
-__device__ __forceinline__ void tail_smooth_any(int st, int ctxi, int npairs, bool fill, bool whole, int nact) {
-  switch (st) {
-    case TAIL_5: tail_smooth<T, TAIL_5>(ctxi, npairs, fill, whole, nact); break;
-    case TAIL_7: tail_smooth<T, TAIL_7>(ctxi, npairs, fill, whole, nact); break;
-    case TAIL_9: tail_smooth<T, TAIL_9>(ctxi, npairs, fill, whole, nact); break;
-    case TAIL_19: tail_smooth<T, TAIL_19>(ctxi, npairs, fill, whole, nact); break;
-    default: tail_smooth<T, TAIL_VC>(ctxi, npairs, fill, whole, nact); break;
   }
 }
 
@@ -206,69 +196,57 @@ __device__ __forceinline__ Geom tail_geom(int tx, int ty, int tz, int nh) {
   return g;
 }
 
-template <class T>
-__device__ __noinline__ void tail_resid(const TailOp* opp) {
-  const TailOp& op = *opp;
+template <class T, int ST>
+__device__ __forceinline__ void tail_resid(const TailOp& op) {
   const T* x = tail_ptr<const T>(op.x);
   const T* b = tail_ptr<const T>(op.b);
   const T* d = tail_ptr<const T>(op.d);
+  const T* cE = tail_ptr<const T>(op.cE);
+  const T* cN = tail_ptr<const T>(op.cN);
   const uint8_t* m = tail_ptr<const uint8_t>(op.m);
   T* y = tail_ptr<T>(op.y);
   const Geom g = tail_geom(op.tx, op.ty, op.tz, op.nh);
-  const int n = op.n, kind = op.kind;
+  auto cell = [&](long long I) {
+    if (ST == TAIL_5) d_resid5(y, x, b, d, m, g.n1, I);
+    else if (ST == TAIL_VC) d_residvc(y, x, b, d, cE, cN, m, g.n1, I);
+    else if (ST == TAIL_7) d_resid7(y, x, b, d, m, g.n1, g.n2, I);
+    else if (ST == TAIL_9) d_resid9(y, x, b, d, m, g.n1, I);
+    else d_resid19(y, x, b, d, m, g.n1, g.n2, I);
+  };
   if (op.ctxi >= 0) {  // below level 1: the listed cells; +0 at the others (their mask is 0)
     const TailCtx& c = reinterpret_cast<const TailCtx*>(sm)[op.ctxi];
     const int* hdr = reinterpret_cast<const int*>(sm + c.olist);
     const unsigned short* list = reinterpret_cast<const unsigned short*>(sm + c.olist + kTailListHdr);
     const int nact = hdr[0], nrange = hdr[1];
-    const T* cE = tail_ptr<const T>(op.cE);
-    const T* cN = tail_ptr<const T>(op.cN);
-    if (kind == OPK_RESID7) {  // the sweeps cover whole planes, the residual the interior box
-      const unsigned n1 = (unsigned)op.tx, nj = (unsigned)op.ty;
-      for (int t = threadIdx.x; t < nrange; t += kTT) {
-        const unsigned I = list[t], r = I / n1, k = r / nj;
-        const int i = (int)(I - r * n1) + 1, j = (int)(r - k * nj) + 1, kk = (int)k + 1;
-        if (i < op.box.i0 || i > op.box.i1 || j < op.box.j0 || j > op.box.j1 || kk < op.box.k0 || kk > op.box.k1)
-          continue;
-        if (t < nact) d_resid7(y, x, b, d, m, g.n1, g.n2, (long long)I);
-        else y[I] = T(0);
-      }
-      return;
-    }
+    const unsigned n1 = (unsigned)op.tx, nj = (unsigned)op.ty;
     for (int t = threadIdx.x; t < nrange; t += kTT) {
       const unsigned e = list[t];
       if (e & kOut2) continue;  // the residual's range is the second sweep's
-      const long long I = e;
-      if (t >= nact) y[I] = T(0);
-      else if (kind == OPK_RESID5) d_resid5(y, x, b, d, m, g.n1, I);
-      else if (kind == OPK_RESIDVC) d_residvc(y, x, b, d, cE, cN, m, g.n1, I);
-      else if (kind == OPK_RESID9) d_resid9(y, x, b, d, m, g.n1, I);
-      else d_resid19(y, x, b, d, m, g.n1, g.n2, I);
+      if (ST == TAIL_7) {       // whose sweeps cover whole planes, the residual the interior box
+        const unsigned r = e / n1, k = r / nj;
+        const int i = (int)(e - r * n1) + 1, j = (int)(r - k * nj) + 1, kk = (int)k + 1;
+        if (i < op.box.i0 || i > op.box.i1 || j < op.box.j0 || j > op.box.j1 || kk < op.box.k0 || kk > op.box.k1)
+          continue;
+      }
+      if (t < nact) cell((long long)e);
+      else y[e] = T(0);
     }
     return;
   }
-  if (kind == OPK_RESID5) {
-    for (int t = threadIdx.x; t < n; t += kTT) d_resid5(y, x, b, d, m, g.n1, op.lo + t);
-  } else if (kind == OPK_RESIDVC) {
-    const T* cE = tail_ptr<const T>(op.cE);
-    const T* cN = tail_ptr<const T>(op.cN);
-    for (int t = threadIdx.x; t < n; t += kTT) d_residvc(y, x, b, d, cE, cN, m, g.n1, op.lo + t);
+  if (ST == TAIL_5 || ST == TAIL_VC) {
+    for (int t = threadIdx.x; t < op.n; t += kTT) cell(op.lo + t);
   } else {
     const TailBox q(op.box);
-    for (int t = threadIdx.x; t < n; t += kTT) {
+    for (int t = threadIdx.x; t < op.n; t += kTT) {
       int i, j, k;
       q.at(t, i, j, k);
-      const long long I = lin(g, i, j, k);
-      if (kind == OPK_RESID7) d_resid7(y, x, b, d, m, g.n1, g.n2, I);
-      else if (kind == OPK_RESID9) d_resid9(y, x, b, d, m, g.n1, I);
-      else d_resid19(y, x, b, d, m, g.n1, g.n2, I);
+      cell(lin(g, i, j, k));
     }
   }
 }
 
 template <class T, int K>
-__device__ __noinline__ void tail_restrict(const TailOp* opp) {
-  const TailOp& op = *opp;
+__device__ __forceinline__ void tail_restrict(const TailOp& op) {
   const T* x = tail_ptr<const T>(op.x);
   const T* coef = tail_ptr<const T>(op.coef);
   T* y = tail_ptr<T>(op.y);
@@ -284,8 +262,7 @@ __device__ __noinline__ void tail_restrict(const TailOp* opp) {
 // a thread per child instead of per parent: a parent's 29 FP64 instructions in
 // one warp took 1.1 us on a level of 16 parents
 template <class T, int K>
-__device__ __noinline__ void tail_prolong(const TailOp* opp) {
-  const TailOp& op = *opp;
+__device__ __forceinline__ void tail_prolong(const TailOp& op) {
   const T* x = tail_ptr<const T>(op.x);
   const T* coef = tail_ptr<const T>(op.coef);
   T* y = tail_ptr<T>(op.y);
@@ -304,34 +281,29 @@ __device__ __noinline__ void tail_prolong(const TailOp* opp) {
   }
 }
 
-template <class T>
-__device__ __forceinline__ void tail_exec(const TailOp* op) {
-  switch (op->kind) {
-    case OPK_RESTRICT0: tail_restrict<T, 0>(op); break;
-    case OPK_RESTRICT1: tail_restrict<T, 1>(op); break;
-    case OPK_RESTRICT2: tail_restrict<T, 2>(op); break;
-    case OPK_RESTRICT3: tail_restrict<T, 3>(op); break;
-    case OPK_PROLONG0: tail_prolong<T, 0>(op); break;
-    case OPK_PROLONG1: tail_prolong<T, 1>(op); break;
-    case OPK_PROLONG2: tail_prolong<T, 2>(op); break;
-    case OPK_PROLONG3: tail_prolong<T, 3>(op); break;
-    case OPK_FILL: {
-      T* y = tail_ptr<T>(op->y);
-      for (int t = threadIdx.x; t < op->n; t += kTT) d_fill_line(y + (long long)t * op->tx, op->tx, op->nh);
-      break;
-    }
-    case OPK_ZERO: {
-      T* y = tail_ptr<T>(op->y);
-      for (int t = threadIdx.x; t < op->n; t += kTT) y[t] = T(0);
-      break;
-    }
-    default: tail_resid<T>(op); break;
+template <class T, int ST, int K>
+__device__ __forceinline__ void tail_exec(const TailOp& op) {
+  if (op.kind >= OPK_RESTRICT0 && op.kind <= OPK_RESTRICT3) {
+    tail_restrict<T, K>(op);
+  } else if (op.kind >= OPK_PROLONG0 && op.kind <= OPK_PROLONG3) {
+    tail_prolong<T, K>(op);
+  } else if (op.kind == OPK_FILL) {
+    T* y = tail_ptr<T>(op.y);
+    for (int t = threadIdx.x; t < op.n; t += kTT) d_fill_line(y + (long long)t * op.tx, op.tx, op.nh);
+  } else if (op.kind == OPK_ZERO) {
+    T* y = tail_ptr<T>(op.y);
+    for (int t = threadIdx.x; t < op.n; t += kTT) y[t] = T(0);
+  } else {
+    tail_resid<T, ST>(op);
   }
 }
 
 }  // namespace
 
-// one program, run by one block
+// One program, run by one block. A kernel per stencil ST and transfer kind K:
+// with all operators in one kernel, each reached by an indirect call, a lone
+// warp spent some 1900 clocks around a smoothing call of a small level.
+template <int ST, int K>
 __device__ __forceinline__ void tail_run(const unsigned char* __restrict__ blob, int blob_bytes, int nctx, int nstore,
                                          int ncopy, int nops) {
   __shared__ int full[kTailMaxCtx];  // -1: not looked at in this launch; 1: the context sweeps its whole range
@@ -369,8 +341,8 @@ __device__ __forceinline__ void tail_run(const unsigned char* __restrict__ blob,
         if (tid == 0) full[q] = fl;
       }
       const int n = fl ? nrange : nact;
-      if (c.prec) tail_smooth_any<float>(c.stencil, q, op.npairs, op.fill != 0, fl != 0, n);
-      else tail_smooth_any<double>(c.stencil, q, op.npairs, op.fill != 0, fl != 0, n);
+      if (c.prec) tail_smooth<float, ST>(q, op.npairs, op.fill != 0, fl != 0, n);
+      else tail_smooth<double, ST>(q, op.npairs, op.fill != 0, fl != 0, n);
     } else if (op.kind == OPK_F32TO64) {
       const float* x = tail_ptr<const float>(op.x);
       double* y = tail_ptr<double>(op.y);
@@ -380,9 +352,9 @@ __device__ __forceinline__ void tail_run(const unsigned char* __restrict__ blob,
       float* y = tail_ptr<float>(op.y);
       for (int t = tid; t < op.n; t += kTT) y[t] = (float)x[t];
     } else if (op.prec) {
-      tail_exec<float>(&op);
+      tail_exec<float, ST, K>(op);
     } else {
-      tail_exec<double>(&op);
+      tail_exec<double, ST, K>(op);
     }
     if (!op.nobar) __syncthreads();
   }
@@ -395,19 +367,21 @@ __device__ __forceinline__ void tail_run(const unsigned char* __restrict__ blob,
           *reinterpret_cast<const uint4*>(sm + cp[q].off + tid * 16);
 }
 
+template <int ST, int K>
 __global__ void __launch_bounds__(kTT, 1) k_tail(const unsigned char* __restrict__ blob, int blob_bytes, int nctx,
                                                  int nstore, int ncopy, int nops) {
-  tail_run(blob, blob_bytes, nctx, nstore, ncopy, nops);
+  tail_run<ST, K>(blob, blob_bytes, nctx, nstore, ncopy, nops);
 }
 
 // batched solver: a block per program of the table, for instances still iterating
+template <int ST, int K>
 __global__ void __launch_bounds__(kTT, 1) k_tail_batch(const unsigned char* __restrict__ store,
                                                        const TailProg* __restrict__ tab,
                                                        const int* __restrict__ active) {
   const TailProg p = tab[blockIdx.x];  // uploaded before the launch
   dep_wait();
   if (!active[p.inst]) return;
-  tail_run(store + p.off, p.bytes, p.nctx, p.nstore, p.ncopy, p.nops);
+  tail_run<ST, K>(store + p.off, p.bytes, p.nctx, p.nstore, p.ncopy, p.nops);
 }
 
 // The cell lists of the levels, one block a level: {live cells, cells of the
@@ -475,23 +449,51 @@ __global__ void __launch_bounds__(1024) k_tail_lists(TailListArgs a) {
   }
 }
 
-void launch_tail_batch(const void* store, const TailProg* tab, int n, size_t smem, const int* active, cudaStream_t s) {
+template <int ST, int K>
+static void launch_tail_k(const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops, size_t smem,
+                          cudaStream_t s) {
   static const cudaError_t attr =
-      cudaFuncSetAttribute(k_tail_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmemMax);
+      cudaFuncSetAttribute(k_tail<ST, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmemMax);
   (void)attr;
-  if (n > 0) launch_dep(k_tail_batch, (unsigned)n, kTT, smem, s, (const unsigned char*)store, tab, active);
+  launch_dep(k_tail<ST, K>, 1, kTT, smem, s, (const unsigned char*)blob, blob_bytes, nctx, nstore, ncopy, nops);
+}
+void launch_tail(int stencil, int kind, const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops,
+                 size_t smem, cudaStream_t s) {
+#define CFMG_TAIL(ST, K) \
+  if (stencil == ST && kind == K) return launch_tail_k<ST, K>(blob, blob_bytes, nctx, nstore, ncopy, nops, smem, s);
+  CFMG_TAIL(TAIL_5, 0)
+  CFMG_TAIL(TAIL_5, 2)
+  CFMG_TAIL(TAIL_9, 0)
+  CFMG_TAIL(TAIL_9, 2)
+  CFMG_TAIL(TAIL_VC, 0)
+  CFMG_TAIL(TAIL_7, 1)
+  CFMG_TAIL(TAIL_7, 3)
+  CFMG_TAIL(TAIL_19, 1)
+  CFMG_TAIL(TAIL_19, 3)
+#undef CFMG_TAIL
+}
+template <int ST, int K>
+static void launch_tail_batch_k(const void* store, const TailProg* tab, int n, size_t smem, const int* active,
+                                cudaStream_t s) {
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(k_tail_batch<ST, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmemMax);
+  (void)attr;
+  launch_dep(k_tail_batch<ST, K>, (unsigned)n, kTT, smem, s, (const unsigned char*)store, tab, active);
+}
+void launch_tail_batch(int stencil, int kind, const void* store, const TailProg* tab, int n, size_t smem,
+                       const int* active, cudaStream_t s) {
+  if (n <= 0) return;
+  if (stencil == TAIL_9) {
+    if (kind == 2) launch_tail_batch_k<TAIL_9, 2>(store, tab, n, smem, active, s);
+    else launch_tail_batch_k<TAIL_9, 0>(store, tab, n, smem, active, s);
+  } else {
+    if (kind == 2) launch_tail_batch_k<TAIL_5, 2>(store, tab, n, smem, active, s);
+    else launch_tail_batch_k<TAIL_5, 0>(store, tab, n, smem, active, s);
+  }
 }
 
 void launch_tail_lists(const TailListArgs& a, int n, cudaStream_t s) {
   if (n > 0) launch_dep(k_tail_lists, (unsigned)n, 1024, 0, s, a);
-}
-
-void launch_tail(const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops, size_t smem,
-                 cudaStream_t s) {
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmemMax);
-  (void)attr;
-  launch_dep(k_tail, 1, kTT, smem, s, (const unsigned char*)blob, blob_bytes, nctx, nstore, ncopy, nops);
 }
 
 }  // namespace cfmg
