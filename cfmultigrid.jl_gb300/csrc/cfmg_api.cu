@@ -672,6 +672,7 @@ int tail_lists(cfmg_handle* h) {
     TailListLevel& q = a.lev[n++];
     q.w = l.widiag; q.pc = l.Pcoef; q.m = l.msk; q.out = l.tlist;
     q.len = (int)l.len; q.n1 = l.tx; q.nj = l.ty;
+    q.nx = xperio(h) ? l.nx : 0; q.nh = l.nh;
     q.box = h->d.op == CFMG_LAPLACIAN9;
     const int off = threed(h) ? l.tx * l.ty : l.tx;
     q.lo = off; q.hi = (int)l.len - off;
@@ -729,7 +730,7 @@ int flush(cfmg_handle* h) {
 bool blocked_form(const cfmg_handle* h, int lev) {
   if (!h->tb_on || h->record || threed(h) || !h->tail_pool || h->tail_from[1] <= 0) return false;
   if (h->d.op != CFMG_LAPLACIAN && h->d.op != CFMG_LAPLACIAN9) return false;
-  return !xperio(h) || (h->tb_version == 5 && h->d.op == CFMG_LAPLACIAN);
+  return !xperio(h) || (h->tb_version == 5 && h->d.op == CFMG_LAPLACIAN && h->lv[lev - 1].nx >= h->lv[lev - 1].nh);
 }
 bool in_engine(const cfmg_handle* h, int lev, int prec) {
   if (!h->engine_on) return false;
@@ -817,6 +818,8 @@ bool tb_eligible(const cfmg_handle* h, int lev) {
   if (sizeof(T) != 4 || !h->tb_on || (h->record && !h->record_tb)) return false;
   // x-periodic: the lean packed passes of the 2D 5-point operator (standalone launches)
   if (xperio(h) && (h->record || h->tb_version != 5 || threed(h) || h->d.op != CFMG_LAPLACIAN)) return false;
+  // narrower than its halo: the coefficients' halo is not their periodic image, as those passes take it
+  if (xperio(h) && h->lv[lev - 1].nx < h->lv[lev - 1].nh) return false;
   // 3D: 7-point streaming passes, opt-in (CFMG_OPT_TEMPORAL_BLOCKING = 4): at
   // 512 x 512 x 256 a 4-sweep pass measured 1.0-1.3 ms, no faster than
   // four single-sweep kernels at 66 % of HBM
@@ -873,7 +876,6 @@ int smooth_tb(cfmg_handle* h, int lev, int nite) {
       }
       l.xswap ^= 1;
       left -= n;
-      if (l.nx < l.nh) TRY(fill_if<float>(h, lev, view<float>(l).x));  // else the pass wrote the halo columns
     }
     LAUNCH_OK(h);
     return CFMG_OK;

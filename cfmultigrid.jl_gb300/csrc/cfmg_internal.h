@@ -306,6 +306,7 @@ struct TailListLevel {
   const double *w, *pc;
   const uint8_t* m;
   unsigned char* out;  // kTailListHdr bytes, then one 16-bit entry a cell
+  int nx, nh;                    // nx: 0 unless x-periodic
   int len, n1, nj, box, lo, hi;  // box != 0: the ranges are the boxes, else lo .. hi
   Box ext, in;
 };
@@ -348,8 +349,7 @@ bool launch_smooth_tb(int version, int stencil, int nite, const float* x, float*
                       float cff, int tx, int ty, int nz, int ui0, int ui1, int uj0, int uj1, cudaStream_t s);
 // the lean packed passes for the x-periodic topology, 5-point operator: the
 // tiles cover the interior columns [ui0, ui1], read the periodic images of
-// the columns beside them and write the images of the end columns (the caller
-// fills the halo columns of a level with nx < nh)
+// the columns beside them and write the images of the end columns (nx >= nh)
 bool launch_smooth_tb_periodic(int nite, const float* x, float* xo, const float* b, const float* w, float cff,
                                int tx, int ty, int nz, int ui0, int ui1, int uj0, int uj1, cudaStream_t s);
 // The last pass of a V-cycle's pre-smoothing with the step that follows it

@@ -336,7 +336,9 @@ __device__ __forceinline__ void tail_run(const unsigned char* __restrict__ blob,
       const int nact = hdr[0], nrange = hdr[1];
       int fl = full[q];
       if (fl < 0) {
-        const bool bad = c.cff < 0.0 || (c.prec ? tail_dirty<float>(c, nact, nrange) : tail_dirty<double>(c, nact, nrange));
+        // nx < nh: the periodic halo of so narrow a level is not the image of its coefficients, and
+        // fill! brings values to cells that the list leaves out
+        const bool bad = c.cff < 0.0 || (op.fill && c.nx < c.nh) || (c.prec ? tail_dirty<float>(c, nact, nrange) : tail_dirty<double>(c, nact, nrange));
         fl = __syncthreads_or(bad) ? 1 : 0;
         if (tid == 0) full[q] = fl;
       }
@@ -402,8 +404,13 @@ __global__ void __launch_bounds__(1024) k_tail_lists(TailListArgs a) {
     };
     return in(l.ext) ? (in(l.in) ? 2 : 1) : 0;
   };
+  auto live1 = [&](int I) { return nonzero_bits(l.w[I]) || nonzero_bits(l.pc[I]) || l.m[I] != 0; };
   auto live = [&](int I) {
-    return nonzero_bits(l.w[I]) || nonzero_bits(l.pc[I]) || l.m[I] != 0;
+    if (live1(I)) return true;
+    if (!l.nx) return false;
+    // x-periodic: fill! copies between a cell and its images, so they are listed together
+    const int col = (int)((unsigned)I % (unsigned)l.n1);
+    return ((col < 2 * l.nh && I + l.nx < l.len && live1(I + l.nx)) || (col >= l.nx && I >= l.nx && live1(I - l.nx)));
   };
   const int words = (l.len + 31) >> 5, per = (words + nw - 1) / nw;
   const int w0 = wid * per, w1 = min(words, (wid + 1) * per);

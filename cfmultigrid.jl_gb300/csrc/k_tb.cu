@@ -430,7 +430,7 @@ __device__ __forceinline__ void tb5_resid(const float* __restrict__ src, float* 
 // is what the reference's interior gets from its linear-range sweeps with a
 // fill! after each pair; the output phase writes the nh = ui0 - 1 columns at
 // either end to their images in the halo too, as fill! would in a launch of
-// its own (2 us of a 240 us cycle, 8 times; nx < nh: the caller fills).
+// its own (2 us of a 240 us cycle, 8 times).
 //
 // UPD (the last post-smoothing pass of a mixed-precision cycle on level 1):
 // the smoothed FP32 correction e is not stored; the pass applies the FP64
@@ -702,10 +702,8 @@ __device__ __forceinline__ void tb5_tile(const float* __restrict__ x, float* __r
         xo[I] = v;
         if (PER) {
           const int nx = ui1 - ui0 + 1, hw = ui0 - 1, gi = gi0 + e;
-          if (nx >= hw) {
-            if (gi < ui0 + hw) xo[I + nx] = v;
-            if (gi > ui1 - hw) xo[I - nx] = v;
-          }
+          if (gi < ui0 + hw) xo[I + nx] = v;
+          if (gi > ui1 - hw) xo[I - nx] = v;
         }
       }
     }

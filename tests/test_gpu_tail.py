@@ -47,6 +47,8 @@ CASES = {
     "2d5-layers": dict(nx=24, ny=20, nz=2, case="twod"),
     "2d9-vertices": dict(nx=40, ny=56, nz=1, case="twod", location="vertices", operator="laplacian9"),
     "2d5-periodic": dict(nx=48, ny=32, nz=1, case="twod", topology="xperio"),
+    "2d5-periodic-narrow": dict(nx=28, ny=36, nz=1, case="twod", topology="xperio"),  # down to nx = 1 < nh
+    "3d7-periodic": dict(nx=12, ny=16, nz=12, case="threed", topology="xperio"),
     "varcoef": dict(nx=44, ny=52, nz=1, case="twod", operator="varcoef"),
     "3d7": dict(nx=24, ny=20, nz=12, case="threed"),
     "3d19-vertices": dict(nx=20, ny=24, nz=16, case="threed", location="vertices", operator="laplacian9"),
@@ -86,7 +88,7 @@ def test_tail_smoothing_of_any_x(name, omega):
         assert np.array_equal(out[0][k], out[1][k]), k
 
 
-@pytest.mark.parametrize("name", ["2d5", "2d9-vertices", "2d5-periodic", "varcoef", "3d7", "3d19-vertices"])
+@pytest.mark.parametrize("name", ["2d5", "2d9-vertices", "2d5-periodic", "2d5-periodic-narrow", "varcoef", "3d7", "3d19-vertices"])
 def test_tail_mixed_solve_is_bit_identical(name):
     out = []
     for small in (4, 0):
