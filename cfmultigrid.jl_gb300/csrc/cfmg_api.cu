@@ -68,7 +68,7 @@ struct cfmg_handle {
   // its wet interior (written by the caller or by the setup, not zeroed since)
   bool coef_setup = false;
   std::vector<unsigned> dirt;
-  bool graph_steps = false;  // whether the captured graphs were made with steps_clean (see step_ok)
+  int graph_steps = 0;  // the captured graphs' steps_clean and coef_clean (see step_ok)
   std::unordered_map<std::string, size_t> tail_cache;
   bool tb_on = true;  // temporally blocked FP32 smoothing on fine levels
   bool fuse_on = true;  // V-cycle descent: residual and restriction in the last pre-smoothing pass
@@ -737,7 +737,9 @@ bool in_engine(const cfmg_handle* h, int lev, int prec) {
   if (in_tail(h, lev, prec)) return true;
   if ((long long)h->lv[lev - 1].len > engine_limit(h, prec)) return false;
   // FP64 levels between the tail and the threshold take one-launch steps
-  return !(prec ? blocked_form(h, lev) : h->tail_pool && h->tail_from[0] > 0 && steps_form(h));
+  // and so do FP32 ones of the variable-coefficient operator
+  const bool steps = h->tail_pool && h->tail_from[prec ? 1 : 0] > 0 && steps_form(h);
+  return !(prec ? blocked_form(h, lev) || (steps && h->d.op == CFMG_VARCOEF) : steps);
 }
 
 int emit(cfmg_handle* h, const Op& op) {
@@ -1236,39 +1238,59 @@ int resid_restrict3d(cfmg_handle* h, int lev) {
 // level lost 1.5 % of its solve and a 390 x 294 variable-coefficient one 10 %.
 constexpr long long kStepCells = 150000;  // levels that get the scratch array
 constexpr long long kStepWork = 800000, kStepWork1 = 400000;
+bool coef_clean(const cfmg_handle* h) { return h->coef_setup && !h->coef_exposed; }
 bool steps_clean(const cfmg_handle* h) {
-  if (!h->coef_setup || h->coef_exposed) return false;
+  if (!coef_clean(h)) return false;
   for (int k = 2; k <= L(h); ++k)
     if (h->dirt[k - 1]) return false;
   return true;
 }
+template <class T>
 bool step_ok(const cfmg_handle* h, int lev) {
   if (h->record || !steps_form(h) || lev >= L(h)) return false;
   if (h->d.npre < 1 || h->d.npre > kTbgMaxPairs || h->d.npost < 1 || h->d.npost > kTbgMaxPairs) return false;
   const Level& l = h->lv[lev - 1];
+  // FP32 variable coefficient, levels of every size: a level-1 descent of 2048^2 reads its five
+  // arrays once instead of in each of four sweeps (its fields hold +0 outside the wet interior always)
+  if (sizeof(T) == 4) return h->d.op == CFMG_VARCOEF && l.s32 && !in_engine(h, lev, CFMG_MIXED) && coef_clean(h);
   if ((long long)l.len * (h->d.op == CFMG_LAPLACIAN ? 7 : 11) > (lev == 1 ? kStepWork1 : kStepWork)) return false;
   return l.s64 && !in_engine(h, lev, CFMG_FP64) && steps_clean(h);
 }
 
+template <class T>
+T* step_scratch(const Level& l);
+template <>
+double* step_scratch<double>(const Level& l) { return l.s64; }
+template <>
+float* step_scratch<float>(const Level& l) { return l.s32; }
+
+template <class T>
 int step2d(cfmg_handle* h, int lev, int mode, int np) {
   const Level& l = h->lv[lev - 1];
   const Level& c = h->lv[lev];
+  const View<T> v = view<T>(l), vc = view<T>(c);
   TRY(flush(h));
-  TbgArgs a;
+  TbgArgs<T> a;
   std::memset(&a, 0, sizeof(a));
-  const bool first = lev == 1 && mode != 2;  // the descent of level 1 starts from x and leaves x and y alone
-  a.xs = mode == 2 ? l.s64 : first ? l.x : nullptr;
-  a.b = l.b; a.w = l.widiag; a.cE = l.cE; a.cN = l.cN; a.d = l.diag; a.pc = l.Pcoef;
-  a.xc = c.x; a.rc = c.Rcoef; a.m = l.msk;
-  a.x = first ? nullptr : l.x; a.y = first ? nullptr : l.y; a.r = l.r; a.s = l.s64; a.bc = c.b; a.xcz = c.x;
-  a.cff = 1.0 - h->d.omega;
+  // the FP64 descent of level 1 starts from x and leaves x and y alone; the FP32 one from +0
+  const bool first = sizeof(T) == 8 && lev == 1 && mode != 2;
+  a.s = step_scratch<T>(l);
+  a.xs = mode == 2 ? a.s : first ? v.x : nullptr;
+  a.b = v.b; a.w = v.widiag; a.cE = v.cE; a.cN = v.cN; a.d = v.diag; a.pc = v.Pcoef;
+  a.xc = vc.x; a.rc = vc.Rcoef; a.m = v.msk;
+  a.bc = vc.b; a.xcz = vc.x;
+  if (!first) a.x = v.x;
+  if (sizeof(T) == 8) {  // the FP32 y and r of a cycle are read by nothing after the step
+    if (!first) a.y = v.y;
+    a.r = v.r;
+  }
+  a.cff = (T)(1.0 - h->d.omega);
   a.np = np;
   a.tx = l.tx; a.ty = l.ty; a.nh = l.nh; a.ctx = c.tx; a.cty = c.ty;
   a.np_i = (l.nx + 1) / 2; a.np_j = (l.ny + 1) / 2;
   {
-    Launch k(h, mode == 2 ? CFMG_K_SWEEP : CFMG_K_DESCENT, lev, CFMG_FP64);
-    launch_step2d(a, h->d.op == CFMG_LAPLACIAN9 ? TAIL_9 : h->d.op == CFMG_VARCOEF ? TAIL_VC : TAIL_5, mode,
-                  vertices(h), h->stream);
+    Launch k(h, mode == 2 ? CFMG_K_SWEEP : CFMG_K_DESCENT, lev, prec_of<T>());
+    launch_step2d(a, tail_stencil(h), mode, vertices(h), h->stream);
   }
   LAUNCH_OK(h);
   return CFMG_OK;
@@ -1295,15 +1317,15 @@ template <class T>
 int vcycle_t(cfmg_handle* h, int lev0, bool prolonged = false) {
   const cfmg_desc& d = h->d;
   const int nl = L(h);
-  auto step = [&](int lev) { return sizeof(T) == 8 && (lev > lev0 || lev == 1 || prolonged) && step_ok(h, lev); };
+  auto step = [&](int lev) { return (lev > lev0 || lev == 1 || prolonged) && step_ok<T>(h, lev); };
   for (int lev = lev0; lev <= nl - 1; ++lev) {
-    if (step(lev)) TRY(step2d(h, lev, lev == lev0 && prolonged ? 1 : 0, d.npre));
+    if (step(lev)) TRY(step2d<T>(h, lev, lev == lev0 && prolonged ? 1 : 0, d.npre));
     else TRY(descend_t<T>(h, lev, d.npre, !(lev + 1 < nl && step(lev + 1))));
   }
   TRY(coarsest_t<T>(h, d.ndeepest));
   for (int lev = nl - 1; lev >= lev0; --lev) {
     if (step(lev)) {
-      TRY(step2d(h, lev, 2, d.npost));
+      TRY(step2d<T>(h, lev, 2, d.npost));
       continue;
     }
     TRY(prolong_t<T>(h, lev, false, d.npost > 0));
@@ -1330,12 +1352,12 @@ int fcycle_t(cfmg_handle* h, bool x1_zero = false) {
   const bool lazy = sizeof(T) == 4 && !xperio(h);
   for (int lev = 1; lev <= nl - 1; ++lev) {
     TRY(restrict_t<T>(h, lev, lev > 1 ? CFMG_B : CFMG_R));
-    const bool step = sizeof(T) == 8 && step_ok(h, lev + 1);  // its first step assigns x
+    const bool step = step_ok<T>(h, lev + 1);  // its first step assigns x
     if ((!lazy && !step) || lev + 1 == nl) TRY(zero_t<T>(h, lev + 1, CFMG_X));  // the coarsest solve reads it
   }
   TRY(coarsest_t<T>(h, h->d.ndeepest));
   for (int lev = nl - 1; lev >= 1; --lev) {
-    const bool step = sizeof(T) == 8 && step_ok(h, lev);
+    const bool step = step_ok<T>(h, lev);
     if (!step) TRY(prolong_t<T>(h, lev, lev >= 2 ? lazy : x1_zero, h->d.npre > 0));
     TRY(vcycle_t<T>(h, lev, step));
   }
@@ -1848,7 +1870,7 @@ int mixed_iteration(cfmg_handle* h, int kind) {
     launch_dep(k_scale_from_norm, 1, kNormParts, 0, h->stream, h->dscal, h->partials, kNormParts, remove_mean);
     launch_dep(k_rhs32, nb, 256, 0, h->stream, l1.r, l1.msk, h->dscal, l1.b32, l1.r32, n);
   }
-  if (!lazy && !h->x1_zero) TRY(zero_t<float>(h, 1, CFMG_X));
+  if (!lazy && !h->x1_zero && !step_ok<float>(h, 1)) TRY(zero_t<float>(h, 1, CFMG_X));
   LAUNCH_OK(h);
   const int st = cycle_t<float>(h, kind, lazy);
   h->x1_zero = false;
@@ -2179,6 +2201,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
     total += coded ? al(n) : 0;               // wq
     total += tailed(l) ? al(kTailListHdr + 2 * n) : 0;  // tlist
     total += stepped(l) ? al(n * 8) : 0;                // s64
+    total += mixed && vc && !shared && l.tz == 1 ? al(n * 4) : 0;  // s32
   }
   total += coded ? al(256 * sizeof(float)) : 0;  // wtab
   if (cudaMalloc(&h->arena, total) != cudaSuccess) {
@@ -2215,6 +2238,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
     if (coded) l.wq = (uint8_t*)take(n);
     if (tailed(l)) l.tlist = (unsigned char*)take(kTailListHdr + 2 * n);
     if (stepped(l)) l.s64 = (double*)take(n * 8);
+    if (mixed && vc && !shared && l.tz == 1) l.s32 = (float*)take(n * 4);
   }
   if (coded) h->wtab = (float*)take(256 * sizeof(float));
   // the fixed-point residual pass reads kResidIntReach elements beside level
@@ -2545,10 +2569,11 @@ int cfmg_solve(cfmg_handle* h, double* res_out, int* nite_out, double* history) 
     return fail(h, CFMG_ERR_UNSUPPORTED, "the mixed-precision form runs V and F cycles");
   if (prec == CFMG_MIXED) TRY(prepare_mixed(h));
   TRY(tail_lists(h));
-  if (steps_clean(h) != h->graph_steps) {  // the captured iterations took the other route
+  const int route = (steps_clean(h) ? 1 : 0) | (coef_clean(h) ? 2 : 0);
+  if (route != h->graph_steps) {  // the captured iterations took another route
     TRY(sync(h));
     drop_graphs(h);
-    h->graph_steps = steps_clean(h);
+    h->graph_steps = route;
   }
   // normb = norm(mg, 1, :b) (src/gmg_solver.jl:22)
   const Level& l1 = h->lv[0];

@@ -68,7 +68,8 @@ struct Level {
   // plane) holding a wet cell (launch_make_qact); dry quads are skipped
   uint8_t* qact;
   unsigned char* tlist;  // the coarse tail's cell list (launch_tail_lists); null on levels too large for it
-  double* s64;  // scratch of the one-launch FP64 steps (k_tbg.cu); null where the level does not take them
+  double* s64;  // scratch of the one-launch steps (k_tbg.cu); null where the level does not take them
+  float* s32;
   int xswap;  // 1: the FP32 x currently lives in y32 (after a temporally blocked smoothing)
   int ic0, ic1, jc0, jc1, kc0, kc1;  // interior box (1-based inclusive)
 };
@@ -315,21 +316,23 @@ struct TailListArgs {
 };
 void launch_tail_lists(const TailListArgs& a, int n, cudaStream_t s);
 
-// ---- a descent or ascent step of an FP64 2D level in one launch (k_tbg.cu)
+// ---- a descent or ascent step of a 2D level in one launch (k_tbg.cu): FP64, and the FP32 variable-coefficient operator
 constexpr int kTbgMaxPairs = 3;
+template <class T>
 struct TbgArgs {
-  const double *xs;                          // ascent: the descent's result (the level's scratch); descent
-                                             // of level 1: its x (x and y null: only s is written)
-  const double *b, *w, *cE, *cN, *d, *pc;    // pc: the level's Pcoef
-  const double *xc, *rc;                     // coarse x (prolonged), coarse Rcoef
+  const T *xs;                          // ascent: the descent's result (the level's scratch); descent of
+                                        // FP64 level 1: its x (x and y null: only s is written)
+  const T *b, *w, *cE, *cN, *d, *pc;    // pc: the level's Pcoef
+  const T *xc, *rc;                     // coarse x (prolonged), coarse Rcoef
   const uint8_t* m;
-  double *x, *y, *r, *s, *bc, *xcz;          // s: the scratch; bc, xcz: coarse b, and coarse x to zero
-  double cff;
+  T *x, *y, *r, *s, *bc, *xcz;          // s: the scratch; bc, xcz: coarse b, and coarse x to zero (y, r may be null)
+  T cff;
   int np, tx, ty, nh, ctx, cty, np_i, np_j;  // np: pairs of sweeps; np_i x np_j prolongation parents
 };
 // stencil TAIL_5 / TAIL_9 / TAIL_VC; mode 0: descent from x = +0 (or xs), 1:
 // descent from x = +0 (or xs) + Pcoef P(coarse x), 2: ascent
-void launch_step2d(const TbgArgs& a, int stencil, int mode, bool vertices, cudaStream_t s);
+void launch_step2d(const TbgArgs<double>& a, int stencil, int mode, bool vertices, cudaStream_t s);
+void launch_step2d(const TbgArgs<float>& a, int stencil, int mode, bool vertices, cudaStream_t s);  // TAIL_VC
 
 // 3D 7-point streaming blocked passes (k_tb3d.cu): nite (1 or 2) pairs over U
 bool launch_smooth_tb3d(int nite, const float* x, float* xo, const float* b, const float* w, float cff, int tx,

@@ -1,4 +1,5 @@
-"""The one-launch descent and ascent steps of FP64 2D levels (k_tbg.cu) against
+"""The one-launch descent and ascent steps of 2D levels (k_tbg.cu; FP64, and the
+FP32 ones of the variable-coefficient operator) against
 the separate kernels (option fused_descent = 0): every field of every level
 after cycles, bit for bit: the same operations in the same order, tolerance
 zero. Sizes put tile edges inside, at and beyond the array, on levels through
@@ -96,3 +97,20 @@ def test_values_outside_the_wet_interior_take_the_separate_kernels(upload):
         mg.close()
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("cycle", ["v", "f"])
+@pytest.mark.parametrize("size,pairs", [((470, 378), (2, 2)), ((661, 333), (3, 1)), ((392, 401), (1, 3)),
+                                        ((222, 150), (2, 2))])
+def test_mixed_varcoef_steps_are_bit_identical(cycle, size, pairs):
+    """The first three sizes' level 1 takes the register form of the FP32 steps, the other levels the general one."""
+    p = dict(operator="varcoef", cycle=cycle, npre=pairs[0], npost=pairs[1], omega=0.8, nlevels=6, precision="mixed",
+             residual_norm="l2")
+    out = []
+    for fused in (1, 0):
+        mg = _make(fused, *size, 9, **p)
+        _, _, hist = cfmg.solve(mg, history=True, maxite=6, tol=0.0)
+        out.append((hist, mg.data[1].x))
+        mg.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
