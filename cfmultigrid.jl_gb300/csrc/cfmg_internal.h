@@ -93,6 +93,12 @@ inline Geom geom(const Level& l) {
   return g;
 }
 
+// ---- the FP64 9-point operator on large levels (k_fix.cu)
+void launch_fix_sweep9(const double* x, double* y, const double* b, const double* w, double cff, const Geom& g,
+                       const Box& bx, cudaStream_t s);
+void launch_fix_resid9(double* r, const double* x, const double* b, const double* d, const uint8_t* m, const Geom& g,
+                       const Box& bx, cudaStream_t s);
+
 // ---- per-level operators (k_ops.cu), templated on the field type T
 // (double: bit-exact parity form; float: the mixed-precision cycles).
 template <class T>

@@ -84,6 +84,10 @@ inline long long box_cells(const Box& bx) {
 // all latency); at 104 x 88 x 56 (620 000 cells of a basin, a third wet) 10.2
 // and 13.6.
 constexpr long long kZeroMin = 1LL << 19;
+// The FP64 9-point operators' integer form (k_fix.cu) pays from a quarter of a
+// million cells: at 512^2 a sweep took 10.5 us with it and 12.6 without, at
+// 384^2 9.8 and 9.9.
+constexpr long long kFixMin = 1LL << 18;
 #define CFMG_ZS(K, N, ...)                                                                     \
   do {                                                                                         \
     if (sizeof(T) == 8 && (N) >= kZeroMin) launch_dep(K<T, sizeof(T) == 8>, __VA_ARGS__);      \
@@ -92,7 +96,7 @@ constexpr long long kZeroMin = 1LL << 19;
 inline bool box_empty(const Box& bx) { return bx.i1 < bx.i0 || bx.j1 < bx.j0 || bx.k1 < bx.k0; }
 static const dim3 kBoxBlk(64, 4, 1);
 
-template <class T, bool ZS>
+template <class T>
 __global__ void __launch_bounds__(kThreads) k_sweep9_2d(const T* __restrict__ x, T* __restrict__ y,
                                                         const T* __restrict__ b, const T* __restrict__ w, T cff,
                                                         Geom g, Box bx) {
@@ -100,7 +104,6 @@ __global__ void __launch_bounds__(kThreads) k_sweep9_2d(const T* __restrict__ x,
   BoxIdx q = box_idx(bx);
   if (!q.ok) return;
   const long long I = lin(g, q.i, q.j, q.k);
-  CFMG_ZERO_WARP(y[I], (zero_sweep<ZS_9>(x, b, w, x, x, cff, g.n1, 0, I, z)))
   d_sweep9(x, y, b, w, cff, g.n1, I);
 }
 
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(kThreads) k_resid7_3d(T* __restrict__ r, const
 }
 
 // residual of the 2D 9-point extension, interior box.
-template <class T, bool ZS>
+template <class T>
 __global__ void __launch_bounds__(kThreads) k_resid9_2d(T* __restrict__ r, const T* __restrict__ x,
                                                         const T* __restrict__ b, const T* __restrict__ d,
                                                         const uint8_t* __restrict__ m, Geom g, Box bx) {
@@ -164,7 +167,6 @@ __global__ void __launch_bounds__(kThreads) k_resid9_2d(T* __restrict__ r, const
   BoxIdx q = box_idx(bx);
   if (!q.ok) return;
   const long long I = lin(g, q.i, q.j, q.k);
-  CFMG_ZERO_WARP(r[I], (zero_resid<ZS_9>(x, b, d, x, x, g.n1, 0, I, z)))
   d_resid9(r, x, b, d, m, g.n1, I);
 }
 
@@ -895,7 +897,10 @@ template <class T>
 void launch_sweep9_2d(const T* x, T* y, const T* b, const T* w, T cff, const Geom& g, const Box& bx,
                       cudaStream_t s) {
   if (box_empty(bx)) return;
-  CFMG_ZS(k_sweep9_2d, box_cells(bx), box_grid(bx, kBoxBlk), kBoxBlk, 0, s, x, y, b, w, cff, g, bx);
+  if constexpr (sizeof(T) == 8) {
+    if (g.tz == 1 && box_cells(bx) >= kFixMin) return launch_fix_sweep9(x, y, b, w, cff, g, bx, s);
+  }
+  launch_dep(k_sweep9_2d<T>, box_grid(bx, kBoxBlk), kBoxBlk, 0, s, x, y, b, w, cff, g, bx);
 }
 template <class T>
 void launch_sweep19_3d(const T* x, T* y, const T* b, const T* w, T cff, const Geom& g, const Box& bx,
@@ -926,7 +931,10 @@ template <class T>
 void launch_resid9_2d(T* r, const T* x, const T* b, const T* d, const uint8_t* m, const Geom& g, const Box& bx,
                       cudaStream_t s) {
   if (box_empty(bx)) return;
-  CFMG_ZS(k_resid9_2d, box_cells(bx), box_grid(bx, kBoxBlk), kBoxBlk, 0, s, r, x, b, d, m, g, bx);
+  if constexpr (sizeof(T) == 8) {
+    if (g.tz == 1 && box_cells(bx) >= kFixMin) return launch_fix_resid9(r, x, b, d, m, g, bx, s);
+  }
+  launch_dep(k_resid9_2d<T>, box_grid(bx, kBoxBlk), kBoxBlk, 0, s, r, x, b, d, m, g, bx);
 }
 template <class T>
 void launch_resid19_3d(T* r, const T* x, const T* b, const T* d, const uint8_t* m, const Geom& g, const Box& bx,

@@ -237,8 +237,8 @@ struct ZeroAcc {
 __device__ __forceinline__ bool is_neg(double v) { return __double2hiint(v) < 0; }
 __device__ __forceinline__ bool is_fin(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 __device__ __forceinline__ double signed_zero(bool neg) { return neg ? -0.0 : 0.0; }
-enum ZeroStencil { ZS_5, ZS_7, ZS_9, ZS_19, ZS_VC };
-// faces (and for the 9- and 19-point operators diagonals) of cell I; false when a value is not a zero
+enum ZeroStencil { ZS_5, ZS_7, ZS_19, ZS_VC };
+// faces (and for the 19-point operator diagonals) of cell I; false when a value is not a zero
 template <int ST>
 __device__ __forceinline__ bool zero_nb(const double* x, const double* cE, const double* cN, long long I, long long n1,
                                         long long n2, bool& fneg, bool& dneg) {
@@ -252,13 +252,11 @@ __device__ __forceinline__ bool zero_nb(const double* x, const double* cE, const
     f.add(x[I - n2]);
     f.add(x[I + n2]);
   }
-  if (ST == ZS_9 || ST == ZS_19) {
+  if (ST == ZS_19) {
     d.add(x[I - 1 - n1]);
     d.add(x[I + 1 - n1]);
     d.add(x[I - 1 + n1]);
     d.add(x[I + 1 + n1]);
-  }
-  if (ST == ZS_19) {
     d.add(x[I - 1 - n2]);
     d.add(x[I + 1 - n2]);
     d.add(x[I - 1 + n2]);
@@ -275,7 +273,7 @@ __device__ __forceinline__ bool zero_nb(const double* x, const double* cE, const
   }
   fneg = f.neg();
   dneg = d.neg();
-  return ok && f.zero() && (ST == ZS_9 || ST == ZS_19 ? d.zero() : true);
+  return ok && f.zero() && (ST == ZS_19 ? d.zero() : true);
 }
 template <int ST>
 __device__ __forceinline__ bool zero_sweep(const double* x, const double* b, const double* w, const double* cE,
@@ -291,7 +289,7 @@ __device__ __forceinline__ bool zero_sweep(const double* x, const double* b, con
     return false;
   // b - faces (- diagonals) is -0 only from -0 minus sums that are all +0
   bool tneg = is_neg(bv) && !fneg;
-  if (ST == ZS_9 || ST == ZS_19) tneg = tneg && !dneg;
+  if (ST == ZS_19) tneg = tneg && !dneg;
   out = signed_zero(is_neg(xv) && !tneg);
   return true;
 }
@@ -305,7 +303,7 @@ __device__ __forceinline__ bool zero_resid(const double* x, const double* b, con
   c.add(bv);
   if (!zero_nb<ST>(x, cE, cN, I, n1, n2, fneg, dneg) || !c.zero() || !is_fin(dv)) return false;
   bool v = (is_neg(dv) != is_neg(xv)) && is_neg(bv) && !fneg;  // (d x + b) - faces
-  if (ST == ZS_9 || ST == ZS_19) v = v && !dneg;
+  if (ST == ZS_19) v = v && !dneg;
   out = signed_zero(v);  // whatever the mask: it keeps the sign of a zero
   return true;
 }
