@@ -1661,24 +1661,6 @@ __global__ void k_scale_from_norm(double* dscal, const double* partials, int npa
   }
 }
 
-__global__ void k_rhs32(const double* r, const uint8_t* m, const double* dscal, float* b32, float* r32, long long n) {
-  dep_wait();
-  long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= n) return;
-  double v = m[I] ? (r[I] - dscal[S_MEAN]) * dscal[S_SCALE] : 0.0;
-  float f = (float)v;
-  b32[I] = f;
-  r32[I] = f;
-}
-
-// x += e / scale (the FP64 solution update)
-__global__ void k_update(double* x, const float* e, const double* dscal, long long n) {
-  dep_wait();
-  long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= n) return;
-  x[I] = __fma_rn((double)e[I], dscal[S_ISCALE], x[I]);
-}
-
 // ------------------------------------------------------------- adjoint
 // wet-mean removal: x -= (sum msk x)/(sum msk) on wet cells, the sum in
 // Neumaier-compensated FP64 (k_mean_partial above) with a fixed-order final
@@ -1800,7 +1782,7 @@ int fused_residual(cfmg_handle* h) {
   }
   if (neumann) {
     Launch k(h, CFMG_K_CONVERT, 1, CFMG_MIXED);
-    launch_rhs32_mean(l1.r, l1.msk, h->dscal + S_MEAN2, l1.b32, l1.r32, (long long)l1.len, h->stream);
+    launch_rhs32(l1.r, l1.msk, h->dscal + S_MEAN2, h->dscal + S_CUR, l1.b32, l1.r32, (long long)l1.len, h->stream);
   }
   LAUNCH_OK(h);
   return CFMG_OK;
@@ -1861,14 +1843,14 @@ int mixed_iteration(cfmg_handle* h, int kind) {
   }
   const Level& l1 = h->lv[0];
   const long long n = (long long)l1.len;
-  const unsigned nb = (unsigned)((n + 255) / 256);
   const bool remove_mean = !vertices(h);
   TRY(flush(h));
   {
     Launch k(h, CFMG_K_CONVERT, 1, CFMG_MIXED, remove_mean ? 3 : 2);
     if (remove_mean) launch_mean_fix(l1.r, l1.msk, n, h->dscal, h->partials, h->stream);
     launch_dep(k_scale_from_norm, 1, kNormParts, 0, h->stream, h->dscal, h->partials, kNormParts, remove_mean);
-    launch_dep(k_rhs32, nb, 256, 0, h->stream, l1.r, l1.msk, h->dscal, l1.b32, l1.r32, n);
+    launch_rhs32(l1.r, l1.msk, h->dscal + S_MEAN, h->dscal + S_SCALE, l1.b32,
+                 kind == CFMG_CYCLE_F ? l1.r32 : nullptr, n, h->stream);
   }
   if (!lazy && !h->x1_zero && !step_ok<float>(h, 1)) TRY(zero_t<float>(h, 1, CFMG_X));
   LAUNCH_OK(h);
@@ -1877,7 +1859,7 @@ int mixed_iteration(cfmg_handle* h, int kind) {
   TRY(st);
   {
     Launch k(h, CFMG_K_CONVERT, 1, CFMG_MIXED);
-    launch_dep(k_update, nb, 256, 0, h->stream, l1.x, view<float>(l1).x, h->dscal, n);
+    launch_update_scaled(l1.x, view<float>(l1).x, h->dscal + S_ISCALE, n, h->stream);
   }
   LAUNCH_OK(h);
   return CFMG_OK;

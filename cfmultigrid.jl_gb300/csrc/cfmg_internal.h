@@ -485,8 +485,8 @@ void launch_resid_fused(int kind, double* r, const double* x, const double* b, c
                         float* r32, bool neumann, double* partials, cudaStream_t s);
 void launch_fused_final(const double* partials, double* ds, const double* normb, const double* nwet, int norm_kind,
                         cudaStream_t s, const LoopTest* lt = nullptr);
-void launch_rhs32_mean(const double* r, const uint8_t* m, const double* mean_scale, float* b32, float* r32,
-                       long long n, cudaStream_t s);
+void launch_rhs32(const double* r, const uint8_t* m, const double* mean, const double* scale, float* b32, float* r32,
+                  long long n, cudaStream_t s);
 void launch_update_scaled(double* x, const float* e, const double* iscale, long long n, cudaStream_t s);
 // wet sum of r in fixed point, kNormParts partials; ds[S_NORM] = sum r^2 bounds it
 void launch_mean_fix(const double* r, const uint8_t* m, long long n, const double* ds, double* partials,

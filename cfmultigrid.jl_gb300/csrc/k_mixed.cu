@@ -132,25 +132,58 @@ __global__ void __launch_bounds__(kMxParts) k_fused_final(const double* __restri
   }
 }
 
-// Neumann second pass: b32 = r32 = msk ? (r - mean) * scale : 0, with
-// ms[0] = S_MEAN2 and ms[1] = S_CUR (the scale of this right-hand side)
-__global__ void k_rhs32_mean(const double* __restrict__ r, const uint8_t* __restrict__ m,
-                             const double* __restrict__ ms, float* __restrict__ b32, float* __restrict__ r32,
-                             long long n) {
+// The FP32 right-hand side (r - mean) * scale on wet cells, four cells a
+// thread with their loads in flight. The FP64 pipe bounds it: the conversion
+// is done by integer operations, which leaves that pipe two of three a cell
+// (2048^2: 26 us with all three; 15.2 now). r32: where the cycle reads it.
+__global__ void __launch_bounds__(256) k_rhs32(const double* __restrict__ r, const uint8_t* __restrict__ m,
+                                               const double* __restrict__ mean_at,
+                                               const double* __restrict__ scale_at, float* __restrict__ b32,
+                                               float* __restrict__ r32, long long n) {
   dep_wait();
-  long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= n) return;
-  const float f = m[I] ? (float)((r[I] - ms[0]) * ms[S_CUR - S_MEAN2]) : 0.f;
-  b32[I] = f;
-  r32[I] = f;
+  const double mean = *mean_at, scale = *scale_at;
+  const long long I0 = (long long)blockIdx.x * 1024 + threadIdx.x;
+  double v[4];
+  bool wet[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const long long I = I0 + 256 * q;
+    wet[q] = I < n && m[I] != 0;
+    v[q] = I < n ? r[I] : 0.0;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const long long I = I0 + 256 * q;
+    const float f = wet[q] ? d2f(__dmul_rn(__dsub_rn(v[q], mean), scale)) : 0.f;
+    if (I < n) {
+      b32[I] = f;
+      if (r32) r32[I] = f;
+    }
+  }
 }
 
-// x += e * iscale
-__global__ void k_update_scaled(double* __restrict__ x, const float* __restrict__ e, const double* __restrict__ is,
-                                long long n) {
+// x += e * iscale (the FP64 solution update), four cells a thread: e is
+// converted by integer operations, which leaves the FP64 pipe the FMA and the
+// pass its memory traffic (2048^2: 18.3 us with the conversion on that pipe,
+// 12.2 now)
+__global__ void __launch_bounds__(256) k_update_scaled(double* __restrict__ x, const float* __restrict__ e,
+                                                       const double* __restrict__ iscale, long long n) {
   dep_wait();
-  long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (I < n) x[I] = __fma_rn((double)e[I], is[0], x[I]);
+  const double is = *iscale;
+  const long long I0 = (long long)blockIdx.x * 1024 + threadIdx.x;
+  double v[4];
+  float d[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const long long I = I0 + 256 * q;
+    v[q] = I < n ? x[I] : 0.0;
+    d[q] = I < n ? e[I] : 0.f;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const long long I = I0 + 256 * q;
+    if (I < n) x[I] = __fma_rn(f2d_pow2(d[q], 0, 1.0), is, v[q]);
+  }
 }
 
 // ----------------------------------------------------------------------
@@ -1019,13 +1052,13 @@ void launch_fused_final(const double* partials, double* ds, const double* normb,
   launch_dep(k_fused_final, 1, kMxParts, 0, s, partials, ds, normb, nwet, norm_kind, lt ? *lt : LoopTest{});
 }
 
-void launch_rhs32_mean(const double* r, const uint8_t* m, const double* mean_scale, float* b32, float* r32,
-                       long long n, cudaStream_t s) {
-  launch_dep(k_rhs32_mean, (unsigned)((n + 255) / 256), 256, 0, s, r, m, mean_scale, b32, r32, n);
+void launch_rhs32(const double* r, const uint8_t* m, const double* mean, const double* scale, float* b32, float* r32,
+                  long long n, cudaStream_t s) {
+  launch_dep(k_rhs32, (unsigned)((n + 1023) / 1024), 256, 0, s, r, m, mean, scale, b32, r32, n);
 }
 
 void launch_update_scaled(double* x, const float* e, const double* iscale, long long n, cudaStream_t s) {
-  launch_dep(k_update_scaled, (unsigned)((n + 255) / 256), 256, 0, s, x, e, iscale, n);
+  launch_dep(k_update_scaled, (unsigned)((n + 1023) / 1024), 256, 0, s, x, e, iscale, n);
 }
 
 }  // namespace cfmg

@@ -615,6 +615,19 @@ __device__ __forceinline__ double f2d_pow2(float e, int p, double s2p) {
   if (!zero && !normal) v = f2d_pow2_slow(e, s2p);
   return v;
 }
+// v as a float, to nearest even, with integer operations on the bits where v
+// and the result are zero or normal; else on the FP64 pipe, out of line
+static __device__ __noinline__ float d2f_slow(double v) { return (float)v; }
+__device__ __forceinline__ float d2f(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const int fe = (int)((hi >> 20) & 0x7ffu) - 1023 + 127;
+  const unsigned m = ((hi & 0xfffffu) << 3) | (lo >> 29);
+  const unsigned up = ((lo & 0x1fffffffu) + 0x0fffffffu + (m & 1u)) >> 29;  // past half, or half and odd
+  const bool zero = ((hi << 1) | lo) == 0u;
+  float f = __uint_as_float((hi & 0x80000000u) | (zero ? 0u : ((unsigned)fe << 23) + m + up));
+  if (!zero && (fe < 1 || fe > 253)) f = d2f_slow(v);
+  return f;
+}
 // the exponent p of a power of two 2^p held in a double
 __device__ __forceinline__ int pow2_exponent(double v) {
   return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffULL) - 1023;
