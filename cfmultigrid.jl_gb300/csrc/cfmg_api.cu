@@ -88,7 +88,7 @@ struct cfmg_handle {
   // 3D 7-point: dq with rows padded to 16 bytes for the TMA-staged pass
   // (k_resid3d.cu, CFMG_OPT_STAGED_RESIDUAL); r3_ran once that pass ran
   int8_t* dqp = nullptr;
-  uint8_t* tcol = nullptr;   // wet flags of the staged pass's (tile, plane) pairs
+  int* tcol = nullptr;       // wet planes of the staged pass's tiles
   uint8_t* sflag = nullptr;  // wet flags of the strip pass's (plane, row, strip) triples
   bool r3_on = true, r3_ran = false;
   int r3_rows = 2;  // rows of its tile per thread (1 or 2)
@@ -1524,7 +1524,7 @@ int prepare_int(cfmg_handle* h) {
   const int kind = resid_kind(h);
   if (!fused_ok(h)) return CFMG_OK;
   const Level& l1 = h->lv[0];
-  if (!h->dq) CUDA_OK(h, cudaMalloc((void**)&h->dq, l1.len));
+  if (!h->dq) CUDA_OK(h, cudaMalloc((void**)&h->dq, (l1.len + 3) & ~(size_t)3));
   int* ok = (int*)h->partials;  // scratch
   const int one = 1;
   CUDA_OK(h, cudaMemcpyAsync(ok, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
@@ -1542,7 +1542,7 @@ int prepare_int(cfmg_handle* h) {
     launch_pad_dq(h->dq, h->dqp, l1.tx, txp, (long long)l1.ty * l1.tz, h->stream);
     const long long nt = resid3d_tcol_size(geom(l1), interior(l1));
     if (nt > 0) {
-      if (!h->tcol) CUDA_OK(h, cudaMalloc((void**)&h->tcol, (size_t)nt));
+      if (!h->tcol) CUDA_OK(h, cudaMalloc((void**)&h->tcol, sizeof(int) * (size_t)nt));
       launch_make_tcol(l1.msk, h->tcol, geom(l1), interior(l1), h->stream);
     }
   }
@@ -1754,7 +1754,7 @@ int fused_residual(cfmg_handle* h) {
       float* r32 = h->d.cycle == CFMG_CYCLE_F ? l1.r32 : nullptr;
       const bool r3 = kind == OPK_RESID7 && h->r3_on &&
                       launch_resid_int3d(l1.x, l1.b, h->dqp, g, bx, h->dscal, l1.b32, r32, neumann, h->partials,
-                                         h->stream, h->r3_rows, h->dry_on ? h->tcol : nullptr);
+                                         h->stream, h->r3_rows, h->tcol, r32 || !h->dry_on);
       h->r3_ran |= r3;
       if (kind == OPK_RESID19)
         launch_resid_int19(l1.x, l1.b, h->dq, g, bx, h->dscal, l1.b32, r32, neumann, h->partials, h->stream);
@@ -1763,7 +1763,8 @@ int fused_residual(cfmg_handle* h) {
         launch_resid_int(kind, l1.x, l1.b, h->dq, g, bx, lo, n, h->dscal, l1.b32, r32, neumann, h->partials,
                          h->stream);
       launch_fused_final(h->partials, h->dscal, h->dscal + S_NORMB, neumann ? h->dscal + S_NWET : nullptr,
-                         h->d.norm_kind, h->stream, h->loop);
+                         h->d.norm_kind, h->stream, h->loop,
+                         kind == OPK_RESID7 ? 0 : kFloatSums);
     }
     if (neumann) {
       Launch k(h, CFMG_K_CONVERT, 1, CFMG_MIXED);

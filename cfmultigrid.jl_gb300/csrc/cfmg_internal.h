@@ -195,12 +195,13 @@ void launch_loop_start(const LoopTest& lt, cudaStream_t s);
 constexpr int kNormParts = 1024;
 // the handle's partial-sum scratch: two sums per block for the fused
 // residual pass of the mixed loop (k_mixed.cu), one for the norms
-constexpr int kPartials = 2 * kNormParts;
+constexpr int kPartials = 3 * kNormParts;
 // the fused residual passes of the mixed loop (k_mixed.cu, k_resid3d.cu):
-// threads per block, and at most kMxParts blocks with two partial sums each
+// threads per block, and at most kMxParts blocks with a sum of r^2 and one of r
+// (two words in the fixed-point 7-point passes) each
 constexpr int kMxThreads = 256;
 constexpr int kMxParts = 1024;
-static_assert(2 * kMxParts <= kPartials, "the fused pass writes 2*kMxParts partial sums");
+static_assert(3 * kMxParts <= kPartials, "a fused pass writes up to 3*kMxParts partial sums");
 
 // ---- operator descriptors and the coarse-level program engine (k_coarse.cu)
 // One Op describes one launch-worth of work on one level: its kind, the
@@ -483,8 +484,11 @@ enum Scal { S_NORM = 0, S_RES = 1, S_NORMB = 2, S_NWET = 3, S_SCALE = 4, S_MEAN 
 void launch_resid_fused(int kind, double* r, const double* x, const double* b, const double* d, const uint8_t* m,
                         const Geom& g, const Box& bx, long long lo, long long n, const double* scale, float* b32,
                         float* r32, bool neumann, double* partials, cudaStream_t s);
+// q: partials whose sums of r are integers in units of 2^-(fix_exponent + q) (the
+// fixed-point 7-point passes); kFloatSums: FP64 ones
+constexpr int kFloatSums = 1 << 20;
 void launch_fused_final(const double* partials, double* ds, const double* normb, const double* nwet, int norm_kind,
-                        cudaStream_t s, const LoopTest* lt = nullptr);
+                        cudaStream_t s, const LoopTest* lt = nullptr, int q = kFloatSums);
 void launch_rhs32(const double* r, const uint8_t* m, const double* mean, const double* scale, float* b32, float* r32,
                   long long n, cudaStream_t s);
 void launch_update_scaled(double* x, const float* e, const double* iscale, long long n, cudaStream_t s);
@@ -517,13 +521,13 @@ void launch_resid_int19(const double* x, const double* b, const int8_t* dq, cons
 // (odd tx, misaligned arrays, no tensor-map encoder): use launch_resid_int2d.
 int dq_pitch(int tx);
 void launch_pad_dq(const int8_t* dq, int8_t* dqp, int tx, int txp, long long rows, cudaStream_t s);
-// tcol (optional): per-(tile, plane) wet flags (launch_make_tcol); tasks whose
-// planes are all dry are skipped (two rows a thread, and r32 not written, only)
+// tcol (optional): the tiles' ranges of wet planes (launch_make_tcol), by which two-row
+// blocks share the work; all: the dry planes outside are written too
 bool launch_resid_int3d(const double* x, const double* b, const int8_t* dqp, const Geom& g, const Box& bx,
                         double* ds, float* b32, float* r32, bool neumann, double* partials, cudaStream_t s,
-                        int rows_per_thread, const uint8_t* tcol = nullptr);
+                        int rows_per_thread, const int* tcol, bool all);
 long long resid3d_tcol_size(const Geom& g, const Box& bx);
-void launch_make_tcol(const uint8_t* m, uint8_t* tcol, const Geom& g, const Box& bx, cudaStream_t s);
+void launch_make_tcol(const uint8_t* m, int* tcol, const Geom& g, const Box& bx, cudaStream_t s);
 // skip_dry: groups of 16 dry cells are neither read nor written (their b32 is +0 already)
 void launch_rhs32_shift(const uint8_t* m, const double* mean_scale, float* b32, float* r32, long long n,
                         cudaStream_t s, bool skip_dry = false);

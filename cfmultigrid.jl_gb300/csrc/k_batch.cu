@@ -300,6 +300,7 @@ __global__ void __launch_bounds__(kBThreads) k_bres(const BInst* __restrict__ bi
   }
 }
 
+constexpr int kBRing = 3;  // rows in flight; a ring of kBRing + 1 slots (a power of two)
 // Integer form of the fused residual (see k_resid_int2d in k_mixed.cu):
 // one warp per task {instance, strip of 32 columns, chunk of kBIntRows
 // rows}; the fixed-point exponent is the instance's own (BS_MAXX from its
@@ -312,6 +313,8 @@ __global__ void __launch_bounds__(kBThreads) k_bres_int(const BInst* __restrict_
                                                         double* __restrict__ partials) {
   dep_wait();
   constexpr int q = (KIND == OPK_RESID9) ? 2 : 0;
+  __shared__ double2 ring[kBThreads / 32][kBRing + 1][32];
+  __shared__ int dring[kBThreads / 32][kBRing + 1][32];
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -322,7 +325,7 @@ __global__ void __launch_bounds__(kBThreads) k_bres_int(const BInst* __restrict_
     const double mx = fmax(B.sc[BS_MAXX], B.sc[BS_MAXB]);
     int ex = 0;
     if (mx > 0 && isfinite(mx)) frexp(mx, &ex);
-    const int k = 58 - ex;
+    const int k = fix_k(ex);
     const double scale = B.sc[BS_NEXT];
     const float fm = (float)ldexp(scale, -(k + q));
     const long long n1 = B.g.n1, len = B.len;
@@ -330,52 +333,65 @@ __global__ void __launch_bounds__(kBThreads) k_bres_int(const BInst* __restrict_
     const int c = B.c0 + en.y * kBIntCols + lane - 1;  // lanes 1..30 own the strip
     const bool col_ok = lane >= 1 && lane <= kBIntCols && c < B.c0 + B.ncols;
     const int ra = en.z * kBIntRows, rb = min(ra + kBIntRows, B.nrows);
-    auto at = [&](long long J) { return x[J < 0 ? 0 : (J >= len ? len - 1 : J)]; };
-    auto conv_row = [&](double xc, long long& W, long long& C, long long& E) {
-      C = to_fix(xc, k);
-      W = __shfl_up_sync(0xffffffffu, C, 1);
-      E = __shfl_down_sync(0xffffffffu, C, 1);
+    auto in = [&](long long J) { return J < 0 ? 0 : (J >= len ? len - 1 : J); };
+    const long long I0 = B.row0 + (long long)ra * n1 + c;
+    // copy j: x of row ra+1+j, b of row ra+j and the word that holds its dq, into slot j of the lane's ring
+    auto request = [&](int j) {
+      const long long I = I0 + (long long)j * n1;
+      if (ra + j < rb) {
+        double2* at = &ring[threadIdx.x >> 5][j & kBRing][lane];
+        cp_async<8>(&at->x, x + in(I + n1));
+        if (col_ok) {
+          cp_async<8>(&at->y, B.b + I);
+          cp_async<4>(&dring[threadIdx.x >> 5][j & kBRing][lane], B.dq + (I & ~3LL));
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    long long I = B.row0 + (long long)ra * n1 + c;
-    long long Wm, Cm, Em, W0, C0, E0, Wp, Cp, Ep;
-    conv_row(at(I - n1), Wm, Cm, Em);
-    conv_row(at(I), W0, C0, E0);
-    double nc = at(I + n1);  // one row of look-ahead (see k_resid_int2d)
-    double nb = col_ok ? B.b[I] : 0.0;
-    int nd = col_ok ? B.dq[I] : -1;
+#pragma unroll
+    for (int j = 0; j < kBRing; ++j) request(j);
+    // of the row before and the row at hand: the centre and the sum of its two neighbours
+    long long Cm = to_fix(x[in(I0 - n1)], k), C0 = to_fix(x[in(I0)], k);
+    long long rsm = __shfl_up_sync(0xffffffffu, Cm, 1) + __shfl_down_sync(0xffffffffu, Cm, 1);
+    long long rs0 = __shfl_up_sync(0xffffffffu, C0, 1) + __shfl_down_sync(0xffffffffu, C0, 1);
     float hi = 0.f, lo = 0.f;
     __int128 s1 = 0;
-    for (int r = ra; r < rb; ++r, I += n1) {
-      conv_row(nc, Wp, Cp, Ep);
-      const double cb = nb;
-      const int d = nd;
-      if (r + 1 < rb) {
-        nc = at(I + 2 * n1);
-        nb = col_ok ? B.b[I + n1] : 0.0;
-        nd = col_ok ? B.dq[I + n1] : -1;
-      }
-      if (col_ok) {
-        long long R = 0;
-        if (d >= 0) {
-          const long long Bf = to_fix(cb, k);
-          if (KIND == OPK_RESID9)
-            R = (long long)d * C0 + 4 * Bf - 2 * (((W0 + E0) + Cm) + Cp) - (((Wm + Em) + Wp) + Ep);
-          else
-            R = (long long)d * C0 + Bf - (((W0 + E0) + Cm) + Cp);
-        }
+#pragma unroll 3
+    for (int r = ra; r < rb; ++r) {
+      const long long I = I0 + (long long)(r - ra) * n1;
+      asm volatile("cp.async.wait_group %0;" ::"n"(kBRing - 1) : "memory");
+      const double2 v = ring[threadIdx.x >> 5][(r - ra) & kBRing][lane];
+      const int dw = dring[threadIdx.x >> 5][(r - ra) & kBRing][lane];
+      request(r - ra + kBRing);
+      const int d = col_ok ? (dw << (24 - 8 * (int)(I & 3))) >> 24 : -1;
+      const long long Cp = to_fix(v.x, k);
+      const long long rsp = __shfl_up_sync(0xffffffffu, Cp, 1) + __shfl_down_sync(0xffffffffu, Cp, 1);
+      if (__any_sync(0xffffffffu, d >= 0)) {
+        const long long Bf = to_fix(v.y, k);
+        long long R;
+        if (KIND == OPK_RESID9) R = (long long)d * C0 + 4 * Bf - 2 * (rs0 + Cm + Cp) - (rsm + rsp);
+        else R = (long long)d * C0 + Bf - (rs0 + Cm + Cp);
+        R = d >= 0 ? R : 0LL;
         const float f = __fmul_rn(__ll2float_rn(R), fm);
-        B.b32[I] = f;
+        if (col_ok) {
+          B.b32[I] = f;
+          if (!NEUMANN) B.r32[I] = f;
+        }
         if (NEUMANN) s1 += (__int128)R;
-        else B.r32[I] = f;
         // p + e = f^2 exactly; (hi, lo) += p + e by TwoSum (explicit _rn
         // operations: a contracted hi + f*f would break the error terms)
         const float p = __fmul_rn(f, f), e = __fmaf_rn(f, f, -p);
         const float sn = __fadd_rn(hi, p), bp = __fsub_rn(sn, hi);
         lo = __fadd_rn(lo, __fadd_rn(__fadd_rn(__fsub_rn(hi, __fsub_rn(sn, bp)), __fsub_rn(p, bp)), e));
         hi = sn;
+      } else if (col_ok) {
+        B.b32[I] = 0.f;
+        if (!NEUMANN) B.r32[I] = 0.f;
       }
-      Wm = W0; Cm = C0; Em = E0;
-      W0 = Wp; C0 = Cp; E0 = Ep;
+      Cm = C0;
+      rsm = rs0;
+      C0 = Cp;
+      rs0 = rsp;
     }
     double a2 = ((double)hi + (double)lo) / (scale * scale);
     double a1 = NEUMANN ? ldexp(__dadd_rn(__dmul_rn((double)(long long)(s1 >> 64), 18446744073709551616.0),

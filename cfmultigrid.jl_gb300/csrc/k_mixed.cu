@@ -92,16 +92,24 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_fused(double* __restrict__
 // 2^-round(log2(rms)) goes to S_NEXT (powers of two, exact both ways).
 __global__ void __launch_bounds__(kMxParts) k_fused_final(const double* __restrict__ partials, double* ds,
                                                           const double* normb, const double* nwet, int norm_kind,
-                                                          LoopTest lt) {
+                                                          LoopTest lt, int q) {
   dep_wait();
   __shared__ double a[kMxParts], c[kMxParts];
+  __shared__ __int128 ci[kMxParts];
+  const bool exact = q != kFloatSums;
   a[threadIdx.x] = partials[threadIdx.x];
   c[threadIdx.x] = partials[kMxParts + threadIdx.x];
+  if (exact)
+    ci[threadIdx.x] = (__int128)(((unsigned __int128)(unsigned long long)__double_as_longlong(
+                                      partials[2 * kMxParts + threadIdx.x])
+                                  << 64) |
+                                 (unsigned long long)__double_as_longlong(c[threadIdx.x]));
   __syncthreads();
   for (int w = kMxParts / 2; w > 0; w >>= 1) {
     if ((int)threadIdx.x < w) {
       a[threadIdx.x] += a[threadIdx.x + w];
-      c[threadIdx.x] += c[threadIdx.x + w];
+      if (exact) ci[threadIdx.x] += ci[threadIdx.x + w];
+      else c[threadIdx.x] += c[threadIdx.x + w];
     }
     __syncthreads();
   }
@@ -117,7 +125,8 @@ __global__ void __launch_bounds__(kMxParts) k_fused_final(const double* __restri
       ds[S_RES] = (*normb > 0.0) ? sqrt(sum / *normb) : 0.0;
     }
     const double nw = (nwet && *nwet > 0) ? *nwet : 1.0;
-    ds[S_MEAN2] = nwet ? c[0] / nw : 0.0;
+    const double s1 = exact ? ldexp(int_to_double(ci[0]), -(fix_exponent(ds) + q)) : c[0];
+    ds[S_MEAN2] = nwet ? s1 / nw : 0.0;
     const double used = ds[S_NEXT];
     ds[S_CUR] = used;
     ds[S_ICUR] = 1.0 / used;
@@ -257,31 +266,7 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int(const double* __restri
     if (NEUMANN) s1 += (__int128)R;
     else if (r32) r32[I] = f;
   }
-  // per-thread exact sum r -> double (hi 2^64 + lo)
-  const double s1d = NEUMANN ? __dadd_rn(__dmul_rn((double)(long long)(s1 >> 64), 18446744073709551616.0),
-                                         (double)(unsigned long long)s1)
-                             : 0.0;
-  __shared__ double sh2[kMxThreads / 32], sh1[kMxThreads / 32];
-  double a2 = s2, a1 = s1d;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a2 += __shfl_down_sync(0xffffffffu, a2, o);
-    a1 += __shfl_down_sync(0xffffffffu, a1, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    sh2[threadIdx.x >> 5] = a2;
-    sh1[threadIdx.x >> 5] = a1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double u = 0.0, v = 0.0;
-    for (int w = 0; w < kMxThreads / 32; ++w) {
-      u += sh2[w];
-      v += sh1[w];
-    }
-    partials[blockIdx.x] = ldexp(u, -2 * (k + q));
-    partials[kMxParts + blockIdx.x] = ldexp(v, -(k + q));
-  }
+  int_partials<KIND == OPK_RESID7>(s2, s1, -2 * (k + q), k + q, partials);
 }
 
 // Strips of rows (2D, and 3D plane by plane): the same residual with every
@@ -293,8 +278,11 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int(const double* __restri
 // adjacent lanes. Integer sums are exact, so each row's west + east sum
 // serves as the start of its faces (as centre row) and of the diagonals of
 // the rows above and below. The loop body covers 6 rows, so the rotation of
-// the row window (period 3) and of the load queue (period 2) costs no moves;
-// x is loaded two rows ahead, b and dq one row ahead of their use. The
+// the row window (period 3) costs no moves. x, b and dq come through a ring in
+// shared memory that each lane fills for itself with asynchronous copies, three
+// rows ahead: loads into registers that far ahead waited for one another on the
+// few scoreboards a warp has, and the one-byte loads of dq, a row ahead, held
+// each row up (4096^2: 114 us with those, 107 now, 99 without dq at all). The
 // residual norm is summed from the FP32 right-hand-side values f = r*scale
 // (exact squares via FMA, double-float accumulation per thread, FP64
 // across threads), so the FP64 pipe does one conversion a cell. The grid is
@@ -306,6 +294,7 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int(const double* __restri
 constexpr int kIntCols = 30;  // output columns per warp strip
 static_assert(kIntCols + 1 < kResidIntReach, "a warp reaches kIntCols + 1 columns beyond its strip's first");
 constexpr int kIntUnroll = 6;  // rows per loop body; rows per task is a multiple
+constexpr int kIntRing = 3;    // rows in flight; a ring of kIntRing + 1 slots (a power of two)
 
 struct StripSpace {
   long long len;   // array length
@@ -340,6 +329,8 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int2d(const double* __rest
   const long long per_plane = (long long)sp.nstrips * nchunks;
   const long long ntasks = per_plane * sp.nplanes;
   const long long n1 = sp.n1;
+  __shared__ double2 ring[kMxThreads / 32][kIntRing + 1][32];
+  __shared__ int dring[kMxThreads / 32][kIntRing + 1][32];
   float hi = 0.f, lo = 0.f;  // double-float sum of f^2
   __int128 s1 = 0;
   for (long long task = warp0; task < ntasks; task += nwarps) {
@@ -363,10 +354,21 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int2d(const double* __rest
     long long Cm = to_fix(xp[-n1], k), C0 = to_fix(xp[0], k);
     long long rsm = __shfl_up_sync(0xffffffffu, Cm, 1) + __shfl_down_sync(0xffffffffu, Cm, 1);
     long long rs0 = __shfl_up_sync(0xffffffffu, C0, 1) + __shfl_down_sync(0xffffffffu, C0, 1);
-    double xa = xp[n1];
-    double xb = ra + 2 <= rb ? xp[2 * n1] : 0.0;
-    double ba = col_ok ? b[I0] : 0.0;
-    int da = col_ok ? dq[I0] : -1;
+    // copy j: x of row ra+1+j, b of row ra+j and the word that holds its dq, into slot j of the lane's ring
+    auto request = [&](int j) {
+      const long long I = I0 + (long long)j * n1;
+      double2* at = &ring[threadIdx.x >> 5][j & kIntRing][lane];
+      if (ra + j < rb) {
+        cp_async<8>(&at->x, x + I + n1);
+        if (col_ok) {
+          cp_async<8>(&at->y, b + I);
+          cp_async<4>(&dring[threadIdx.x >> 5][j & kIntRing][lane], dq + (I & ~3LL));
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int j = 0; j < kIntRing; ++j) request(j);
     double za = 0.0, zb = 0.0;  // 7-point: x of the planes below and above, row ra
     if (KIND == OPK_RESID7 && col_ok) {
       za = xp[-sp.n2];
@@ -376,16 +378,16 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int2d(const double* __rest
     // last step, so in the unguarded 6-row groups it costs no register moves
     auto row_step = [&](int r) {
       const long long I = I0 + (long long)(r - ra) * n1;
-      // row r+1 converted; row r+3 of x and row r+1 of b, dq requested
-      const long long Cp = to_fix(xa, k);
+      // row r+1 converted; the rows kIntRing further on requested
+      asm volatile("cp.async.wait_group %0;" ::"n"(kIntRing - 1) : "memory");
+      const double2 v = ring[threadIdx.x >> 5][(r - ra) & kIntRing][lane];
+      const int dw = dring[threadIdx.x >> 5][(r - ra) & kIntRing][lane];
+      request(r - ra + kIntRing);
+      const long long Cp = to_fix(v.x, k);
       const long long rsp = __shfl_up_sync(0xffffffffu, Cp, 1) + __shfl_down_sync(0xffffffffu, Cp, 1);
-      const double cb = ba, clo = za, chi = zb;
-      const int d = da;
-      xa = xb;
-      if (r + 3 <= rb) xb = x[I + 3 * n1];
+      const double cb = v.y, clo = za, chi = zb;
+      const int d = col_ok ? (dw << (24 - 8 * (int)(I & 3))) >> 24 : -1;
       if (r + 1 < rb) {
-        ba = col_ok ? b[I + n1] : 0.0;
-        da = col_ok ? dq[I + n1] : -1;
         if (KIND == OPK_RESID7 && col_ok) {
           za = x[I + n1 - sp.n2];
           zb = x[I + n1 + sp.n2];
@@ -424,34 +426,7 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int2d(const double* __rest
     for (; r0 < rb; ++r0) row_step(r0);
   }
   // sum f^2 -> sum r^2 = sum f^2 / scale^2 (exact power of two)
-  const double s2d = ((double)hi + (double)lo) / (scale * scale);
-  const double s1d = NEUMANN ? ldexp(__dadd_rn(__dmul_rn((double)(long long)(s1 >> 64), 18446744073709551616.0),
-                                               (double)(unsigned long long)s1),
-                                     -(k + q))
-                             : 0.0;
-  __shared__ double sh2[kMxThreads / 32], sh1[kMxThreads / 32];
-  double a2 = s2d, a1 = s1d;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a2 += __shfl_down_sync(0xffffffffu, a2, o);
-    a1 += __shfl_down_sync(0xffffffffu, a1, o);
-  }
-  if (lane == 0) {
-    sh2[threadIdx.x >> 5] = a2;
-    sh1[threadIdx.x >> 5] = a1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double u = 0.0, v = 0.0;
-    for (int w = 0; w < kMxThreads / 32; ++w) {
-      u += sh2[w];
-      v += sh1[w];
-    }
-    partials[blockIdx.x] = u;
-    partials[kMxParts + blockIdx.x] = v;
-    // the final pass reads kMxParts partials: the blocks clear the unused ones
-    for (int i = gridDim.x + blockIdx.x; i < kMxParts; i += gridDim.x) partials[i] = partials[kMxParts + i] = 0.0;
-  }
+  int_partials<KIND == OPK_RESID7>(((double)hi + (double)lo) / (scale * scale), s1, 0, k + q, partials);
 }
 
 template <int KIND, bool NEUMANN>
@@ -552,7 +527,7 @@ __global__ void __launch_bounds__(256) k_mean_fix(const double* __restrict__ r, 
     s += (__int128)((m2 ? to_fix(v2, k) : 0LL)) + (m3 ? to_fix(v3, k) : 0LL);
   }
   for (; I < n; I += st) s += m[I] ? to_fix(r[I], k) : 0LL;
-  double v = __dadd_rn(__dmul_rn((double)(long long)(s >> 64), 18446744073709551616.0), (double)(unsigned long long)s);
+  double v = int_to_double(s);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   __shared__ double sh[8];
@@ -657,32 +632,7 @@ __global__ void __launch_bounds__(kMxThreads, 4) k_resid_int19(const double* __r
       C0 = C; F0 = F; D0 = D;
     }
   }
-  double a2 = s2;
-  double a1 = NEUMANN ? ldexp(__dadd_rn(__dmul_rn((double)(long long)(s1 >> 64), 18446744073709551616.0),
-                                        (double)(unsigned long long)s1),
-                              -(k + q))
-                      : 0.0;
-  __shared__ double sh2[kMxThreads / 32], sh1[kMxThreads / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a2 += __shfl_down_sync(0xffffffffu, a2, o);
-    a1 += __shfl_down_sync(0xffffffffu, a1, o);
-  }
-  if (li == 0) {
-    sh2[lj] = a2;
-    sh1[lj] = a1;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    double u = 0.0, v = 0.0;
-    for (int w = 0; w < kMxThreads / 32; ++w) {
-      u += sh2[w];
-      v += sh1[w];
-    }
-    partials[blockIdx.x] = ldexp(u, -2 * (k + q));
-    partials[kMxParts + blockIdx.x] = v;
-    for (int i = gridDim.x + blockIdx.x; i < kMxParts; i += gridDim.x) partials[i] = partials[kMxParts + i] = 0.0;
-  }
+  int_partials<false>(s2, s1, -2 * (k + q), k + q, partials);
 }
 
 void launch_resid_int19(const double* x, const double* b, const int8_t* dq, const Geom& g, const Box& bx,
@@ -1048,8 +998,8 @@ void launch_resid_fused(int kind, double* r, const double* x, const double* b, c
 }
 
 void launch_fused_final(const double* partials, double* ds, const double* normb, const double* nwet, int norm_kind,
-                        cudaStream_t s, const LoopTest* lt) {
-  launch_dep(k_fused_final, 1, kMxParts, 0, s, partials, ds, normb, nwet, norm_kind, lt ? *lt : LoopTest{});
+                        cudaStream_t s, const LoopTest* lt, int q) {
+  launch_dep(k_fused_final, 1, kMxParts, 0, s, partials, ds, normb, nwet, norm_kind, lt ? *lt : LoopTest{}, q);
 }
 
 void launch_rhs32(const double* r, const uint8_t* m, const double* mean, const double* scale, float* b32, float* r32,

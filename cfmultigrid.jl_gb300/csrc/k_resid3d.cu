@@ -69,7 +69,6 @@ struct R3Space {
   int c0, r0, p0;    // 0-based column, row and plane of the box's first cell
   int ni, nj, nk;    // box extent
   int nti, ntj;      // column tiles in i and j
-  int kt, nkc;       // planes per task, runs of planes along k
   long long n1, n2;  // strides of b32 and r32 (elements)
 };
 
@@ -109,36 +108,85 @@ __device__ __forceinline__ void tma3(unsigned dst, const CUtensorMap* map, int c
       : "memory");
 }
 
-struct R3Task {
-  int c0t, r0t, ka, np;  // first column and row of the tile, first plane, planes streamed (kt + 2 at most)
+// The blocks share the work evenly: block i of G takes planes i W/G ..
+// (i+1) W/G of the W wet planes of all tiles, put one after another (a tile's
+// planes from its first to its last with a wet cell), as runs of one tile each,
+// which stream two planes more than they compute. cum[t]: wet planes before
+// tile t (cum[tiles] = W); first[t]: a tile's first; without them every plane
+// counts as wet. Where the dry planes are to be written too (all), the block
+// then takes its share of those: their zeros leave its sums as they are, so the
+// norm does not depend on it. 512 x 512 x 256: 186 us; tasks of equal runs
+// dealt out in turn, with dry ones skipped, took 285 (of 24 resident warps an
+// SM had 19 at work on average, and their flags took registers that now hold a
+// fourth block).
+struct R3Span {
+  const int *cum, *first;
+  long long at, end;  // planes of the block left to do
+  int tile;
+  bool dry, more;     // at the dry planes; those come next
 };
-template <int JT>
-__device__ __forceinline__ R3Task r3_task(const R3Space& sp, int T) {
-  R3Task t;
-  const int tI = T % sp.nti, rest = T / sp.nti;
-  const int tJ = rest % sp.ntj, kc = rest / sp.ntj;
-  t.c0t = sp.c0 + R3Cfg<JT>::TI * tI;
-  t.r0t = sp.r0 + R3Cfg<JT>::TJ * tJ;
-  t.ka = sp.p0 + kc * sp.kt;
-  const int kb = min(t.ka + sp.kt, sp.p0 + sp.nk);
-  t.np = kb - t.ka + 2;  // planes ka-1 .. kb
+template <bool ALL>
+__device__ __forceinline__ long long r3_cum(const R3Span& w, const R3Space& sp, int t) {
+  const long long all = (long long)t * sp.nk;
+  return !ALL || w.cum ? (ALL && w.dry ? all - w.cum[t] : w.cum[t]) : all;
+}
+template <bool ALL>
+__device__ __forceinline__ void r3_begin(R3Span& w, const R3Space& sp, bool dry) {
+  w.dry = dry;
+  const int nt = sp.nti * sp.ntj;
+  const long long W = r3_cum<ALL>(w, sp, nt);
+  w.at = W * blockIdx.x / gridDim.x;
+  w.end = W * (blockIdx.x + 1) / gridDim.x;
+  int lo = 0, hi = nt;  // the last tile with cum <= at
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (r3_cum<ALL>(w, sp, mid) <= w.at) lo = mid;
+    else hi = mid;
+  }
+  w.tile = lo;
+}
+struct R3Task {
+  int c0t, r0t, ka, np;  // first column and row of the tile, first plane, planes streamed (2 more than computed)
+};
+// the block's next run; np = 0 after the last
+template <int JT, bool ALL>
+__device__ __forceinline__ R3Task r3_next(R3Span& w, const R3Space& sp) {
+  R3Task t = {0, 0, 0, 0};
+  if (w.at >= w.end) {
+    if (!ALL || !w.more) return t;
+    w.more = false;
+    r3_begin<ALL>(w, sp, true);
+    if (w.at >= w.end) return t;
+  }
+  long long c0 = r3_cum<ALL>(w, sp, w.tile), c1 = r3_cum<ALL>(w, sp, w.tile + 1);
+  while (c1 <= w.at) {  // tiles without such a plane
+    ++w.tile;
+    c0 = c1;
+    c1 = r3_cum<ALL>(w, sp, w.tile + 1);
+  }
+  int n = (int)(min(c1, w.end) - w.at), o = (int)(w.at - c0);
+  if (!ALL || w.cum) {
+    const int f = w.first[w.tile];
+    if (!ALL || !w.dry) o += f;
+    else if (o < f) n = min(n, f - o);  // below the wet planes, then above them
+    else o += w.cum[w.tile + 1] - w.cum[w.tile];
+  }
+  t.c0t = sp.c0 + R3Cfg<JT>::TI * (w.tile % sp.nti);
+  t.r0t = sp.r0 + R3Cfg<JT>::TJ * (w.tile / sp.nti);
+  t.ka = sp.p0 + o;
+  t.np = n + 2;
+  w.at += n;
   return t;
 }
 
-// tcol (optional, JT = 2 tiles): 1 for each (tile, interior plane) with a wet
-// cell. A task whose output planes are all dry is skipped: its cells' b32 is
-// +0 already and their residuals add exact zeros to the sums. The block's
-// tasks' flags are gathered in shared memory first (up to kR3MaxTasks per
-// block; later ones count as wet), and the issue cursor and the consumers
-// skip the same tasks.
-constexpr int kR3MaxTasks = 64;
-template <int JT, bool NEUMANN>
-__global__ void __launch_bounds__(kMxThreads) k_resid_int3d(const __grid_constant__ CUtensorMap mx,
+template <int JT, bool NEUMANN, bool ALL>
+__global__ void __launch_bounds__(kMxThreads, ALL ? 1 : 4) k_resid_int3d(const __grid_constant__ CUtensorMap mx,
                                                             const __grid_constant__ CUtensorMap mb,
                                                             const __grid_constant__ CUtensorMap md, R3Space sp,
                                                             double* ds, float* __restrict__ b32,
                                                             float* __restrict__ r32, double* __restrict__ partials,
-                                                            const uint8_t* __restrict__ tcol) {
+                                                            const int* __restrict__ cum,
+                                                            const int* __restrict__ first) {
   typedef R3Cfg<JT> G;
   extern __shared__ __align__(128) unsigned char smem[];
   long long* pring = reinterpret_cast<long long*>(smem + G::Stages * G::StageBytes);
@@ -158,34 +206,15 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int3d(const __grid_constan
   const int k = fix_exponent(ds);
   const double scale = ds[S_NEXT];
   const float fm = (float)ldexp(scale, -(k + q));  // power of two: R -> r * scale
-  const int ntasks = sp.nti * sp.ntj * sp.nkc;
-  // wet flags of the block's tasks (bit m: task blockIdx.x + m * gridDim.x),
-  // the same in every thread
-  unsigned long long wt = ~0ULL;
-  if (tcol) {
-    wt = 0;
-    for (int m = 0; m < kR3MaxTasks; ++m) {
-      const int T = blockIdx.x + m * gridDim.x;
-      if (T >= ntasks) break;
-      const R3Task t = r3_task<JT>(sp, T);
-      const long long tile = (long long)((t.r0t - sp.r0) / R3Cfg<JT>::TJ) * sp.nti + (t.c0t - sp.c0) / R3Cfg<JT>::TI;
-      int any = 0;
-      for (int p = tid; p < t.np - 2; p += kMxThreads) any |= tcol[tile * sp.nk + (t.ka - sp.p0) + p];
-      if (__syncthreads_or(any)) wt |= 1ULL << m;
-    }
-  }
-  auto wet = [&](int T) {  // tasks beyond kR3MaxTasks count as wet
-    const int m = (T - (int)blockIdx.x) / (int)gridDim.x;
-    return m >= kR3MaxTasks || ((wt >> m) & 1ULL);
-  };
-
-  // issue cursor (thread 0): the block's sequence of (task, plane) in order
-  int iT = blockIdx.x, iq = 0;
-  while (iT < ntasks && !wet(iT)) iT += gridDim.x;
+  // issue cursor (thread 0): the block's sequence of (run, plane) in order
+  R3Span span = {cum, first, 0, 0, 0, false, ALL && cum};
+  r3_begin<ALL>(span, sp, false);
+  R3Span is = span;
+  R3Task it = r3_next<JT, ALL>(is, sp);
+  int iq = 0;
   unsigned long long in = 0;
-  R3Task it = r3_task<JT>(sp, iT < ntasks ? iT : 0);
   auto issue_next = [&]() {
-    if (iT >= ntasks) return;
+    if (it.np == 0) return;
     const int s = (int)(in % G::Stages);
     const unsigned bar = smem_u32(bars + s);
     unsigned char* st = smem + s * G::StageBytes;
@@ -200,10 +229,8 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int3d(const __grid_constan
     }
     ++in;
     if (++iq == it.np) {
-      iT += gridDim.x;
-      while (iT < ntasks && !wet(iT)) iT += gridDim.x;
       iq = 0;
-      if (iT < ntasks) it = r3_task<JT>(sp, iT);
+      it = r3_next<JT, ALL>(is, sp);
     }
   };
   if (tid == 0)
@@ -231,9 +258,8 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int3d(const __grid_constan
   __int128 s1 = 0;
   unsigned long long n = 0;  // planes consumed
   bool fault = false;
-  for (int T = blockIdx.x; T < ntasks && !fault; T += gridDim.x) {
-    if (!wet(T)) continue;
-    const R3Task t = r3_task<JT>(sp, T);
+  R3Span cs = span;
+  for (R3Task t = r3_next<JT, ALL>(cs, sp); t.np != 0 && !fault; t = r3_next<JT, ALL>(cs, sp)) {
     const int ox = (t.c0t - 1) - ((t.c0t - 1) & ~1), ob = t.c0t - (t.c0t & ~1), od = t.c0t - (t.c0t & ~15);
     const int col = t.c0t + ti;
     bool own[JT];
@@ -314,57 +340,68 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int3d(const __grid_constan
         if (!mbar_wait(smem_u32(bars + (m % G::Stages)), (unsigned)((m / G::Stages) & 1))) break;
       ds[S_FAULT] = 1.0;
       partials[blockIdx.x] = __longlong_as_double(0x7ff8000000000000LL);
-      partials[kMxParts + blockIdx.x] = __longlong_as_double(0x7ff8000000000000LL);
-      for (int i = gridDim.x + blockIdx.x; i < kMxParts; i += gridDim.x) partials[i] = partials[kMxParts + i] = 0.0;
+      partials[kMxParts + blockIdx.x] = partials[2 * kMxParts + blockIdx.x] = 0.0;
+      for (int i = gridDim.x + blockIdx.x; i < kMxParts; i += gridDim.x)
+        partials[i] = partials[kMxParts + i] = partials[2 * kMxParts + i] = 0.0;
     }
     return;
   }
   // sum f^2 -> sum r^2 = sum f^2 / scale^2 (exact power of two)
-  const double s2d = ((double)hi + (double)lo) / (scale * scale);
-  const double s1d = NEUMANN ? ldexp(__dadd_rn(__dmul_rn((double)(long long)(s1 >> 64), 18446744073709551616.0),
-                                               (double)(unsigned long long)s1),
-                                     -(k + q))
-                             : 0.0;
-  __shared__ double sh2[kMxThreads / 32], sh1[kMxThreads / 32];
-  double a2 = s2d, a1 = s1d;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a2 += __shfl_down_sync(0xffffffffu, a2, o);
-    a1 += __shfl_down_sync(0xffffffffu, a1, o);
-  }
-  if (ti == 0) {
-    sh2[tj] = a2;
-    sh1[tj] = a1;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    double u = 0.0, v = 0.0;
-    for (int w = 0; w < kMxThreads / 32; ++w) {
-      u += sh2[w];
-      v += sh1[w];
-    }
-    partials[blockIdx.x] = u;
-    partials[kMxParts + blockIdx.x] = v;
-    // the final pass reads kMxParts partials: the blocks clear the unused ones
-    for (int i = gridDim.x + blockIdx.x; i < kMxParts; i += gridDim.x) partials[i] = partials[kMxParts + i] = 0.0;
-  }
+  int_partials<true>(((double)hi + (double)lo) / (scale * scale), s1, 0, k + q, partials);
 }
 
-// tcol[(tJ * nti + tI) * nk + p] = 1 when tile (tI, tJ) of the JT = 2
-// tiling holds a wet cell in interior plane p
-__global__ void k_make_tcol(const uint8_t* __restrict__ m, uint8_t* __restrict__ tcol, R3Space sp) {
-  const long long T = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long ntiles = (long long)sp.nti * sp.ntj;
-  if (T >= ntiles * sp.nk) return;
-  const long long tile = T / sp.nk;
-  const int p = (int)(T - tile * sp.nk);
-  const int tI = (int)(tile % sp.nti), tJ = (int)(tile / sp.nti);
-  const int c0 = sp.c0 + R3Cfg<2>::TI * tI, r0 = sp.r0 + R3Cfg<2>::TJ * tJ;
-  const int c1 = min(c0 + R3Cfg<2>::TI, sp.c0 + sp.ni), r1 = min(r0 + R3Cfg<2>::TJ, sp.r0 + sp.nj);
-  unsigned any = 0;
-  for (int r = r0; r < r1; ++r)
-    for (int c = c0; c < c1; ++c) any |= m[(long long)c + sp.n1 * r + sp.n2 * (sp.p0 + p)];
-  tcol[T] = any ? 1 : 0;
+// a block per tile of the JT = 2 tiling: its first wet interior plane, and in
+// cum[tile + 1] the number of planes from there to its last one
+__global__ void __launch_bounds__(256) k_tile_planes(const uint8_t* __restrict__ m, int* __restrict__ cum,
+                                                     int* __restrict__ first, R3Space sp) {
+  const int tile = blockIdx.x, tI = tile % sp.nti, tJ = tile / sp.nti;
+  const int c = sp.c0 + R3Cfg<2>::TI * tI + (threadIdx.x & 31);
+  const int r0 = sp.r0 + R3Cfg<2>::TJ * tJ, r1 = min(r0 + R3Cfg<2>::TJ, sp.r0 + sp.nj);
+  __shared__ int lo, hi;
+  if (threadIdx.x == 0) {
+    lo = sp.nk;
+    hi = -1;
+  }
+  __syncthreads();
+  for (int p = threadIdx.x >> 5; p < sp.nk; p += 8) {
+    unsigned any = 0;
+    if (c < sp.c0 + sp.ni)
+      for (int r = r0; r < r1; ++r) any |= m[(long long)c + sp.n1 * r + sp.n2 * (sp.p0 + p)];
+    if (__any_sync(~0u, any != 0) && (threadIdx.x & 31) == 0) {
+      atomicMin(&lo, p);
+      atomicMax(&hi, p);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    first[tile] = hi < 0 ? 0 : lo;
+    cum[tile + 1] = hi < 0 ? 0 : hi - lo + 1;
+    if (tile == 0) cum[0] = 0;
+  }
+}
+// running sums, one block
+__global__ void __launch_bounds__(1024) k_running_sum(int* __restrict__ a, int n) {
+  __shared__ int ws[32];
+  int base = 0;
+  for (int i0 = 0; i0 < n; i0 += 1024) {
+    const int i = i0 + threadIdx.x, lane = threadIdx.x & 31;
+    int v = i < n ? a[i] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(~0u, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane == 31) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < (int)(threadIdx.x >> 5)) before += ws[w];
+      all += ws[w];
+    }
+    if (i < n) a[i] = base + before + v;
+    base += all;
+    __syncthreads();
+  }
 }
 
 R3Space r3_space(const Geom& g, const Box& bx, int ti, int tj) {
@@ -424,24 +461,27 @@ bool encode3(CUtensorMap* m, CUtensorMapDataType dt, int esize, const void* base
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int JT, bool NEUMANN>
+template <int JT, bool NEUMANN, bool ALL>
 int r3_grid() {
-  static int blocks = 0;  // one wave: resident blocks per SM x SMs, at most kMxParts
+  // one wave of the form that skips dry planes: resident blocks per SM x SMs, at
+  // most kMxParts (the form that writes them too takes the same blocks)
+  static int blocks = 0;
   if (!blocks) {
     int dev = 0, nsm = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(k_resid_int3d<JT, NEUMANN>, cudaFuncAttributeMaxDynamicSharedMemorySize, R3Cfg<JT>::Smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resid_int3d<JT, NEUMANN>, kMxThreads, R3Cfg<JT>::Smem);
+    cudaFuncSetAttribute(k_resid_int3d<JT, NEUMANN, ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, R3Cfg<JT>::Smem);
+    cudaFuncSetAttribute(k_resid_int3d<JT, NEUMANN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, R3Cfg<JT>::Smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resid_int3d<JT, NEUMANN, ALL>, kMxThreads, R3Cfg<JT>::Smem);
     blocks = nsm * (per > 0 ? per : 1);
     if (blocks > kMxParts || blocks <= 0) blocks = kMxParts;
   }
   return blocks;
 }
 
-template <int JT>
+template <int JT, bool ALL>
 bool launch_r3(const double* x, const double* b, const int8_t* dqp, const Geom& g, const Box& bx, double* ds,
-               float* b32, float* r32, bool neumann, double* partials, cudaStream_t s, const uint8_t* tcol) {
+               float* b32, float* r32, bool neumann, double* partials, cudaStream_t s, const int* tcol) {
   typedef R3Cfg<JT> G;
   R3Space sp = r3_space(g, bx, G::TI, G::TJ);
   // the boxes start at column c0t-1 >= 0, row r0t-1 >= 0 and plane ka-1 >= 0
@@ -452,17 +492,14 @@ bool launch_r3(const double* x, const double* b, const int8_t* dqp, const Geom& 
       !encode3(&mb, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, b, g.tx, g.tx, g.ty, g.tz, G::BW, G::TJ) ||
       !encode3(&md, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dqp, txp, txp, g.ty, g.tz, G::DW, G::TJ))
     return false;
-  const int grid = neumann ? r3_grid<JT, true>() : r3_grid<JT, false>();
-  // about 8 tasks per block: runs of kt planes (each streams kt + 2)
-  const long long cols = (long long)sp.nti * sp.ntj;
-  long long kt = (sp.nk * cols + 8LL * grid - 1) / (8LL * grid);
-  kt = kt < 4 ? 4 : kt;
-  sp.kt = (int)(kt > sp.nk ? sp.nk : kt);
-  sp.nkc = (sp.nk + sp.kt - 1) / sp.kt;
+  const int grid = neumann ? r3_grid<JT, true, JT == 1>() : r3_grid<JT, false, JT == 1>();
+  const int* first = tcol ? tcol + sp.nti * sp.ntj + 1 : nullptr;
   if (neumann)
-    launch_dep(k_resid_int3d<JT, true>, grid, kMxThreads, G::Smem, s, mx, mb, md, sp, ds, b32, r32, partials, tcol);
+    launch_dep(k_resid_int3d<JT, true, ALL>, grid, kMxThreads, G::Smem, s, mx, mb, md, sp, ds, b32, r32, partials, tcol,
+               first);
   else
-    launch_dep(k_resid_int3d<JT, false>, grid, kMxThreads, G::Smem, s, mx, mb, md, sp, ds, b32, r32, partials, tcol);
+    launch_dep(k_resid_int3d<JT, false, ALL>, grid, kMxThreads, G::Smem, s, mx, mb, md, sp, ds, b32, r32, partials, tcol,
+               first);
   return true;
 }
 
@@ -477,24 +514,25 @@ void launch_pad_dq(const int8_t* dq, int8_t* dqp, int tx, int txp, long long row
 
 bool launch_resid_int3d(const double* x, const double* b, const int8_t* dqp, const Geom& g, const Box& bx,
                         double* ds, float* b32, float* r32, bool neumann, double* partials, cudaStream_t s,
-                        int rows_per_thread, const uint8_t* tcol) {
+                        int rows_per_thread, const int* tcol, bool all) {
   // TMA: global addresses on 16 bytes, row and plane pitches multiples of 16 bytes
   if (!dqp || g.tx % 2 != 0 || ((uintptr_t)x | (uintptr_t)b | (uintptr_t)dqp) % 16 != 0) return false;
-  // the skipped tasks' r32 would keep older values: skip only where r32 is not written
-  if (rows_per_thread == 2) return launch_r3<2>(x, b, dqp, g, bx, ds, b32, r32, neumann, partials, s, r32 ? nullptr : tcol);
-  return launch_r3<1>(x, b, dqp, g, bx, ds, b32, r32, neumann, partials, s, nullptr);
+  if (rows_per_thread != 2) return launch_r3<1, true>(x, b, dqp, g, bx, ds, b32, r32, neumann, partials, s, nullptr);
+  return all || !tcol ? launch_r3<2, true>(x, b, dqp, g, bx, ds, b32, r32, neumann, partials, s, tcol)
+                      : launch_r3<2, false>(x, b, dqp, g, bx, ds, b32, r32, neumann, partials, s, tcol);
 }
 
 long long resid3d_tcol_size(const Geom& g, const Box& bx) {
   const R3Space sp = r3_space(g, bx, R3Cfg<2>::TI, R3Cfg<2>::TJ);
-  return (long long)sp.nti * sp.ntj * sp.nk;
+  return sp.ni > 0 && sp.nj > 0 && sp.nk > 0 ? 2LL * sp.nti * sp.ntj + 1 : 0;
 }
 
-void launch_make_tcol(const uint8_t* m, uint8_t* tcol, const Geom& g, const Box& bx, cudaStream_t s) {
+void launch_make_tcol(const uint8_t* m, int* tcol, const Geom& g, const Box& bx, cudaStream_t s) {
   const R3Space sp = r3_space(g, bx, R3Cfg<2>::TI, R3Cfg<2>::TJ);
-  const long long n = (long long)sp.nti * sp.ntj * sp.nk;
-  if (n <= 0) return;
-  k_make_tcol<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(m, tcol, sp);
+  const int nt = sp.nti * sp.ntj;
+  if (resid3d_tcol_size(g, bx) == 0) return;
+  k_tile_planes<<<nt, 256, 0, s>>>(m, tcol, tcol + nt + 1, sp);
+  k_running_sum<<<1, 1024, 0, s>>>(tcol + 1, nt);
 }
 
 }  // namespace cfmg

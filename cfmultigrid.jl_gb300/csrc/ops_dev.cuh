@@ -569,25 +569,88 @@ __device__ __forceinline__ bool zero_prolong(const double* xf, const double* x, 
 
 // ------------------------------------------------------- fixed point
 // Integer form of the mixed loop's level-1 residual (k_mixed.cu, k_batch.cu).
+// N bytes to shared memory behind the thread's back (cp.async)
+template <int N>
+__device__ __forceinline__ void cp_async(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "n"(N)
+               : "memory");
+}
+
 // round(v * 2^k) for |v| 2^k < 2^59, ties away from zero; zero and
 // subnormal v give 0. Branch-free: with M = m << 10 (m the 53-bit
-// significand, v = m 2^(ex-1075)), round(m 2^sh) = ((M >> (t-1)) + 1) >> 1
-// for t = 10 - sh: the range bound keeps sh <= 5, so t >= 5, and t is
-// capped at 64, where the result is 0 as for any shift past the significand.
+// significand, v = m 2^(ex-1075)) and y = M >> n for n = 1084 - ex - k, the
+// magnitude is (y + 1) >> 1 and its negative (-y) >> 1 = (~y + 1) >> 1, so one
+// exclusive or serves the sign. The range bound keeps n >= 4; n is capped at
+// 63, where y = 0 as for any shift past the significand, and as for ex = 0
+// with k <= 1021 (fix_k).
 __device__ __forceinline__ long long to_fix(double v, int k) {
-  const long long u = __double_as_longlong(v);
-  const int ex = (int)(((unsigned long long)u >> 52) & 0x7ffULL);
-  const unsigned long long M = (((unsigned long long)u & 0x000FFFFFFFFFFFFFULL) | 0x0010000000000000ULL) << 10;
-  const int t = min(max(1085 - ex - k, 1), 64);
-  const long long r = ex ? (long long)(((M >> (t - 1)) + 1ULL) >> 1) : 0LL;
-  return u < 0 ? -r : r;
+  const int hi = __double2hiint(v);
+  const unsigned lo = (unsigned)__double2loint(v);
+  const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+  const int n = min(max(1084 - k - (int)(((unsigned)hi << 1) >> 21), 0), 63);
+  const unsigned long long M = ((unsigned long long)__funnelshift_l(lo, mh, 10) << 32) | (lo << 10);
+  return (((long long)(M >> n) ^ (long long)(hi >> 31)) + 1LL) >> 1;
 }
-// k = 58 - E for max(|x|, |b|) < 2^E (device scalars S_MAXX, S_MAXB)
+// 58 - E for values below 2^E
+__device__ __forceinline__ int fix_k(int E) { return 58 - max(E, -963); }
+// k for max(|x|, |b|) (device scalars S_MAXX, S_MAXB)
 __device__ __forceinline__ int fix_exponent(const double* ds) {
   const double mx = fmax(ds[S_MAXX], ds[S_MAXB]);
   int e = 0;
   if (mx > 0 && isfinite(mx)) frexp(mx, &e);  // mx < 2^e
-  return 58 - e;
+  return fix_k(e);
+}
+
+__device__ __forceinline__ double int_to_double(__int128 v) {
+  return __dadd_rn(__dmul_rn((double)(long long)(v >> 64), 18446744073709551616.0), (double)(unsigned long long)v);
+}
+// The end of the fixed-point residual passes, for blocks of kMxThreads: the
+// block's sum r^2 (s2 of each thread, times 2^e2) into partials[blk] and its
+// sum r (s1 of each thread, exact, in units of 2^-e1) into partials[kMxParts +
+// blk], both combined in FP64. EXACT (the 7-point passes): sum r stays an
+// integer, its low word there and its high word in partials[2 kMxParts + blk],
+// so that the split of the cells over threads does not show in the wet mean,
+// which is rounding noise of a sum that cancels. Unused ones are cleared for
+// the final pass.
+template <bool EXACT>
+__device__ __forceinline__ void int_partials(double s2, __int128 s1, int e2, int e1, double* __restrict__ partials) {
+  __shared__ double sh2[kMxThreads / 32], sd[EXACT ? 1 : kMxThreads / 32];
+  __shared__ __int128 si[EXACT ? kMxThreads / 32 : 1];
+  double d1 = EXACT ? 0.0 : ldexp(int_to_double(s1), -e1);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s2 += __shfl_down_sync(0xffffffffu, s2, o);
+    if (EXACT) {
+      const unsigned long long l = __shfl_down_sync(0xffffffffu, (unsigned long long)s1, o);
+      const long long h = __shfl_down_sync(0xffffffffu, (long long)(s1 >> 64), o);
+      s1 += (__int128)(((unsigned __int128)(unsigned long long)h << 64) | l);
+    } else {
+      d1 += __shfl_down_sync(0xffffffffu, d1, o);
+    }
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sh2[threadIdx.x >> 5] = s2;
+    if (EXACT) si[threadIdx.x >> 5] = s1;
+    else sd[threadIdx.x >> 5] = d1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double u = 0.0, v = 0.0;
+    __int128 vi = 0;
+    for (int w = 0; w < kMxThreads / 32; ++w) {
+      u += sh2[w];
+      if (EXACT) vi += si[w];
+      else v += sd[w];
+    }
+    partials[blockIdx.x] = ldexp(u, e2);
+    partials[kMxParts + blockIdx.x] = EXACT ? __longlong_as_double((long long)vi) : v;
+    if (EXACT) partials[2 * kMxParts + blockIdx.x] = __longlong_as_double((long long)(vi >> 64));
+    for (int i = gridDim.x + blockIdx.x; i < kMxParts; i += gridDim.x) {
+      partials[i] = partials[kMxParts + i] = 0.0;
+      if (EXACT) partials[2 * kMxParts + i] = 0.0;
+    }
+  }
 }
 
 // e * 2^p as a double, exactly, with integer operations on the bits of the
