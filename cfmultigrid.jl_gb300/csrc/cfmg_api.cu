@@ -932,6 +932,9 @@ int smooth_tb(cfmg_handle* h, int lev, int nite) {
   return CFMG_OK;
 }
 
+bool smooth_steps_ok(const cfmg_handle* h, int lev, int nite);
+int smooth_steps(cfmg_handle* h, int lev, int nite);
+
 // mg.smoother[lev] (src/gmg_setup.jl:124-139 selects among these)
 // A long smoothing call (the coarsest solve) on a level whose four arrays fit
 // one block's shared memory runs as one block (k_small_smooth) instead of
@@ -978,6 +981,7 @@ int small_smooth_run(cfmg_handle* h, int lev, int nite) {
 template <class T>
 int smooth_t(cfmg_handle* h, int lev, int nite) {
   if (tb_eligible<T>(h, lev)) return smooth_tb(h, lev, nite);
+  if (sizeof(T) == 8 && smooth_steps_ok(h, lev, nite)) return smooth_steps(h, lev, nite);
   if (small_smooth_ok<T>(h, lev, nite)) return small_smooth_run<T>(h, lev, nite);
   const Level& l = h->lv[lev - 1];
   View<T> v = view<T>(l);
@@ -1291,6 +1295,42 @@ int step2d(cfmg_handle* h, int lev, int mode, int np) {
   {
     Launch k(h, mode == 2 ? CFMG_K_SWEEP : CFMG_K_DESCENT, lev, prec_of<T>());
     launch_step2d(a, tail_stencil(h), mode, vertices(h), h->stream);
+  }
+  LAUNCH_OK(h);
+  return CFMG_OK;
+}
+
+// A long FP64 smoothing of the last level (the coarsest solve) where that level
+// is too large for the tail: passes of up to kSmoothPairs pairs of sweeps each,
+// from x to the scratch array and back, instead of a launch a sweep (the 2048^2
+// F-cycle of five levels, 50 pairs on 134^2: about 2.27 ms a cycle with a launch a
+// sweep, 2.07 with 3 pairs a pass; solves against a launch a sweep 1.03, 1.05
+// and 1.09 times as fast with 1, 2 and 3 pairs, level with 4 or 5).
+constexpr int kSmoothPairs = 3;
+bool smooth_steps_ok(const cfmg_handle* h, int lev, int nite) {
+  if (h->record || nite < 4 || lev != L(h) || lev < 2 || !steps_form(h)) return false;
+  const Level& l = h->lv[lev - 1];
+  return (long long)l.len * (h->d.op == CFMG_LAPLACIAN ? 7 : 11) <= kStepWork && l.s64 &&
+         !in_engine(h, lev, CFMG_FP64) && steps_clean(h);
+}
+int smooth_steps(cfmg_handle* h, int lev, int nite) {
+  const Level& l = h->lv[lev - 1];
+  const View<double> v = view<double>(l);
+  TRY(flush(h));
+  TbgArgs<double> a;
+  std::memset(&a, 0, sizeof(a));
+  a.b = v.b; a.w = v.widiag; a.cE = v.cE; a.cN = v.cN;
+  a.cff = 1.0 - h->d.omega;
+  a.tx = l.tx; a.ty = l.ty; a.nh = l.nh;
+  const int passes = 2 * ((nite + 2 * kSmoothPairs - 1) / (2 * kSmoothPairs));  // even: the last one writes x
+  for (int k = 0; k < passes; ++k) {
+    a.np = nite * (k + 1) / passes - nite * k / passes;
+    a.xs = k % 2 ? l.s64 : v.x;
+    a.s = k % 2 ? nullptr : l.s64;
+    a.x = k % 2 ? v.x : nullptr;
+    a.y = k == passes - 1 ? v.y : nullptr;
+    Launch c(h, CFMG_K_SWEEP, lev, CFMG_FP64);
+    launch_step2d(a, tail_stencil(h), 3, vertices(h), h->stream);
   }
   LAUNCH_OK(h);
   return CFMG_OK;

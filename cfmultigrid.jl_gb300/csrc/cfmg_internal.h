@@ -337,7 +337,8 @@ struct TbgArgs {
   int np, tx, ty, nh, ctx, cty, np_i, np_j;  // np: pairs of sweeps; np_i x np_j prolongation parents
 };
 // stencil TAIL_5 / TAIL_9 / TAIL_VC; mode 0: descent from x = +0 (or xs), 1:
-// descent from x = +0 (or xs) + Pcoef P(coarse x), 2: ascent
+// descent from x = +0 (or xs) + Pcoef P(coarse x), 2: ascent, 3 (FP64): pairs of
+// sweeps from xs into one of x and s
 void launch_step2d(const TbgArgs<double>& a, int stencil, int mode, bool vertices, cudaStream_t s);
 void launch_step2d(const TbgArgs<float>& a, int stencil, int mode, bool vertices, cudaStream_t s);  // TAIL_VC
 

@@ -94,7 +94,8 @@ __device__ __forceinline__ bool g_land(const double* x, int L, int S, double b, 
   return z.zero() && (__double_as_longlong(x[L]) | __double_as_longlong(w)) == 0ll;
 }
 
-// MODE 0: descent from x = +0; 1: descent from x = Pcoef P(xc); 2: ascent.
+// MODE 0: descent from x = +0; 1: descent from x = Pcoef P(xc); 2: ascent; 3:
+// np pairs of sweeps from xs into x or s, the other null.
 // KIND 0: cell centres, 2: vertices (restriction and prolongation).
 template <class T, int ST, int MODE, int KIND>
 __global__ void __launch_bounds__(g_threads<T>()) k_step2d(TbgArgs<T> a, int S, int core) {
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(g_threads<T>()) k_step2d(TbgArgs<T> a, int S, 
       E[t] = in ? a.cE[I] : T(0);
       N[t] = in ? a.cN[I] : T(0);
     }
-    if (MODE != 0) {
+    if (MODE == 1 || MODE == 2) {
       // parents (p, q) update their children; the others keep x
       const int p = gi - nh - 1, q = gj - nh - 1;
       const bool fam = p >= 0 && p < 2 * a.np_i && q >= 0 && q < 2 * a.np_j;
@@ -179,9 +180,9 @@ __global__ void __launch_bounds__(g_threads<T>()) k_step2d(TbgArgs<T> a, int S, 
     const bool r2 = ST == TAIL_9 ? gi > nh && gi <= tx - nh && gj > nh && gj <= ty - nh : r1;
     if (r1 && a.y) a.y[I] = Y[L];
     if (r2 && a.x) a.x[I] = X[L];
-    if (MODE != 2 && (r2 || a.xs)) a.s[I] = X[L];  // level 1's x out of range counts too
+    if (MODE != 2 && a.s && (r2 || a.xs)) a.s[I] = X[L];  // level 1's x out of range counts too
   }
-  if (MODE == 2) return;
+  if (MODE >= 2) return;
   __syncthreads();
   // residual of the smoothed x into Y, one cell beyond the core
   const int m = H - 1, nr = core + 2;
@@ -244,7 +245,8 @@ __global__ void __launch_bounds__(g_threads<T>()) k_step2d(TbgArgs<T> a, int S, 
 }
 
 // the core side with the least work (FP64 instructions, or cells) for the busiest of 152 SMs
-int tbg_tile(int max_tile, int tx, int ty, int np, bool descent) {
+int tbg_tile(int max_tile, int tx, int ty, int np, int mode) {
+  const bool descent = mode < 2;
   const int H = 2 * np + (descent ? 2 : 0);
   int best = 4;
   double cost = 0.0;
@@ -254,7 +256,7 @@ int tbg_tile(int max_tile, int tx, int ty, int np, bool descent) {
     double w = 200.0 + 0.3 * S * S;  // loads and barriers, in cells of a sweep
     for (int s = 0; s < 2 * np; ++s) w += (S - 2 * (s + 1)) * (S - 2 * (s + 1));
     if (descent) w += 1.2 * (core + 2) * (core + 2);
-    else w += S * S;
+    else if (mode == 2) w += S * S;
     w *= (double)((tiles + 151) / 152);
     if (cost == 0.0 || w < cost) {
       cost = w;
@@ -267,7 +269,7 @@ int tbg_tile(int max_tile, int tx, int ty, int np, bool descent) {
 template <class T, int ST, int MODE, int KIND>
 void launch_step(const TbgArgs<T>& a, cudaStream_t s) {
   constexpr int mt = g_max_tile<T>();
-  const int core = tbg_tile(mt, a.tx, a.ty, a.np, MODE != 2), S = core + 2 * (2 * a.np + (MODE != 2 ? 2 : 0));
+  const int core = tbg_tile(mt, a.tx, a.ty, a.np, MODE), S = core + 2 * (2 * a.np + (MODE < 2 ? 2 : 0));
   const size_t smem = (size_t)(ST == TAIL_VC ? 6 : 4) * S * S * sizeof(T);
   static const cudaError_t attr = cudaFuncSetAttribute(
       k_step2d<T, ST, MODE, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * mt * mt * (int)sizeof(T));
@@ -279,7 +281,8 @@ template <class T, int ST, int KIND>
 void launch_step_m(const TbgArgs<T>& a, int mode, cudaStream_t s) {
   if (mode == 0) launch_step<T, ST, 0, KIND>(a, s);
   else if (mode == 1) launch_step<T, ST, 1, KIND>(a, s);
-  else launch_step<T, ST, 2, KIND>(a, s);
+  else if (mode == 2) launch_step<T, ST, 2, KIND>(a, s);
+  else if constexpr (sizeof(T) == 8) launch_step<T, ST, 3, KIND>(a, s);
 }
 
 }  // namespace

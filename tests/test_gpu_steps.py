@@ -114,3 +114,14 @@ def test_mixed_varcoef_steps_are_bit_identical(cycle, size, pairs):
         mg.close()
     assert np.array_equal(out[0][0], out[1][0])
     assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("name,cycle,size,nlevels", [("5", "v", (300, 212), 2), ("5-vertices", "f", (520, 390), 3),
+                                                     ("9-vertices", "f", (512, 512), 3), ("9", "v", (470, 330), 3),
+                                                     ("varcoef", "v", (333, 270), 2)])
+def test_long_smoothing_of_the_last_level(name, cycle, size, nlevels):
+    """A hierarchy that ends above the tail's sizes smooths its last level in passes of several pairs."""
+    p = dict(cycle=cycle, npre=2, npost=2, omega=0.8, nlevels=nlevels, **OPS[name])
+    a, b = (_run(fused, *size, 3, **p) for fused in (1, 0))
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
