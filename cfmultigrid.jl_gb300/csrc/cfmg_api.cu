@@ -3044,18 +3044,22 @@ int lockstep_build(cfmg_batch* b) {
     std::vector<long long> nc(ops.size());
     long long mx = 0;
     const int o0 = (int)all.size();
+    long long items = 0;
+    for (const Op& o : ops) items += o.n;
+    int chunk = kBStageChunk;
+    while (chunk > kBStageMin && items < (long long)chunk * 152 * kBStageBlocks * kBStageFill) chunk /= 2;
     for (size_t j = 0; j < ops.size(); ++j) {
       all.push_back(ops[j]);
-      nc[j] = tb ? ops[j].n : (ops[j].n + kBStageChunk - 1) / kBStageChunk;
+      nc[j] = tb ? ops[j].n : (ops[j].n + chunk - 1) / chunk;
       mx = std::max(mx, nc[j]);
     }
     if (b->interleave) {  // chunk c of every Op, then chunk c + 1, ...
       for (long long c = 0; c < mx; ++c)
         for (size_t j = 0; j < ops.size(); ++j)
-          if (c < nc[j]) tab.push_back(make_int4(o0 + (int)j, (int)c, ops[j].inst, 0));
+          if (c < nc[j]) tab.push_back(make_int4(o0 + (int)j, (int)c, ops[j].inst, chunk));
     } else {
       for (size_t j = 0; j < ops.size(); ++j)
-        for (long long c = 0; c < nc[j]; ++c) tab.push_back(make_int4(o0 + (int)j, (int)c, ops[j].inst, 0));
+        for (long long c = 0; c < nc[j]; ++c) tab.push_back(make_int4(o0 + (int)j, (int)c, ops[j].inst, chunk));
     }
     st.nchunks = (long long)tab.size() - st.tab0;
     b->steps.push_back(st);

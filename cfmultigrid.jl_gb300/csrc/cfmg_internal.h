@@ -398,7 +398,12 @@ bool launch_smooth_tb_upd(int stencil, int nite, const float* x, const float* b,
 // Ops; a chunk of an instance that has converged is skipped.
 constexpr int kBChunk = 1024;
 constexpr int kBThreads = 256;
-constexpr int kBStageChunk = 8192;  // items of one entry of a generic step's table (k_bstage)
+// Generic batched steps (k_bstage): items of a table entry, halved for a step
+// until it has kBStageFill entries for every resident block, and resident
+// blocks an SM (their loads in flight are what bounds them: a batch of 128
+// took 24.8 ms with 8192 items and 2 blocks, 23.3 with smaller entries, 21.9
+// with 4 blocks, 21.65 with 6, 21.7 with 8)
+constexpr int kBStageChunk = 8192, kBStageMin = 512, kBStageFill = 2, kBStageBlocks = 6;
 // per-instance scalar block (double): see k_bfinal for their use
 enum BSlot { BS_NORMB = 0, BS_RES, BS_NITE, BS_NWET, BS_NEXT, BS_CUR, BS_ICUR, BS_MEAN, BS_T0, BS_T1, BS_ZEROX,
              BS_MAXX, BS_MAXB, BS_SHIFT, BS_HIST };

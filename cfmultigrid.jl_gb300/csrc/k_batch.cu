@@ -72,11 +72,11 @@ __device__ __forceinline__ double bsum(double v, double* sh) {
 }
 
 // ------------------------------------------------------------ cycle steps
-// Generic step: the active chunks (kBStageChunk items) of a list of Ops
-// (tab[c] = {op, chunk of the op, instance}), each executed with the
+// Generic step: the active chunks of a list of Ops (tab[c] = {op, chunk of the
+// op, instance, items of a chunk}), each executed with the
 // per-item code of the program engine, 4 (FP32) or 2 (FP64) items per
 // thread in flight.
-__global__ void __launch_bounds__(kBThreads, 2) k_bstage(const Op* __restrict__ ops, const int4* __restrict__ tab,
+__global__ void __launch_bounds__(kBThreads, kBStageBlocks) k_bstage(const Op* __restrict__ ops, const int4* __restrict__ tab,
                                                          long long nchunks, int win, const int* __restrict__ active) {
   dep_wait();
   __shared__ Op op;
@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(kBThreads, 2) k_bstage(const Op* __restrict__ 
         __syncthreads();
         cur = en.x;
       }
-      const long long t0 = (long long)en.y * kBStageChunk;
-      const long long e = t0 + kBStageChunk < op.n ? t0 + kBStageChunk : op.n;
+      const long long t0 = (long long)en.y * en.w;
+      const long long e = t0 + en.w < op.n ? t0 + en.w : op.n;
       if (op.prec == 0) exec<double, 2>(op, t0 + threadIdx.x, kBThreads, e);
       else exec<float, 4>(op, t0 + threadIdx.x, kBThreads, e);
     }
@@ -700,7 +700,7 @@ static long long grid_for(long long nchunks, int per_sm, int* win) {
 void launch_bstage(const Op* ops, const int4* tab, long long nchunks, const int* active, cudaStream_t s) {
   if (nchunks <= 0) return;
   int win;
-  const unsigned g = (unsigned)grid_for(nchunks, 2, &win);
+  const unsigned g = (unsigned)grid_for(nchunks, kBStageBlocks, &win);
   launch_dep(k_bstage, g, kBThreads, 0, s, ops, tab, nchunks, win, active);
 }
 
