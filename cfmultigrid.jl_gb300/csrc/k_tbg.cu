@@ -11,6 +11,8 @@
 //            np pairs of sweeps; residual; restriction into the coarse b, the
 //            coarse x zeroed
 //   ascent:  x = x + Pcoef P(coarse x), np pairs of sweeps
+//   smoothing: np pairs of sweeps from x into the scratch, or back (a long
+//            smoothing of the last level, pass after pass)
 // Each sweep covers the tile's cells that later ones need: sweep s leaves a
 // margin of s + 1 cells. The tiles overlap, so a step must not read what it
 // writes: a descent reads no x at all, and leaves a copy of its result in the
