@@ -115,10 +115,14 @@ extern "C" {
 #define CFMG_OPT_HOST_LOOP 4 /* cfmg_solve: 0 (default) runs the whole loop as one graph launch (a
                                 `while` node); 1 launches one graph per iteration from the host, which
                                 profilers that do not descend into conditional nodes can see */
-#define CFMG_OPT_FUSED_DESCENT 5 /* mixed form, 2D closed topology, lean packed passes: 1 (default)
-                                    the last pre-smoothing pass of a cycle's descent step also forms
-                                    the residual, restricts it to the coarse b and zeroes the coarse x;
-                                    0 separate kernels. Both give the same bits. */
+#define CFMG_OPT_FUSED_DESCENT 5 /* 2D closed topology: 1 (default) a cycle's steps on a level take fewer
+                                    launches. Mixed form, lean packed passes: the last pre-smoothing pass
+                                    also forms the residual, restricts it to the coarse b and zeroes the
+                                    coarse x. FP64 levels between the coarse tail and 150 000 cells, and
+                                    FP32 levels of the variable-coefficient operator, with omega <= 1: one
+                                    launch for the descent, one for the ascent, and few for a long
+                                    smoothing of the last FP64 level. 0 separate kernels. Both give the
+                                    same bits. */
 #define CFMG_OPT_FUSED_UPDATE 6 /* mixed form, 2D closed topology, integer residual, lean packed passes:
                                    1 (default) the cycle's last level-1 post-smoothing pass also applies
                                    the FP64 solution update x += e * iscale (and collects max |x|)
@@ -139,7 +143,8 @@ extern "C" {
                                      shared memory; 0 never (separate sweeps). The same bits. With a
                                      value > 0 every operator of a cycle below the level whose arrays fit
                                      one block's shared memory (all operators and topologies; FP64 levels
-                                     up to 6/5 of their engine threshold) runs in one launch there; with 0
+                                     up to 6/5 of their engine threshold, or 12/25 of it where
+                                     CFMG_OPT_FUSED_DESCENT serves the larger ones) runs in one launch there; with 0
                                      they are Ops of the cluster engine. Same values either way. */
 #define CFMG_OPT_SKIP_DRY 10 /* mixed form, closed topology: 1 (default) passes skip groups of cells
                                that are all dry (their FP32 fields hold +0 and stay +0): the FP32
