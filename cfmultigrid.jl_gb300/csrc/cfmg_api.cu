@@ -1450,8 +1450,21 @@ int norm_dev(cfmg_handle* h, int lev, const double* x, const double* normb, int 
   return CFMG_OK;
 }
 
+int resid_kind(const cfmg_handle* h);
 // residual at level 1 followed by its norm ratio into dscal[S_RES]
 int normresidual_dev(cfmg_handle* h, int kind) {
+  const Level& l = h->lv[0];
+  if ((long long)l.len <= kResidNormMax && !xperio(h) && !h->record && !in_engine(h, 1, CFMG_FP64)) {
+    TRY(flush(h));
+    {
+      Launch k(h, CFMG_K_RESIDUAL, 1, CFMG_FP64);
+      launch_resid_norm(h->d.op == CFMG_VARCOEF ? OPK_RESIDVC : resid_kind(h), l.r, l.x, l.b, l.diag, l.cE, l.cN,
+                        l.msk, geom(l), interior(l), h->partials, norm_counter(h), h->dscal + S_NORM,
+                        h->dscal + S_NORMB, kind, h->stream, h->loop);
+    }
+    LAUNCH_OK(h);
+    return CFMG_OK;
+  }
   TRY(residual_t<double>(h, 1));
   return norm_dev(h, 1, h->lv[0].r, h->dscal + S_NORMB, kind);
 }

@@ -193,6 +193,12 @@ void launch_norm(const T* x, const uint8_t* msk, size_t n, double* partials, uns
 // before the loop: hist[0] and the test of the first residual (ds[S_RES])
 void launch_loop_start(const LoopTest& lt, cudaStream_t s);
 constexpr int kNormParts = 1024;
+// residual (kind) and its norm in one launch, for levels of at most kResidNormMax cells
+constexpr long long kResidNormMax = kNormParts * 256LL;
+void launch_resid_norm(int kind, double* r, const double* x, const double* b, const double* d, const double* cE,
+                       const double* cN, const uint8_t* m, const Geom& g, const Box& bx, double* partials,
+                       unsigned* counter, double* out, const double* normb, int norm_kind, cudaStream_t s,
+                       const LoopTest* lt);
 // the handle's partial-sum scratch: two sums per block for the fused
 // residual pass of the mixed loop (k_mixed.cu), one for the norms
 constexpr int kPartials = 3 * kNormParts;

@@ -576,30 +576,9 @@ __global__ void __launch_bounds__(kThreads) k_fill_xperio(T* __restrict__ x, int
 static __device__ __noinline__ double weighted_square(uint8_t mm, double v, double s) {
   return __dadd_rn(s, __dmul_rn((double)mm, __dmul_rn(v, v)));
 }
-template <class T>
-__global__ void __launch_bounds__(kThreads) k_norm(const T* __restrict__ x, const uint8_t* __restrict__ m, long long n,
-                                                   double* __restrict__ partials, unsigned* counter, double* out,
-                                                   const double* normb, int norm_kind, LoopTest lt) {
-  dep_wait();
-  double s = 0.0;
-  const long long st = (long long)kNormParts * kThreads;
-  auto add = [&](uint8_t mm, T xv) {
-    if (mm) {
-      const double v = (double)xv;
-      if (mm == 1) s = __fma_rn(v, v, s);
-      else s = weighted_square(mm, v, s);
-    }
-  };
-  long long I = (long long)blockIdx.x * kThreads + threadIdx.x;
-  for (; I + 3 * st < n; I += 4 * st) {  // four elements' loads in flight, added in their order
-    const uint8_t m0 = m[I], m1 = m[I + st], m2 = m[I + 2 * st], m3 = m[I + 3 * st];
-    const T x0 = x[I], x1 = x[I + st], x2 = x[I + 2 * st], x3 = x[I + 3 * st];
-    add(m0, x0);
-    add(m1, x1);
-    add(m2, x2);
-    add(m3, x3);
-  }
-  for (; I < n; I += st) add(m[I], x[I]);
+// s: each thread's sum
+__device__ __forceinline__ void norm_finish(double s, double* __restrict__ partials, unsigned* counter, double* out,
+                                            const double* normb, int norm_kind, const LoopTest& lt) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_down_sync(0xffffffffu, s, o));
   __shared__ double ws[kThreads / 32];
@@ -639,11 +618,100 @@ __global__ void __launch_bounds__(kThreads) k_norm(const T* __restrict__ x, cons
     }
   }
 }
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_norm(const T* __restrict__ x, const uint8_t* __restrict__ m, long long n,
+                                                   double* __restrict__ partials, unsigned* counter, double* out,
+                                                   const double* normb, int norm_kind, LoopTest lt) {
+  dep_wait();
+  double s = 0.0;
+  const long long st = (long long)kNormParts * kThreads;
+  auto add = [&](uint8_t mm, T xv) {
+    if (mm) {
+      const double v = (double)xv;
+      if (mm == 1) s = __fma_rn(v, v, s);
+      else s = weighted_square(mm, v, s);
+    }
+  };
+  long long I = (long long)blockIdx.x * kThreads + threadIdx.x;
+  for (; I + 3 * st < n; I += 4 * st) {  // four elements' loads in flight, added in their order
+    const uint8_t m0 = m[I], m1 = m[I + st], m2 = m[I + 2 * st], m3 = m[I + 3 * st];
+    const T x0 = x[I], x1 = x[I + st], x2 = x[I + 2 * st], x3 = x[I + 3 * st];
+    add(m0, x0);
+    add(m1, x1);
+    add(m2, x2);
+    add(m3, x3);
+  }
+  for (; I < n; I += st) add(m[I], x[I]);
+  norm_finish(s, partials, counter, out, normb, norm_kind, lt);
+}
 __global__ void k_loop_start(LoopTest lt) {
   lt.ds[S_NITE] = 0.0;
   loop_test(lt, lt.ds[S_RES], lt.ds[S_NORMB]);
 }
 void launch_loop_start(const LoopTest& lt, cudaStream_t s) { k_loop_start<<<1, 1, 0, s>>>(lt); }
+
+// An FP64 level's residual and its norm in one launch, for levels of at most
+// one cell a thread of the norm (kNormParts blocks: 262 144 cells), whose two
+// launches are latency: the cell's residual as the separate kernel stores it
+// (cells out of its range keep their r), then the norm's own sums. A 64^2 FP64
+// solve takes 909 us with it and 963 with two launches.
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) k_resid_norm(double* __restrict__ r, const double* __restrict__ x,
+                                                         const double* __restrict__ b, const double* __restrict__ d,
+                                                         const double* __restrict__ cE, const double* __restrict__ cN,
+                                                         const uint8_t* __restrict__ m, Geom g, Box bx, long long lo,
+                                                         long long hi, long long n, double* __restrict__ partials,
+                                                         unsigned* counter, double* out, const double* normb,
+                                                         int norm_kind, LoopTest lt) {
+  dep_wait();
+  const long long I = (long long)blockIdx.x * kThreads + threadIdx.x;
+  double s = 0.0;
+  if (I < n) {
+    bool in;
+    if (KIND == OPK_RESID5 || KIND == OPK_RESIDVC) {
+      in = I >= lo && I < hi;
+    } else {
+      const int k = (int)(I / g.n2), q = (int)(I - k * g.n2), j = q / (int)g.n1, i = q - j * (int)g.n1;
+      in = i + 1 >= bx.i0 && i + 1 <= bx.i1 && j + 1 >= bx.j0 && j + 1 <= bx.j1 && k + 1 >= bx.k0 && k + 1 <= bx.k1;
+    }
+    const uint8_t mm = m[I];
+    double v = 0.0;
+    if (in) {
+      if (KIND == OPK_RESID5) v = v_resid5(x, b, d, m, g.n1, I);
+      if (KIND == OPK_RESID7) v = v_resid7(x, b, d, m, g.n1, g.n2, I);
+      if (KIND == OPK_RESID9) v = v_resid9(x, b, d, m, g.n1, I);
+      if (KIND == OPK_RESID19) v = v_resid19(x, b, d, m, g.n1, g.n2, I);
+      if (KIND == OPK_RESIDVC) v = v_residvc(x, b, d, cE, cN, m, g.n1, I);
+      r[I] = v;
+    } else if (mm) {
+      v = r[I];
+    }
+    if (mm == 1) s = __fma_rn(v, v, s);
+    else if (mm) s = weighted_square(mm, v, s);
+  }
+  norm_finish(s, partials, counter, out, normb, norm_kind, lt);
+}
+void launch_resid_norm(int kind, double* r, const double* x, const double* b, const double* d, const double* cE,
+                       const double* cN, const uint8_t* m, const Geom& g, const Box& bx, double* partials,
+                       unsigned* counter, double* out, const double* normb, int norm_kind, cudaStream_t s,
+                       const LoopTest* lt) {
+  const long long n = g.len;
+  const unsigned nb = nblocks(n);
+  switch (kind) {
+#define CFMG_RN(K)                                                                                              \
+  case K:                                                                                                       \
+    launch_dep(k_resid_norm<K>, nb, kThreads, 0, s, r, x, b, d, cE, cN, m, g, bx, g.n1, g.len - g.n1, n, partials, \
+               counter, out, normb, norm_kind, lt ? *lt : LoopTest{});                                         \
+    return;
+    CFMG_RN(OPK_RESID5)
+    CFMG_RN(OPK_RESID7)
+    CFMG_RN(OPK_RESID9)
+    CFMG_RN(OPK_RESID19)
+    CFMG_RN(OPK_RESIDVC)
+#undef CFMG_RN
+    default: break;
+  }
+}
 
 // --------------------------------------------------------------- launchers
 template <class T>
