@@ -1282,7 +1282,8 @@ int step2d(cfmg_handle* h, int lev, int mode, int np) {
   a.xs = mode == 2 ? a.s : first ? v.x : nullptr;
   a.b = v.b; a.w = v.widiag; a.cE = v.cE; a.cN = v.cN; a.d = v.diag; a.pc = v.Pcoef;
   a.xc = vc.x; a.rc = vc.Rcoef; a.m = v.msk;
-  a.bc = vc.b; a.xcz = vc.x;
+  a.bc = vc.b;
+  if (mode == 0) a.xcz = vc.x;
   if (!first) a.x = v.x;
   if (sizeof(T) == 8) {  // the FP32 y and r of a cycle are read by nothing after the step
     if (!first) a.y = v.y;
@@ -1359,8 +1360,14 @@ int vcycle_t(cfmg_handle* h, int lev0, bool prolonged = false) {
   const int nl = L(h);
   auto step = [&](int lev) { return (lev > lev0 || lev == 1 || prolonged) && step_ok<T>(h, lev); };
   for (int lev = lev0; lev <= nl - 1; ++lev) {
-    if (step(lev)) TRY(step2d<T>(h, lev, lev == lev0 && prolonged ? 1 : 0, d.npre));
-    else TRY(descend_t<T>(h, lev, d.npre, !(lev + 1 < nl && step(lev + 1))));
+    const bool zero_coarse = !(lev + 1 < nl && step(lev + 1));  // a step assigns its x
+    if (!step(lev)) {
+      TRY(descend_t<T>(h, lev, d.npre, zero_coarse));
+      continue;
+    }
+    const bool pro = lev == lev0 && prolonged;
+    TRY(step2d<T>(h, lev, pro ? 1 : 0, d.npre));
+    if (pro && zero_coarse) TRY(zero_t<T>(h, lev + 1, CFMG_X));  // which that step reads (k_tbg.cu)
   }
   TRY(coarsest_t<T>(h, d.ndeepest));
   for (int lev = nl - 1; lev >= lev0; --lev) {

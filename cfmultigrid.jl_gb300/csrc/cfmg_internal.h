@@ -338,7 +338,7 @@ struct TbgArgs {
   const T *b, *w, *cE, *cN, *d, *pc;    // pc: the level's Pcoef
   const T *xc, *rc;                     // coarse x (prolonged), coarse Rcoef
   const uint8_t* m;
-  T *x, *y, *r, *s, *bc, *xcz;          // s: the scratch; bc, xcz: coarse b, and coarse x to zero (y, r may be null)
+  T *x, *y, *r, *s, *bc, *xcz;          // s: the scratch; bc: coarse b; xcz: coarse x, zeroed by mode 0 (y, r may be null)
   T cff;
   int np, tx, ty, nh, ctx, cty, np_i, np_j;  // np: pairs of sweeps; np_i x np_j prolongation parents
 };

@@ -8,8 +8,8 @@
 // graph node, is what they cost. Here a block loads a tile with a halo wide
 // enough for the whole step into shared memory and runs it there:
 //   descent: x = +0, or x = Pcoef P(coarse x) after an F-cycle's prolongation;
-//            np pairs of sweeps; residual; restriction into the coarse b, the
-//            coarse x zeroed
+//            np pairs of sweeps; residual; restriction into the coarse b; from
+//            x = +0 also the coarse x zeroed
 //   ascent:  x = x + Pcoef P(coarse x), np pairs of sweeps
 //   smoothing: np pairs of sweeps from x into the scratch, or back (a long
 //            smoothing of the last level, pass after pass)
@@ -18,6 +18,9 @@
 // writes: a descent reads no x at all, and leaves a copy of its result in the
 // level's scratch array, which is what the ascent reads. Level 1 starts from
 // the caller's x; its descent writes the scratch only, and the ascent x and y.
+// A descent from Pcoef P(coarse x) reads coarse cells in its neighbours' cores,
+// so it leaves the coarse x as it is: the caller zeroes it in a launch of its
+// own where the next level reads it before writing it.
 //
 // Every cell of the tile is updated by the same formula, which rests on the
 // coefficients that setup_operators made (the caller checks that they are)
@@ -242,7 +245,7 @@ __global__ void __launch_bounds__(g_threads<T>()) k_step2d(TbgArgs<T> a, int S, 
     }
     const long long C = (long long)(ii - 1) + (long long)a.ctx * (jj - 1);
     a.bc[C] = A::mul(a.rc[C], v);
-    a.xcz[C] = T(0);
+    if (MODE == 0) a.xcz[C] = T(0);  // MODE 1: other tiles may still read it
   }
 }
 
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(kVW * kVG, 2) k_step2d_vc(TbgArgs<float> a) {
     const float v = A::add(A::add(A::add(y[0], y[1]), y[kVS]), y[kVS + 1]);
     const long long C = (long long)(ii - 1) + (long long)a.ctx * (jj - 1);
     a.bc[C] = A::mul(a.rc[C], v);
-    a.xcz[C] = 0.f;
+    if (MODE == 0) a.xcz[C] = 0.f;
   }
 }
 

@@ -125,3 +125,20 @@ def test_long_smoothing_of_the_last_level(name, cycle, size, nlevels):
     a, b = (_run(fused, *size, 3, **p) for fused in (1, 0))
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("size,pairs", [((1500, 1404), (2, 2)), ((1537, 1210), (3, 1))])
+def test_fcycle_steps_of_several_waves_of_tiles(size, pairs):
+    """The descent after an F-cycle's prolongation, on a level of some 1100 tiles and more where 304 are resident: every
+    tile prolongs the coarse x as it was before the step, whichever tiles have finished, and a second run repeats."""
+    p = dict(operator="varcoef", cycle="f", npre=pairs[0], npost=pairs[1], omega=0.8, nlevels=6, precision="mixed",
+             residual_norm="l2")
+    out = []
+    for fused in (0, 1, 1):
+        mg = _make(fused, *size, 13, **p)
+        _, _, hist = cfmg.solve(mg, history=True, maxite=4, tol=0.0)
+        out.append((hist, mg.data[1].x))
+        mg.close()
+    for hist, x in out[1:]:
+        assert np.array_equal(out[0][0], hist)
+        assert np.array_equal(out[0][1], x)
