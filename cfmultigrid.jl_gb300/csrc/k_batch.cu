@@ -140,6 +140,8 @@ __global__ void __cluster_dims__(kInitCtas, 1, 1) __launch_bounds__(kBThreads)
   __shared__ double sh[kBThreads / 32];
   __shared__ unsigned long long shu[kBThreads / 32];
   __shared__ double part[kInitCtas][3];  // block 0's copy collects every block's results
+  // a block's shared memory may be written once the block runs: all arrive here, and wait before the stores below
+  asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
   const int inst = blockIdx.x / kInitCtas, rank = blockIdx.x % kInitCtas;
   const BInst& B = bi[inst];
   const bool zx = zero_x != 0;
@@ -181,6 +183,7 @@ __global__ void __cluster_dims__(kInitCtas, 1, 1) __launch_bounds__(kBThreads)
   }
   const double s0 = bsum(v, sh);
   const unsigned long long m0 = bmax_bits(mx, shu), m1 = bmax_bits(mb, shu);
+  asm volatile("barrier.cluster.wait;" ::: "memory");
   if (threadIdx.x == 0) {
     const double res[3] = {s0, __longlong_as_double((long long)m0), __longlong_as_double((long long)m1)};
 #pragma unroll
@@ -190,6 +193,7 @@ __global__ void __cluster_dims__(kInitCtas, 1, 1) __launch_bounds__(kBThreads)
       asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(res[q]) : "memory");
     }
   }
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (rank == 0 && threadIdx.x == 0) {
     double* sc = B.sc;
