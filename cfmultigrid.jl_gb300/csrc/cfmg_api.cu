@@ -449,8 +449,9 @@ bool build_tail(const cfmg_handle* h, const std::vector<Op>& P, std::vector<Tail
         const Level& l = h->lv[a.lev - 1];
         TailCtx c;
         std::memset(&c, 0, sizeof(c));
-        c.stencil = a.kind == OPK_SWEEP5 ? TAIL_5 : a.kind == OPK_SWEEP7 ? TAIL_7 : a.kind == OPK_SWEEP9 ? TAIL_9
-                    : a.kind == OPK_SWEEP19 ? TAIL_19 : TAIL_VC;
+        c.scan = 1;
+        for (size_t z = 0; z < i; ++z)
+          if ((P[z].kind == OPK_ZERO || P[z].kind == OPK_F32TO64) && P[z].y == a.x) c.scan = 0;
         c.prec = a.prec;
         c.n1 = (int)a.g.n1; c.n2 = (int)a.g.n2;
         c.lines = l.ty * l.tz; c.nh = l.nh; c.nx = l.nx;

@@ -287,7 +287,8 @@ enum TailStencil { TAIL_5 = 0, TAIL_7, TAIL_9, TAIL_19, TAIL_VC };
 constexpr int TAIL_SMOOTH = 1000;  // TailOp kind: npairs pairs of sweeps of context ctxi
 constexpr int kTailListHdr = 16;  // bytes in front of a list: {listed cells, cells of the range}
 struct alignas(16) TailCtx {
-  int stencil, prec, n1, n2, lines, nh, nx;  // lines: rows of the level (x-periodic fill)
+  // scan: x was not written as a whole by the program before the first smoothing call; lines: rows of the level
+  int scan, prec, n1, n2, lines, nh, nx;
   unsigned ox, oy, ob, ow, oE, oN, olist;
   double cff;
 };

@@ -17,8 +17,9 @@
 // out changes no bit. On the coarsest levels most of the range is halo and
 // land (a 4^2 level: 16 of 80 cells), and the FP64 pipe (one warp instruction
 // in 76 clocks per quarter of an SM, measured) is what bounds a sweep there.
-// A level that fails the check, or omega > 1 (whose zeros change sign),
-// sweeps its whole range as the reference does. The residual below level 1
+// A level that fails the check, one with a NaN or an infinity in x, y or b
+// (t is not finite then), or omega > 1 (whose zeros change sign), sweeps its
+// whole range as the reference does. The residual below level 1
 // is formed at the listed cells; the others, whose mask is 0, get +0.
 //
 // The per-cell arithmetic and ranges are those of the standalone kernels
@@ -157,17 +158,26 @@ __device__ __forceinline__ bool nonzero_bits(float v) { return __float_as_uint(v
 template <>
 __device__ __forceinline__ bool nonzero_bits(double v) { return __double_as_longlong(v) != 0ll; }
 
-// whether a cell that the context's list leaves out of its sweeps holds something in x or y
+__device__ __forceinline__ bool finite_bits(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ bool finite_bits(double v) { return is_fin(v); }
+
+// whether the level must sweep its whole range: a cell that the context's list
+// leaves out holds something in x or y or a NaN or an infinity in b, or (where
+// x was not zeroed in the program) any cell of the array one in x or y: the
+// sweeps carry them on
 template <class T>
 __device__ __forceinline__ bool tail_dirty(const TailCtx& c, int nact, int nrange) {
   const T* x = reinterpret_cast<const T*>(sm + c.ox);
   const T* y = reinterpret_cast<const T*>(sm + c.oy);
+  const T* b = reinterpret_cast<const T*>(sm + c.ob);
   const unsigned short* list = reinterpret_cast<const unsigned short*>(sm + c.olist + kTailListHdr);
   bool bad = false;
   for (int t = nact + (int)threadIdx.x; t < nrange; t += kTT) {
     const int I = list[t] & (kOut2 - 1);
-    bad |= nonzero_bits(x[I]) || nonzero_bits(y[I]);
+    bad |= nonzero_bits(x[I]) || nonzero_bits(y[I]) || !finite_bits(b[I]);
   }
+  if (c.scan)
+    for (int I = threadIdx.x; I < c.lines * c.n1; I += kTT) bad |= !finite_bits(x[I]) || !finite_bits(y[I]);
   return bad;
 }
 
