@@ -32,6 +32,8 @@ struct cfmg_handle {
   double* hscal = nullptr;     // pinned host mirror of dscal
   std::string err;
   bool mixed_dirty = true;     // FP32 coefficient copies need refreshing
+  // a mask changed / FP32 cycles have run since the FP32 fields were cleared (see prepare_mixed)
+  bool msk_changed = false, f32_used = false;
   // captured graphs: one cycle + normresidual per cycle kind and precision
   cudaGraphExec_t graph[2][6] = {{nullptr}};
   long long graph_launches[2][6] = {{0}};
@@ -1648,7 +1650,14 @@ int prepare_wq(cfmg_handle* h) {
 }
 
 int prepare_mixed(cfmg_handle* h) {
+  const bool clear = h->mixed_dirty && h->f32_used && (h->msk_changed || h->coef_exposed);
+  if (h->mixed_dirty) h->msk_changed = false;
+  h->f32_used = true;
   if (!h->mixed_dirty) return CFMG_OK;
+  if (clear)  // passes that skip dry cells rely on +0 there: cells that were wet hold their old values
+    for (Level& l : h->lv)
+      for (float* f : {l.x32, l.y32, l.r32, l.b32})
+        CUDA_OK(h, cudaMemsetAsync(f, 0, l.len * sizeof(float), h->stream));
   for (Level& l : h->lv) {
     launch_to_f32(l.widiag, l.widiag32, l.len, h->stream);
     launch_to_f32(l.diag, l.diag32, l.len, h->stream);
@@ -2415,6 +2424,7 @@ static int refresh_derived(cfmg_handle* h, int lev, int field) {
   if (field >= CFMG_DIAG) {
     h->mixed_dirty = h->lists_dirty = true;
     h->coef_setup = false;
+    if (field == CFMG_MSK) h->msk_changed = true;
   }
   LAUNCH_OK(h);
   return CFMG_OK;
@@ -2468,7 +2478,7 @@ int cfmg_set_default_msk(cfmg_handle* h) {
   Level& l = h->lv[0];
   launch_default_msk(DEFMSK_SET, l.msk, nullptr, 0.0, l, vertices(h), threed(h), xperio(h), h->stream);
   LAUNCH_OK(h);
-  h->lists_dirty = true;
+  h->lists_dirty = h->msk_changed = true;
   h->coef_setup = false;
   return sync(h);
 }
@@ -2538,7 +2548,7 @@ int cfmg_fill(cfmg_handle* h, int lev, int field) {
   if (!xperio(h)) return CFMG_OK;
   TRY(flush(h));
   if (field >= CFMG_DIAG) {
-    h->lists_dirty = true;
+    h->lists_dirty = h->msk_changed = true;
     h->coef_setup = false;
   }
   if (elt == 1) launch_fill_xperio<uint8_t>((uint8_t*)p, geom(l), h->stream);
