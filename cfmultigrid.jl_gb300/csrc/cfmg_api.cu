@@ -56,9 +56,10 @@ struct cfmg_handle {
   cfmg::Op* prog_pool = nullptr;   // device program store
   int pool_cap = 0, pool_used = 0;
   std::unordered_map<std::string, int> prog_cache;
-  // coarse tail (k_tail.cu): levels >= tail_from[prec] run there (0: none);
+  // coarse tail (k_tail.cu): levels >= tail_from[prec] run there (0: none),
+  // FP64 ones from tail_steps on while those above it take one-launch steps;
   // pending_tail: the pending Ops are the tail's, not the cluster engine's
-  int tail_from[2] = {0, 0};
+  int tail_from[2] = {0, 0}, tail_steps = 0;
   bool pending_tail = false;
   unsigned char* tail_pool = nullptr;  // device store of tail programs
   size_t tail_cap = 0, tail_used = 0;
@@ -70,6 +71,7 @@ struct cfmg_handle {
   // its wet interior (written by the caller or by the setup, not zeroed since)
   bool coef_setup = false;
   std::vector<unsigned> dirt;
+  bool step_cycle = false;  // while a V- or F-cycle is emitted, whose steps may be one launch each (StepScope)
   int graph_steps = 0;  // the captured graphs' steps_clean and coef_clean (see step_ok)
   std::unordered_map<std::string, size_t> tail_cache;
   bool tb_on = true;  // temporally blocked FP32 smoothing on fine levels
@@ -353,8 +355,8 @@ bool coarsest_in_fp64(const cfmg_handle* h) {
 // levels of more than 6/5 of the engine's FP64 threshold (1500 cells by
 // default) stay out, because one SM's FP64 pipe then takes longer for a sweep
 // than a launch on all SMs does: a 38^2 level with every cell wet takes
-// 2.1 us a sweep in the tail and 2.2 us as a launch. Where the level's steps
-// can be one launch each (k_tbg.cu) the line lies at 2/5 of that, 600 cells: a
+// 2.1 us a sweep in the tail and 2.2 us as a launch. While the level's steps
+// are one launch each (steps_run) the line lies at 2/5 of that, 600 cells: a
 // 38^2 disk level takes 21 us a cycle in the tail and 10 us as two steps.
 constexpr size_t kTailBlobReserve = 24 * 1024;
 constexpr size_t tail_al(size_t b) { return (b + 15) & ~(size_t)15; }
@@ -362,16 +364,34 @@ size_t tail_hot_bytes(const cfmg_handle* h, const Level& l, int prec) {
   const size_t n = l.len, es = prec ? 4 : 8;
   return (h->d.op == CFMG_VARCOEF ? 6 : 4) * tail_al(n * es) + tail_al(kTailListHdr + 2 * n);
 }
-// whether the handle's FP64 levels can take one-launch steps (see step_ok)
+// whether the handle's 2D levels can take one-launch steps at all (k_tbg.cu), and
+// whether they do now (see step_ok): the fields and coefficients allow it
 bool steps_form(const cfmg_handle* h) {
   return !threed(h) && !xperio(h) && h->lv[0].tz == 1 && h->fuse_on && h->d.omega <= 1.0;
 }
+bool steps_clean(const cfmg_handle* h);
+bool coef_clean(const cfmg_handle* h);
+bool step_size(const cfmg_handle* h, int lev, int prec);
+// While it lives, levels are shared out between tail, engine and launches as
+// for a V- or F-cycle (on) or as for anything else (single smoothing calls, the
+// other cycles), which take no one-launch steps
+struct StepScope {
+  cfmg_handle* h;
+  bool was;
+  StepScope(cfmg_handle* hh, bool on) : h(hh), was(hh->step_cycle) { h->step_cycle = on; }
+  ~StepScope() { h->step_cycle = was; }
+};
+bool steps_run(const cfmg_handle* h, int prec) {
+  return h->step_cycle && steps_form(h) && h->d.npre >= 1 && h->d.npre <= kTbgMaxPairs && h->d.npost >= 1 &&
+         h->d.npost <= kTbgMaxPairs && (prec ? h->d.op == CFMG_VARCOEF && coef_clean(h) : steps_clean(h));
+}
 void plan_tail(cfmg_handle* h) {
   h->lists_dirty = true;  // the levels that need lists may change
+  h->tail_steps = 0;
   for (int prec = 0; prec < 2; ++prec) {
     h->tail_from[prec] = 0;
     if (!h->engine_on || h->small_min <= 0 || (prec == 1 && h->d.precision != CFMG_MIXED)) continue;
-    const long long cap = prec == 0 ? engine_limit(h, 0) * 6 / 5 * 2 / (steps_form(h) ? 5 : 2) : engine_limit(h, 1);
+    const long long cap = prec == 0 ? engine_limit(h, 0) * 6 / 5 : engine_limit(h, 1);
     size_t used = kTailBlobReserve;
     if (prec == 1 && coarsest_in_fp64(h)) used += tail_hot_bytes(h, h->lv.back(), 0);
     for (int lev = L(h); lev >= 1 && L(h) - lev < kTailMaxCtx - 2; --lev) {
@@ -379,11 +399,18 @@ void plan_tail(cfmg_handle* h) {
       used += tail_hot_bytes(h, l, prec);
       if (used > kTailSmemMax || (long long)l.len > cap || !l.tlist) break;
       h->tail_from[prec] = lev;
+      if (prec == 0 && (long long)l.len <= cap * 2 / 5) h->tail_steps = lev;
     }
   }
 }
+// the first level of the tail, 0 without one
+int tail_start(const cfmg_handle* h, int prec) {
+  return prec == 0 && steps_run(h, 0) ? h->tail_steps : h->tail_from[prec];
+}
 bool in_tail(const cfmg_handle* h, int lev, int prec) {
-  return !h->record && h->tail_pool && h->engine_on && h->tail_from[prec] > 0 && lev >= h->tail_from[prec];
+  if (h->record || !h->tail_pool || !h->engine_on) return false;
+  const int from = tail_start(h, prec);
+  return from > 0 && lev >= from;
 }
 
 // Copies a program into its device store, complete on return: allowed while
@@ -739,10 +766,10 @@ bool in_engine(const cfmg_handle* h, int lev, int prec) {
   if (!h->engine_on) return false;
   if (in_tail(h, lev, prec)) return true;
   if ((long long)h->lv[lev - 1].len > engine_limit(h, prec)) return false;
-  // FP64 levels between the tail and the threshold take one-launch steps
+  // while steps run, FP64 levels between the tail and the threshold take them,
   // and so do FP32 ones of the variable-coefficient operator
-  const bool steps = h->tail_pool && h->tail_from[prec ? 1 : 0] > 0 && steps_form(h);
-  return !(prec ? blocked_form(h, lev) || (steps && h->d.op == CFMG_VARCOEF) : steps);
+  const bool steps = h->tail_pool && tail_start(h, prec ? 1 : 0) > 0 && steps_run(h, prec) && step_size(h, lev, prec);
+  return !(prec ? blocked_form(h, lev) || steps : steps);
 }
 
 int emit(cfmg_handle* h, const Op& op) {
@@ -1252,16 +1279,17 @@ bool steps_clean(const cfmg_handle* h) {
     if (h->dirt[k - 1]) return false;
   return true;
 }
+// FP32 (variable coefficient), levels of every size: a level-1 descent of 2048^2 reads its five
+// arrays once instead of in each of four sweeps (its fields hold +0 outside the wet interior always)
+bool step_size(const cfmg_handle* h, int lev, int prec) {
+  return prec || (long long)h->lv[lev - 1].len * (h->d.op == CFMG_LAPLACIAN ? 7 : 11) <=
+                     (lev == 1 ? kStepWork1 : kStepWork);
+}
 template <class T>
 bool step_ok(const cfmg_handle* h, int lev) {
-  if (h->record || !steps_form(h) || lev >= L(h)) return false;
-  if (h->d.npre < 1 || h->d.npre > kTbgMaxPairs || h->d.npost < 1 || h->d.npost > kTbgMaxPairs) return false;
+  if (h->record || lev >= L(h) || !steps_run(h, pc<T>()) || !step_size(h, lev, pc<T>())) return false;
   const Level& l = h->lv[lev - 1];
-  // FP32 variable coefficient, levels of every size: a level-1 descent of 2048^2 reads its five
-  // arrays once instead of in each of four sweeps (its fields hold +0 outside the wet interior always)
-  if (sizeof(T) == 4) return h->d.op == CFMG_VARCOEF && l.s32 && !in_engine(h, lev, CFMG_MIXED) && coef_clean(h);
-  if ((long long)l.len * (h->d.op == CFMG_LAPLACIAN ? 7 : 11) > (lev == 1 ? kStepWork1 : kStepWork)) return false;
-  return l.s64 && !in_engine(h, lev, CFMG_FP64) && steps_clean(h);
+  return (sizeof(T) == 4 ? l.s32 != nullptr : l.s64 != nullptr) && !in_engine(h, lev, pc<T>());
 }
 
 template <class T>
@@ -1443,6 +1471,7 @@ int cycle_body(cfmg_handle* h, int kind, bool x1_zero = false) {
 
 template <class T>
 int cycle_t(cfmg_handle* h, int kind, bool x1_zero = false) {
+  const StepScope sc(h, kind == CFMG_CYCLE_V || kind == CFMG_CYCLE_VREC || kind == CFMG_CYCLE_F);
   TRY(cycle_body<T>(h, kind, x1_zero));
   return flush(h);
 }
@@ -1463,6 +1492,7 @@ int norm_dev(cfmg_handle* h, int lev, const double* x, const double* normb, int 
 int resid_kind(const cfmg_handle* h);
 // residual at level 1 followed by its norm ratio into dscal[S_RES]
 int normresidual_dev(cfmg_handle* h, int kind) {
+  const StepScope sc(h, true);
   const Level& l = h->lv[0];
   if ((long long)l.len <= kResidNormMax && !xperio(h) && !h->record && !in_engine(h, 1, CFMG_FP64)) {
     TRY(flush(h));
@@ -1885,6 +1915,7 @@ bool x1_zero_ok(const cfmg_handle* h, int kind) {
 }
 
 int mixed_iteration(cfmg_handle* h, int kind) {
+  const StepScope sc(h, true);  // a V- or F-cycle
   for (Level& l : h->lv) l.xswap = 0;  // every FP32 x is zeroed before use in the cycle
   // the F-cycle's first write of level 1's x is its last prolongation: the
   // x buffer (+0 outside the wet interior in both buffers) is assigned
