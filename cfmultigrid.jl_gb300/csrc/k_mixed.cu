@@ -504,11 +504,24 @@ bool launch_resid_int2d(int kind, const double* x, const double* b, const int8_t
 
 // ---- wet sum of r for the operators without a fused pass (variable
 // coefficient, x-periodic), per block into partials[kNormParts]. Each r is
-// taken to 64-bit fixed point, 2^58 steps for the bound |r| <= sqrt(sum r^2)
-// that the norm just gave (ds[S_NORM]), and added exactly in 128-bit integers:
-// rounding below 2^-59 of the bound a cell, against the bound's sqrt(n) times
-// smaller rms of r. The compensated FP64 sum it replaces issued six FP64
-// operations a cell: 66 us at 2048^2 against 13.7.
+// taken to fixed point with 94 bits below the bound |r| <= sqrt(sum r^2) that
+// the norm just gave (ds[S_NORM]) and added exactly in 128-bit integers: an r
+// above 2^-41 of the bound keeps all its bits, a smaller one loses less than
+// 2^-94 of it. A thread's sum is then right to the last bit of a double, as
+// the compensated FP64 sum that this replaces was (with 58 bits it was off by
+// up to 2^-59 of the bound a cell, which is sqrt(n) times the rms of r). That
+// sum issued six FP64 operations a cell: 66 us at 2048^2 against 15.
+// v 2^k for |v| 2^k < 2^95, towards zero; zero and subnormal v give 0 (k <= 1022)
+__device__ __forceinline__ __int128 to_fix_wide(double v, int k) {
+  const int hi = __double2hiint(v);
+  const unsigned lo = (unsigned)__double2loint(v);
+  const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+  const int n = min(max(1117 - k - (int)(((unsigned)hi << 1) >> 21), 0), 127);
+  // the significand, 42 bits up
+  const unsigned long long top = __funnelshift_l(lo, mh, 10), low = (unsigned long long)(lo << 10) << 32;
+  const __int128 m = (__int128)((((unsigned __int128)top << 64) | low) >> n);
+  return hi < 0 ? -m : m;
+}
 __global__ void __launch_bounds__(256) k_mean_fix(const double* __restrict__ r, const uint8_t* __restrict__ m,
                                                   long long n, const double* __restrict__ ds,
                                                   double* __restrict__ partials) {
@@ -516,17 +529,20 @@ __global__ void __launch_bounds__(256) k_mean_fix(const double* __restrict__ r, 
   int e2 = 0;
   const double sq = ds[S_NORM];
   if (sq > 0 && isfinite(sq)) frexp(sq, &e2);  // sum r^2 < 2^e2
-  const int k = 58 - ((e2 + 1) >> 1);
+  const int k = 94 - ((e2 + 1) >> 1);
   __int128 s = 0;
   const long long st = (long long)kNormParts * 256;
   long long I = (long long)blockIdx.x * 256 + threadIdx.x;
   for (; I + 3 * st < n; I += 4 * st) {  // four cells' loads in flight
     const double v0 = r[I], v1 = r[I + st], v2 = r[I + 2 * st], v3 = r[I + 3 * st];
     const uint8_t m0 = m[I], m1 = m[I + st], m2 = m[I + 2 * st], m3 = m[I + 3 * st];
-    s += (__int128)((m0 ? to_fix(v0, k) : 0LL)) + (m1 ? to_fix(v1, k) : 0LL);
-    s += (__int128)((m2 ? to_fix(v2, k) : 0LL)) + (m3 ? to_fix(v3, k) : 0LL);
+    if (m0) s += to_fix_wide(v0, k);
+    if (m1) s += to_fix_wide(v1, k);
+    if (m2) s += to_fix_wide(v2, k);
+    if (m3) s += to_fix_wide(v3, k);
   }
-  for (; I < n; I += st) s += m[I] ? to_fix(r[I], k) : 0LL;
+  for (; I < n; I += st)
+    if (m[I]) s += to_fix_wide(r[I], k);
   double v = int_to_double(s);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
