@@ -681,7 +681,9 @@ int flush_tail(cfmg_handle* h, bool& done) {
   for (size_t i = 0; i < built.size(); ++i) {
     const TailBuild& q = built[i];
     Launch k(h, CFMG_K_ENGINE, 0, h->pending[0].prec ? CFMG_MIXED : CFMG_FP64);
-    launch_tail(tail_stencil(h), rp_kind(h), h->tail_pool + at[i], (int)q.bytes.size(), q.nctx, q.nstore, q.ncopy, q.nops, q.smem, h->stream);
+    if (!launch_tail(tail_stencil(h), rp_kind(h), h->tail_pool + at[i], (int)q.bytes.size(), q.nctx, q.nstore,
+                     q.ncopy, q.nops, q.smem, h->stream))
+      return fail(h, CFMG_ERR_UNSUPPORTED, "no coarse-tail kernel for this operator");
   }
   done = true;
   return CFMG_OK;
@@ -1498,9 +1500,10 @@ int normresidual_dev(cfmg_handle* h, int kind) {
     TRY(flush(h));
     {
       Launch k(h, CFMG_K_RESIDUAL, 1, CFMG_FP64);
-      launch_resid_norm(h->d.op == CFMG_VARCOEF ? OPK_RESIDVC : resid_kind(h), l.r, l.x, l.b, l.diag, l.cE, l.cN,
-                        l.msk, geom(l), interior(l), h->partials, norm_counter(h), h->dscal + S_NORM,
-                        h->dscal + S_NORMB, kind, h->stream, h->loop);
+      if (!launch_resid_norm(h->d.op == CFMG_VARCOEF ? OPK_RESIDVC : resid_kind(h), l.r, l.x, l.b, l.diag, l.cE, l.cN,
+                             l.msk, geom(l), interior(l), h->partials, norm_counter(h), h->dscal + S_NORM,
+                             h->dscal + S_NORMB, kind, h->stream, h->loop))
+        return fail(h, CFMG_ERR_UNSUPPORTED, "no residual-and-norm kernel for this operator");
     }
     LAUNCH_OK(h);
     return CFMG_OK;
@@ -3006,7 +3009,9 @@ int lockstep_body(cfmg_batch* b) {
   }
   for (const cfmg_batch::Step& st : b->steps) {
     if (st.tb == 5) {
-      launch_tail_batch(tail_stencil(b->inst[0]), rp_kind(b->inst[0]), b->tstore, b->tprogs + st.tab0, (int)st.nchunks, (size_t)st.smem, b->active, b->stream);
+      if (!launch_tail_batch(tail_stencil(b->inst[0]), rp_kind(b->inst[0]), b->tstore, b->tprogs + st.tab0,
+                             (int)st.nchunks, (size_t)st.smem, b->active, b->stream))
+        return bfail(b, CFMG_ERR_UNSUPPORTED, "no coarse-tail kernel for this operator");
     } else if (st.tb == 3) {
       launch_brun(b->sops, b->ssm, b->rent, b->runs + st.tab0, (int)st.nchunks, st.smem, b->active, b->stream);
     } else if (st.tb == 2) {

@@ -193,9 +193,9 @@ void launch_norm(const T* x, const uint8_t* msk, size_t n, double* partials, uns
 // before the loop: hist[0] and the test of the first residual (ds[S_RES])
 void launch_loop_start(const LoopTest& lt, cudaStream_t s);
 constexpr int kNormParts = 1024;
-// residual (kind) and its norm in one launch, for levels of at most kResidNormMax cells
+// residual (kind) and its norm in one launch, for levels of at most kResidNormMax cells; false: no such form, nothing launched
 constexpr long long kResidNormMax = kNormParts * 256LL;
-void launch_resid_norm(int kind, double* r, const double* x, const double* b, const double* d, const double* cE,
+bool launch_resid_norm(int kind, double* r, const double* x, const double* b, const double* d, const double* cE,
                        const double* cN, const uint8_t* m, const Geom& g, const Box& bx, double* partials,
                        unsigned* counter, double* out, const double* normb, int norm_kind, cudaStream_t s,
                        const LoopTest* lt);
@@ -306,15 +306,16 @@ struct alignas(16) TailOp {
   Box box;
   unsigned long long x, b, d, cE, cN, coef, m, y;
 };
-// stencil: the operator (TailStencil); kind: its restriction and prolongation, 0 .. 3 as in launch_restrict
-void launch_tail(int stencil, int kind, const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops,
+// stencil: the operator (TailStencil); kind: its restriction and prolongation, 0 .. 3 as in launch_restrict;
+// false: no kernel of that pair, nothing launched
+bool launch_tail(int stencil, int kind, const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops,
                  size_t smem, cudaStream_t s);
 // batched solver: programs of many instances in one launch, a block each
 struct TailProg {
   long long off;  // into the store
   int bytes, nctx, nstore, ncopy, nops, inst;
 };
-void launch_tail_batch(int stencil, int kind, const void* store, const TailProg* tab, int n, size_t smem,
+bool launch_tail_batch(int stencil, int kind, const void* store, const TailProg* tab, int n, size_t smem,
                        const int* active, cudaStream_t s);
 // the cell lists that its smoothing calls sweep, one per level
 struct TailListLevel {

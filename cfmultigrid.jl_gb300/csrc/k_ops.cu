@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(kThreads) k_resid_norm(double* __restrict__ r,
   }
   norm_finish(s, partials, counter, out, normb, norm_kind, lt);
 }
-void launch_resid_norm(int kind, double* r, const double* x, const double* b, const double* d, const double* cE,
+bool launch_resid_norm(int kind, double* r, const double* x, const double* b, const double* d, const double* cE,
                        const double* cN, const uint8_t* m, const Geom& g, const Box& bx, double* partials,
                        unsigned* counter, double* out, const double* normb, int norm_kind, cudaStream_t s,
                        const LoopTest* lt) {
@@ -702,14 +702,14 @@ void launch_resid_norm(int kind, double* r, const double* x, const double* b, co
   case K:                                                                                                       \
     launch_dep(k_resid_norm<K>, nb, kThreads, 0, s, r, x, b, d, cE, cN, m, g, bx, g.n1, g.len - g.n1, n, partials, \
                counter, out, normb, norm_kind, lt ? *lt : LoopTest{});                                         \
-    return;
+    return true;
     CFMG_RN(OPK_RESID5)
     CFMG_RN(OPK_RESID7)
     CFMG_RN(OPK_RESID9)
     CFMG_RN(OPK_RESID19)
     CFMG_RN(OPK_RESIDVC)
 #undef CFMG_RN
-    default: break;
+    default: return false;
   }
 }
 

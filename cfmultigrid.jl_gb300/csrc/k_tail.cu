@@ -474,10 +474,13 @@ static void launch_tail_k(const void* blob, int blob_bytes, int nctx, int nstore
   (void)attr;
   launch_dep(k_tail<ST, K>, 1, kTT, smem, s, (const unsigned char*)blob, blob_bytes, nctx, nstore, ncopy, nops);
 }
-void launch_tail(int stencil, int kind, const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops,
+bool launch_tail(int stencil, int kind, const void* blob, int blob_bytes, int nctx, int nstore, int ncopy, int nops,
                  size_t smem, cudaStream_t s) {
-#define CFMG_TAIL(ST, K) \
-  if (stencil == ST && kind == K) return launch_tail_k<ST, K>(blob, blob_bytes, nctx, nstore, ncopy, nops, smem, s);
+#define CFMG_TAIL(ST, K)                                                           \
+  if (stencil == ST && kind == K) {                                                \
+    launch_tail_k<ST, K>(blob, blob_bytes, nctx, nstore, ncopy, nops, smem, s);    \
+    return true;                                                                   \
+  }
   CFMG_TAIL(TAIL_5, 0)
   CFMG_TAIL(TAIL_5, 2)
   CFMG_TAIL(TAIL_9, 0)
@@ -488,6 +491,7 @@ void launch_tail(int stencil, int kind, const void* blob, int blob_bytes, int nc
   CFMG_TAIL(TAIL_19, 1)
   CFMG_TAIL(TAIL_19, 3)
 #undef CFMG_TAIL
+  return false;
 }
 template <int ST, int K>
 static void launch_tail_batch_k(const void* store, const TailProg* tab, int n, size_t smem, const int* active,
@@ -497,16 +501,20 @@ static void launch_tail_batch_k(const void* store, const TailProg* tab, int n, s
   (void)attr;
   launch_dep(k_tail_batch<ST, K>, (unsigned)n, kTT, smem, s, (const unsigned char*)store, tab, active);
 }
-void launch_tail_batch(int stencil, int kind, const void* store, const TailProg* tab, int n, size_t smem,
+bool launch_tail_batch(int stencil, int kind, const void* store, const TailProg* tab, int n, size_t smem,
                        const int* active, cudaStream_t s) {
-  if (n <= 0) return;
-  if (stencil == TAIL_9) {
-    if (kind == 2) launch_tail_batch_k<TAIL_9, 2>(store, tab, n, smem, active, s);
-    else launch_tail_batch_k<TAIL_9, 0>(store, tab, n, smem, active, s);
-  } else {
-    if (kind == 2) launch_tail_batch_k<TAIL_5, 2>(store, tab, n, smem, active, s);
-    else launch_tail_batch_k<TAIL_5, 0>(store, tab, n, smem, active, s);
+  if (n <= 0) return true;
+#define CFMG_TAIL(ST, K)                                                 \
+  if (stencil == ST && kind == K) {                                      \
+    launch_tail_batch_k<ST, K>(store, tab, n, smem, active, s);          \
+    return true;                                                         \
   }
+  CFMG_TAIL(TAIL_5, 0)
+  CFMG_TAIL(TAIL_5, 2)
+  CFMG_TAIL(TAIL_9, 0)
+  CFMG_TAIL(TAIL_9, 2)
+#undef CFMG_TAIL
+  return false;
 }
 
 void launch_tail_lists(const TailListArgs& a, int n, cudaStream_t s) {
