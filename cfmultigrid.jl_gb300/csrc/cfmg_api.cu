@@ -1614,7 +1614,8 @@ int resid_kind(const cfmg_handle* h) {
 }
 
 // Level-1 Q*diag for the integer form of the fused residual; int_ok when
-// every wet cell's value is an integer in 0..127 and the mask is 0/1.
+// every wet cell's value is an integer small enough for the sums (launch_make_dq)
+// and the mask is 0/1.
 int prepare_int(cfmg_handle* h) {
   h->int_ok = false;
   const int kind = resid_kind(h);
@@ -1624,7 +1625,7 @@ int prepare_int(cfmg_handle* h) {
   int* ok = (int*)h->partials;  // scratch
   const int one = 1;
   CUDA_OK(h, cudaMemcpyAsync(ok, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
-  launch_make_dq(l1.diag, l1.msk, kind == OPK_RESID9 || kind == OPK_RESID19 ? 4.0 : 1.0, h->dq, (long long)l1.len, ok, h->stream);
+  launch_make_dq(kind, l1.diag, l1.msk, h->dq, (long long)l1.len, ok, h->stream);
   {
     const long long ns = resid_sflag_size(kind, geom(l1), interior(l1));
     if (ns > 0) {

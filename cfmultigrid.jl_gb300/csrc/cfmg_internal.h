@@ -545,7 +545,7 @@ void launch_make_tcol(const uint8_t* m, int* tcol, const Geom& g, const Box& bx,
 // skip_dry: groups of 16 dry cells are neither read nor written (their b32 is +0 already)
 void launch_rhs32_shift(const uint8_t* m, const double* mean_scale, float* b32, float* r32, long long n,
                         cudaStream_t s, bool skip_dry = false);
-void launch_make_dq(const double* diag, const uint8_t* m, double Q, int8_t* dq, long long n, int* ok, cudaStream_t s);
+void launch_make_dq(int kind, const double* diag, const uint8_t* m, int8_t* dq, long long n, int* ok, cudaStream_t s);
 // max |x|, max |b| and max |x| outside the box U of every layer (S_MAXX, S_MAXB, S_MAXO)
 // m != null: "outside U" is instead every cell with m == 0 (the dry cells)
 void launch_maxabs2(const double* x, const double* b, long long n, int tx, int ty, int ui0, int ui1, int uj0, int uj1,

@@ -766,16 +766,16 @@ __global__ void __launch_bounds__(256) k_rhs32_shift16(const uint8_t* __restrict
 }
 
 // dq from diag and msk; *ok is cleared when a wet cell's Q*diag is not an
-// integer in 0..127 or a mask value is not 0/1
-__global__ void k_make_dq(const double* __restrict__ diag, const uint8_t* __restrict__ m, double Q, int8_t* dq,
-                          long long n, int* ok) {
+// integer in 0..most or a mask value is not 0/1
+__global__ void k_make_dq(const double* __restrict__ diag, const uint8_t* __restrict__ m, double Q, double most,
+                          int8_t* dq, long long n, int* ok) {
   dep_wait();
   long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (I >= n) return;
   int8_t v = -128;
   if (m[I] == 1) {
     const double qd = diag[I] * Q;
-    if (qd >= 0.0 && qd <= 127.0 && qd == floor(qd)) v = (int8_t)qd;
+    if (qd >= 0.0 && qd <= most && qd == floor(qd)) v = (int8_t)qd;
     else atomicAnd(ok, 0);
   } else if (m[I] != 0) {
     atomicAnd(ok, 0);
@@ -971,9 +971,15 @@ void launch_rhs32_shift(const uint8_t* m, const double* mean_scale, float* b32, 
   }
 }
 
-void launch_make_dq(const double* diag, const uint8_t* m, double Q, int8_t* dq, long long n, int* ok,
+// most: |x| and |b| are at most 2^58 steps (2^57 in the 19-point form), so a
+// sum of dq x, Q b and the neighbours' weights in units of 1/Q stays below 2^63
+// while dq + Q + weights <= 31 (63); the setup's own diag gives 4, 6, 12 and 24
+void launch_make_dq(int kind, const double* diag, const uint8_t* m, int8_t* dq, long long n, int* ok,
                     cudaStream_t s) {
-  launch_dep(k_make_dq, (unsigned)((n + 255) / 256), 256, 0, s, diag, m, Q, dq, n, ok);
+  const bool q4 = kind == OPK_RESID9 || kind == OPK_RESID19;
+  const int others = kind == OPK_RESID5 ? 1 + 4 : kind == OPK_RESID7 ? 1 + 6 : kind == OPK_RESID9 ? 4 + 12 : 4 + 24;
+  const int most = (kind == OPK_RESID19 ? 63 : 31) - others;
+  launch_dep(k_make_dq, (unsigned)((n + 255) / 256), 256, 0, s, diag, m, q4 ? 4.0 : 1.0, (double)most, dq, n, ok);
 }
 
 void launch_maxabs2(const double* x, const double* b, long long n, int tx, int ty, int ui0, int ui1, int uj0, int uj1,
