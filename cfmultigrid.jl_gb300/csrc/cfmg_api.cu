@@ -3115,7 +3115,7 @@ int lockstep_build(cfmg_batch* b) {
     long long items = 0;
     for (const Op& o : ops) items += o.n;
     int chunk = kBStageChunk;
-    while (chunk > kBStageMin && items < (long long)chunk * 152 * kBStageBlocks * kBStageFill) chunk /= 2;
+    while (chunk > kBStageMin && items < (long long)chunk * sm_count() * kBStageBlocks * kBStageFill) chunk /= 2;
     for (size_t j = 0; j < ops.size(); ++j) {
       all.push_back(ops[j]);
       nc[j] = tb ? ops[j].n : (ops[j].n + chunk - 1) / chunk;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <string>
 #include <utility>
 #include <vector>
@@ -91,6 +92,18 @@ inline Geom geom(const Level& l) {
   g.n1 = l.tx;
   g.n2 = (long long)l.tx * l.ty;
   return g;
+}
+
+// SMs of the current device, asked for once a device; for rules that weigh waves of blocks
+inline int sm_count() {
+  constexpr int kDevs = 64;
+  static std::atomic<int> known[kDevs];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 1;
+  if (dev < kDevs && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 1;
+  if (dev < kDevs) known[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 // ---- the FP64 9-point operator on large levels (k_fix.cu)

@@ -778,11 +778,11 @@ __global__ void __launch_bounds__(256) k_sweep7_3d_q(const float* __restrict__ x
 //
 // run: planes a thread sweeps, kQRun or 1. A run reads each plane once instead
 // of three times but takes its planes one after the other; a level that gives
-// fewer than kQBlocks blocks in runs is bound by that chain of loads, and
+// fewer than kQBlocks blocks an SM in runs is bound by that chain of loads, and
 // takes a plane a thread (70 x 70 x 38 and below of a 512 x 512 x 256 solve:
 // 7.4-7.9 -> 4.3-5.1 us a sweep).
 constexpr int kQRun = kQRunPlanes;
-constexpr long long kQBlocks = 4 * 152;
+constexpr int kQBlocks = 4;  // an SM
 template <bool ZERO>
 __global__ void __launch_bounds__(256) k_sweep7_3d_q4(const float* __restrict__ x, float* __restrict__ y,
                                                       const float* __restrict__ b, const uint8_t* __restrict__ wq,
@@ -837,7 +837,7 @@ void launch_sweep7_3d_q(const float* x, float* y, const float* b, const uint8_t*
   if (g.tz < 3) return;
   if (sweep7_quad_ok(g, x, y, b, wq)) {
     const long long nb = (g.n2 / 4 + 255) / 256;
-    const int run = nb * ((g.tz - 2 + kQRun - 1) / kQRun) < kQBlocks ? 1 : kQRun;
+    const int run = nb * ((g.tz - 2 + kQRun - 1) / kQRun) < kQBlocks * sm_count() ? 1 : kQRun;
     const dim3 grid((unsigned)nb, (unsigned)((g.tz - 2 + run - 1) / run));
     if (x_zero)
       launch_dep(k_sweep7_3d_q4<true>, grid, 256, 0, s, x, y, b, wq, wtab, cff, g.n1, g.n2, g.tz, qact, run);
@@ -955,7 +955,7 @@ bool launch_sweep19_3d_q4(const float* x, float* y, const float* b, const float*
   const long long q0 = (g.n1 * (bx.j0 - 1)) / 4, qe = (g.n1 * bx.j1 + 3) / 4;  // quads covering rows j0 .. j1
   const long long nq = qe - q0;
   const long long nb = (nq + 255) / 256;
-  const int nk = bx.k1 - bx.k0 + 1, run = nb * ((nk + kQ19Run - 1) / kQ19Run) < kQBlocks ? 1 : kQ19Run;  // see kQBlocks
+  const int nk = bx.k1 - bx.k0 + 1, run = nb * ((nk + kQ19Run - 1) / kQ19Run) < kQBlocks * sm_count() ? 1 : kQ19Run;
   const dim3 grid((unsigned)nb, (unsigned)((nk + run - 1) / run));
   launch_dep(k_sweep19_3d_q4, grid, 256, 0, s, x, y, b, w, cff, g.n1, g.n2, bx, q0, nq, run);
   return true;

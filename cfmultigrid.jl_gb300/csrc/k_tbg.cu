@@ -249,10 +249,11 @@ __global__ void __launch_bounds__(g_threads<T>()) k_step2d(TbgArgs<T> a, int S, 
   }
 }
 
-// the core side with the least work (FP64 instructions, or cells) for the busiest of 152 SMs
+// the core side with the least work (FP64 instructions, or cells) for the busiest SM
 int tbg_tile(int max_tile, int tx, int ty, int np, int mode) {
   const bool descent = mode < 2;
   const int H = 2 * np + (descent ? 2 : 0);
+  const int nsm = sm_count();
   int best = 4;
   double cost = 0.0;
   for (int core = 4; core + 2 * H <= max_tile; core += 2) {
@@ -262,7 +263,7 @@ int tbg_tile(int max_tile, int tx, int ty, int np, int mode) {
     for (int s = 0; s < 2 * np; ++s) w += (S - 2 * (s + 1)) * (S - 2 * (s + 1));
     if (descent) w += 1.2 * (core + 2) * (core + 2);
     else if (mode == 2) w += S * S;
-    w *= (double)((tiles + 151) / 152);
+    w *= (double)((tiles + nsm - 1) / nsm);
     if (cost == 0.0 || w < cost) {
       cost = w;
       best = core;
