@@ -1272,8 +1272,11 @@ int resid_restrict3d(cfmg_handle* h, int lev) {
 // the others): 800 000, as 262^2 9-point cells (a 2048^2 F-cycle solve takes 8 %
 // less with that level in steps); 400 000 on level 1, where a 262^2 5-point
 // level lost 1.5 % of its solve and a 390 x 294 variable-coefficient one 10 %.
-constexpr long long kStepCells = 150000;  // levels that get the scratch array
 constexpr long long kStepWork = 800000, kStepWork1 = 400000;
+// the largest such level in cells: 114 285 and 72 727, level 1 57 142 and 36 363
+long long step_cells(const cfmg_desc& d, bool first) {
+  return (first ? kStepWork1 : kStepWork) / (d.op == CFMG_LAPLACIAN ? 7 : 11);
+}
 bool coef_clean(const cfmg_handle* h) { return h->coef_setup && !h->coef_exposed; }
 bool steps_clean(const cfmg_handle* h) {
   if (!coef_clean(h)) return false;
@@ -1284,8 +1287,7 @@ bool steps_clean(const cfmg_handle* h) {
 // FP32 (variable coefficient), levels of every size: a level-1 descent of 2048^2 reads its five
 // arrays once instead of in each of four sweeps (its fields hold +0 outside the wet interior always)
 bool step_size(const cfmg_handle* h, int lev, int prec) {
-  return prec || (long long)h->lv[lev - 1].len * (h->d.op == CFMG_LAPLACIAN ? 7 : 11) <=
-                     (lev == 1 ? kStepWork1 : kStepWork);
+  return prec || (long long)h->lv[lev - 1].len <= step_cells(h->d, lev == 1);
 }
 template <class T>
 bool step_ok(const cfmg_handle* h, int lev) {
@@ -1344,8 +1346,7 @@ constexpr int kSmoothPairs = 3;
 bool smooth_steps_ok(const cfmg_handle* h, int lev, int nite) {
   if (h->record || nite < 4 || lev != L(h) || lev < 2 || !steps_form(h)) return false;
   const Level& l = h->lv[lev - 1];
-  return (long long)l.len * (h->d.op == CFMG_LAPLACIAN ? 7 : 11) <= kStepWork && l.s64 &&
-         !in_engine(h, lev, CFMG_FP64) && steps_clean(h);
+  return step_size(h, lev, CFMG_FP64) && l.s64 && !in_engine(h, lev, CFMG_FP64) && steps_clean(h);
 }
 int smooth_steps(cfmg_handle* h, int lev, int nite) {
   const Level& l = h->lv[lev - 1];
@@ -2274,7 +2275,7 @@ static int create_handle(const cfmg_desc* d, cudaStream_t shared, cfmg_handle** 
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t tail_bytes = shared ? 0 : kTailPoolBytes;
   auto stepped = [&](const Level& l) {
-    return !shared && !l.threed && l.tz == 1 && (long long)l.len <= kStepCells;
+    return !shared && !l.threed && l.tz == 1 && (long long)l.len <= step_cells(*d, &l == &h->lv[0]);
   };
   auto tailed = [&](const Level& l) { return l.len <= (size_t)kTailMaxLen; };
   size_t total = al(kPartials * sizeof(double)) + al(S_COUNT * sizeof(double)) + al((size_t)pool_ops * sizeof(Op)) +
