@@ -2,7 +2,8 @@
 // one layer): FP64 levels of the 5-point, 9-point and variable-coefficient
 // operators, and FP32 levels of the variable-coefficient operator.
 //
-// A mid-size FP64 level (1500 to 150 000 cells) takes 12 launches a cycle
+// A mid-size FP64 level (600 to 114 285 cells of the 5-point operator, 72 727 of
+// the others; about half of that on level 1) takes 12 launches a cycle
 // (4 sweeps, residual, restriction, zeroing, prolongation, 4 sweeps) whose
 // own work is below a microsecond each: launch and load latency, 2.1 us a
 // graph node, is what they cost. Here a block loads a tile with a halo wide

@@ -592,7 +592,10 @@ __device__ __forceinline__ long long to_fix(double v, int k) {
   const unsigned long long M = ((unsigned long long)__funnelshift_l(lo, mh, 10) << 32) | (lo << 10);
   return (((long long)(M >> n) ^ (long long)(hi >> 31)) + 1LL) >> 1;
 }
-// 58 - E for values below 2^E
+// 58 - E for values below 2^E. The bound at -963 (k <= 1021) shows in no result:
+// where max(|x|, |b|) is below 2^-963, or below 2^-537 already, the squares of b
+// and r are zeros, so |b| and the residual are reported as 0 (or the reference
+// rule's 1) and the FP32 right-hand side, at the scale that they give, is 0.
 __device__ __forceinline__ int fix_k(int E) { return 58 - max(E, -963); }
 // k for max(|x|, |b|) (device scalars S_MAXX, S_MAXB)
 __device__ __forceinline__ int fix_exponent(const double* ds) {

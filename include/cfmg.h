@@ -110,19 +110,27 @@ extern "C" {
                                         for 3D 7-point levels and the 3D 19-point pair in one pass; 0: one
                                         kernel per sweep. All give the same bits. */
 #define CFMG_OPT_INT_RESIDUAL 3 /* mixed form, closed topology, 5-, 7-, 2D 9- and 3D 19-point
-                                   operators: 1 (default) computes the level-1 residual exactly in 64-bit fixed point
-                                   on the integer pipes; 0 in FP64 arithmetic */
+                                   operators: 1 (default) computes the level-1 residual in 64-bit fixed point
+                                   (x and b to 2^-58 of the largest, 2^-57 in the 19-point form, the sums
+                                   exact) on the integer pipes, where the diagonal is the operator's or
+                                   small enough for the sums; 0 in FP64 arithmetic */
 #define CFMG_OPT_HOST_LOOP 4 /* cfmg_solve: 0 (default) runs the whole loop as one graph launch (a
                                 `while` node); 1 launches one graph per iteration from the host, which
                                 profilers that do not descend into conditional nodes can see */
 #define CFMG_OPT_FUSED_DESCENT 5 /* 2D closed topology: 1 (default) a cycle's steps on a level take fewer
                                     launches. Mixed form, lean packed passes: the last pre-smoothing pass
                                     also forms the residual, restricts it to the coarse b and zeroes the
-                                    coarse x. FP64 levels between the coarse tail and 150 000 cells, and
-                                    FP32 levels of the variable-coefficient operator, with omega <= 1: one
-                                    launch for the descent, one for the ascent, and few for a long
-                                    smoothing of the last FP64 level. 0 separate kernels. Both give the
-                                    same bits. */
+                                    coarse x. FP64 levels between the coarse tail and 114 285 cells of the
+                                    5-point operator, 72 727 of the others (level 1: half of that), and
+                                    FP32 levels of the variable-coefficient operator: in V- and F-cycles
+                                    with 1 to 3 pairs and omega <= 1, one launch for the descent, one for
+                                    the ascent, and few for a long smoothing of the last FP64 level. These
+                                    steps need the coefficients that cfmg_setup_operators made (no
+                                    upload, cfmg_bind_level or cfmg_field_ptr of one since), the FP64
+                                    ones also x, y, r and b of levels 2.. zeroed with cfmg_zero after it
+                                    (and not written or exposed since); else the levels take separate
+                                    kernels, or the tail or engine. 0 separate kernels. Both give the same
+                                    bits. */
 #define CFMG_OPT_FUSED_UPDATE 6 /* mixed form, 2D closed topology, integer residual, lean packed passes:
                                    1 (default) the cycle's last level-1 post-smoothing pass also applies
                                    the FP64 solution update x += e * iscale (and collects max |x|)
@@ -143,9 +151,10 @@ extern "C" {
                                      shared memory; 0 never (separate sweeps). The same bits. With a
                                      value > 0 every operator of a cycle below the level whose arrays fit
                                      one block's shared memory (all operators and topologies; FP64 levels
-                                     up to 6/5 of their engine threshold, or 12/25 of it where
+                                     up to 6/5 of their engine threshold, or 12/25 of it while
                                      CFMG_OPT_FUSED_DESCENT serves the larger ones) runs in one launch there; with 0
-                                     they are Ops of the cluster engine. Same values either way. */
+                                     they are Ops of the cluster engine. Same values either way, NaN and
+                                     infinities on land included. */
 #define CFMG_OPT_SKIP_DRY 10 /* mixed form, closed topology: 1 (default) passes skip groups of cells
                                that are all dry (their FP32 fields hold +0 and stay +0): the FP32
                                prolongation's parents, the strip residual's tasks; for the 3D 7-point
