@@ -431,15 +431,13 @@ __global__ void __launch_bounds__(kMxThreads) k_resid_int2d(const double* __rest
 
 template <int KIND, bool NEUMANN>
 static int int2d_grid() {
-  static int blocks = 0;  // one wave: resident blocks per SM x SMs, at most kMxParts
-  if (!blocks) {
-    int dev = 0, nsm = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // one wave: resident blocks per SM x SMs, at most kMxParts; made by one thread
+  // (another that saw it before the cut launched more blocks than there are partials)
+  static const int blocks = [] {
+    int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resid_int2d<KIND, NEUMANN>, kMxThreads, 0);
-    blocks = nsm * (per > 0 ? per : 1);
-    if (blocks > kMxParts || blocks <= 0) blocks = kMxParts;
-  }
+    return std::min(kMxParts, sm_count() * std::max(per, 1));
+  }();
   return blocks;
 }
 

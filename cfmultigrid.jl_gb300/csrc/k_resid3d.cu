@@ -31,6 +31,7 @@
 // residual, and 1 into ds[S_FAULT], which the solve reports.
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "cfmg_internal.h"
@@ -464,18 +465,15 @@ bool encode3(CUtensorMap* m, CUtensorMapDataType dt, int esize, const void* base
 template <int JT, bool NEUMANN, bool ALL>
 int r3_grid() {
   // one wave of the form that skips dry planes: resident blocks per SM x SMs, at
-  // most kMxParts (the form that writes them too takes the same blocks)
-  static int blocks = 0;
-  if (!blocks) {
-    int dev = 0, nsm = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // most kMxParts (the form that writes them too takes the same blocks); made by
+  // one thread, as int2d_grid
+  static const int blocks = [] {
+    int per = 0;
     cudaFuncSetAttribute(k_resid_int3d<JT, NEUMANN, ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, R3Cfg<JT>::Smem);
     cudaFuncSetAttribute(k_resid_int3d<JT, NEUMANN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, R3Cfg<JT>::Smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resid_int3d<JT, NEUMANN, ALL>, kMxThreads, R3Cfg<JT>::Smem);
-    blocks = nsm * (per > 0 ? per : 1);
-    if (blocks > kMxParts || blocks <= 0) blocks = kMxParts;
-  }
+    return std::min(kMxParts, sm_count() * std::max(per, 1));
+  }();
   return blocks;
 }
 
